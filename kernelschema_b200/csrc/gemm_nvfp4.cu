@@ -17,11 +17,11 @@
 // One CTA per SM, warp-specialised: TMA producer, MMA issuer, scale-factor copiers, epilogue warps (roles are listed
 // at each kernel). Stage = 256 FP4 of K: A 16 KB, B BN*128 B, scale factors 2 KB per 128 rows.
 //
-// What bounds the mainloop is the rate at which ONE thread can issue tcgen05 instructions: about 48 cycles per
-// instruction (tcgen05.cp, tcgen05.mma and tcgen05.commit alike), measured on B200 with an issue-only loop. A 128 x 256
-// stage needs 12 scale-factor copies + 4 MMAs (512 tensor cycles): 16 x 48 = 770 cycles from one thread, 12 x 48 + a
-// wait + a commit = 880 from one copier thread beside an MMA thread. Different warps issue concurrently, so the copies
-// are split over kCopiers warps (6 each for BN = 256): every issuing thread stays below the 512 cycles of its stage.
+// The tcgen05 and TMA instructions of a role are issued inside `if (elect_one())`, not `if (lane == 0)`: with elect.sync the
+// compiler knows that one thread runs the branch and keeps descriptors in uniform registers; with a lane test every issue
+// costs about 48 cycles (measured with an issue-only loop). A 128 x 256 stage needs 12 scale-factor copies + 4 MMAs (512
+// tensor cycles), spread over kCopiers warps beside the MMA thread. 8192^3, lane test -> elect.sync: CTA-pair kernel
+// 356 -> 223 us (one thread issues for two SMs), 128 x 128 tiles 279 -> 266 us, 128 x 256 tiles 231 -> 227 us.
 #include "kernels.cuh"
 #include "ptx.cuh"
 
@@ -251,7 +251,7 @@ k_gemm_nvfp4(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
   const uint32_t bar_acc_empty = bar_acc_full + 8 * C::kAccBufs;
   const uint32_t s_tmem_slot = bar_acc_empty + 8 * C::kAccBufs;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_uniform();
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -337,7 +337,7 @@ k_gemm_nvfp4(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
         }
       }
       if (lane == 0) pdl_trigger();
-    } else if (lane == 0) {
+    } else if (elect_one()) {
       uint32_t s = 0, ph = 1;
       bool ok = true;
       // the tile-table entries of an item are fetched one item ahead, so their latency hides behind a whole k-loop
@@ -377,14 +377,14 @@ k_gemm_nvfp4(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
     }
   } else if (warp >= 2 && warp < kFirstEpiWarp) {
     // ------------------------------------------------------------------ scale-factor copiers: shared memory -> TMEM
-    if (lane == 0) {
+    if (elect_one()) {
       if (warp == 2) copier_loop<BN, 0>(p, tmem, s_sfa, s_sfb, bar_full, bar_sf, total_items, nk);
       else if (warp == 3) copier_loop<BN, 1 % kCopiers>(p, tmem, s_sfa, s_sfb, bar_full, bar_sf, total_items, nk);
       else copier_loop<BN, 2 % kCopiers>(p, tmem, s_sfa, s_sfb, bar_full, bar_sf, total_items, nk);
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       // One thread feeds the tensor pipe with four instructions per stage: everything is 32-bit, the stage ring is
       // walked with counters and the shared-memory descriptors are base + stage * stride.
       constexpr uint32_t idesc = make_idesc_nvf4(kBM, BN);
@@ -496,7 +496,7 @@ k_gemm_nvfp4_pair(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   const uint32_t bar_acc_empty = bar_acc_full + 8;            // leader: 32 epilogue warps of the pair
   const uint32_t s_tmem_slot = bar_acc_empty + 8;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_uniform();
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
@@ -529,7 +529,7 @@ k_gemm_nvfp4_pair(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (both CTAs, own halves)
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t s = 0, ph = 1;
       bool ok = true;
       const uint32_t full0 = map_to_cta(bar_full, 0);
@@ -556,7 +556,7 @@ k_gemm_nvfp4_pair(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     }
   } else if (warp >= 2 && warp < kFirstEpiWarp) {
     // ------------------------------------------------------------------ scale-factor copiers (leader; every copy acts on both CTAs)
-    if (leader && lane == 0) {
+    if (leader && elect_one()) {
       constexpr uint32_t kHiSf = (128u >> 4) | (1u << 14);
       const int j0 = warp - 2;
       const uint32_t sfa_lo0 = (s_sfa >> 4) & 0x3FFF, sfb_lo0 = (s_sfb >> 4) & 0x3FFF;
@@ -583,7 +583,7 @@ k_gemm_nvfp4_pair(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (leader && lane == 0) {
+    if (leader && elect_one()) {
       constexpr uint32_t idesc = make_idesc_nvf4(256, BN);
       constexpr uint32_t kHiOp = (1024u >> 4) | (1u << 14) | (2u << 29);
       const uint32_t a_lo0 = ((s_a >> 4) & 0x3FFF) | (1u << 16), b_lo0 = ((s_b >> 4) & 0x3FFF) | (1u << 16);

@@ -22,6 +22,18 @@ DEV void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "m
 DEV void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 DEV uint32_t lane_id() { return threadIdx.x & 31; }
+// Warp index as a value the compiler knows to be the same in the whole warp (role dispatch of the specialised kernels).
+DEV int warp_uniform() { return __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0); }
+// True in exactly one lane of the (converged) warp.
+DEV bool elect_one() {
+  uint32_t e;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xFFFFFFFF;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(e));
+  return e != 0;
+}
 
 // ----------------------------------------------------------------------------- mbarrier
 DEV void mbar_init(uint32_t bar, uint32_t count) {
