@@ -16,7 +16,7 @@ constexpr int kRouteChunk = 2048;        // routes per block: 32 warps x 2 steps
 constexpr int kRouteWarps = 32;          // these kernels are a few thousand dependent instructions per warp and one block per
                                          // chunk: with 8 warps a block issued one instruction every ~5 cycles per scheduler
 constexpr int kRouteThreads = kRouteWarps * 32;
-constexpr int kRouteSmemMax = 176 * 1024;  // (32 + 2) x 1024 experts x 4 B + 32 KB of positions (kGatherMaxRoutes x 4 B)
+constexpr int kRouteSmemMax = 144 * 1024;  // (32 + 2) x 1024 experts x 4 B
 
 struct RouteView {
   const int32_t* ids;
@@ -293,7 +293,8 @@ __global__ void __launch_bounds__(kRouteThreads) k_route_scatter(RouteView r, co
 // the segment). The counts of foreign chunks are accumulated with shared-memory atomics; a count does not depend on the
 // order of the additions, so every output stays reproducible. Block 0 also writes the per-expert tables.
 constexpr int kFusedMaxBlocks = 8;
-constexpr int kGatherMaxRoutes = 8192;           // the fused form that also permutes the rows: 8 routes per lane of ONE chunk
+constexpr int kGatherMaxRoutes = 16384;          // the fused form that also permutes the rows
+constexpr int kGatherMaxChunk = 256;             // routes a block of it may own (8 warps)
 
 // The permute of one routed row from inside the route-map kernel (small batches): payload with 16-byte vectors, the row's
 // scale words straight into the 128x4-tiled image. Scales of padding rows are left as they are: the GEMMs neither store
@@ -334,11 +335,11 @@ DEV void gather_row(const GatherView& g, int tok, int pos, int lane) {
 }
 
 // Block-wide scan over the experts, shared by the one-launch kernels. In: hist[w][e] = routes of expert e that warp w of
-// this block owns, others[e] = routes of e owned by other blocks, before[e] = those of them that precede this block's.
+// this block owns, before[e] / after[e] = routes of e owned by the blocks that precede / follow this one.
 // Out: segment starts, tile and pair tables and totals (stored by the `writer` block only), and hist[w][e] turned into
 // the permuted row of warp w's first route of expert e. Ends with a block barrier.
-template <int NW>                                  // NW = warps of the block = rows of hist
-DEV void scan_experts(int etot, const int* others, const int* before, int* hist, bool writer, const RouteMapBuffers& b) {
+template <int NW>                                  // NW = warps that own routes = rows of hist
+DEV void scan_experts(int etot, const int* after, const int* before, int* hist, bool writer, const RouteMapBuffers& b) {
   constexpr int nw = NW;
   __shared__ int warp_pad[kRouteWarps], warp_tiles[kRouteWarps], warp_pairs[kRouteWarps], warp_cnt[kRouteWarps];
   __shared__ int carry[4];
@@ -349,7 +350,7 @@ DEV void scan_experts(int etot, const int* others, const int* before, int* hist,
     const int e = e0 + threadIdx.x;
     int cnt = 0;
     if (e < etot) {
-      cnt = others[e];
+      cnt = after[e] + before[e];
 #pragma unroll
       for (int w = 0; w < nw; ++w) cnt += hist[w * etot + e];
     }
@@ -393,7 +394,7 @@ DEV void scan_experts(int etot, const int* others, const int* before, int* hist,
     __syncthreads();
     if (threadIdx.x == blockDim.x - 1) {
       int tc = 0;
-      for (int w = 0; w < nw; ++w) tc += warp_cnt[w];
+      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) tc += warp_cnt[w];
       carry[0] = bp + ip;
       carry[1] = bt + it;
       carry[2] += tc;
@@ -416,8 +417,8 @@ DEV int routes_per_warp(int chunk_total, int nw = kRouteWarps) { return max(32, 
 
 __global__ void __launch_bounds__(kRouteThreads) k_route_fused(RouteView r, const float* __restrict__ scores, int etot, RouteMapBuffers b) {
   extern __shared__ int hist[];                    // own chunk [kRouteWarps][etot] | all chunks [etot] | chunks before [etot]
-  int* others = hist + kRouteWarps * etot;         // routes of expert e in the other chunks
-  int* before = others + etot;                     // ... in the chunks before this block's
+  int* after = hist + kRouteWarps * etot;          // routes of expert e in the chunks after this block's
+  int* before = after + etot;                      // ... in the chunks before it
   const int kk = r.K + r.S;
   const int total = (int)(r.T * kk);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -425,7 +426,7 @@ __global__ void __launch_bounds__(kRouteThreads) k_route_fused(RouteView r, cons
   const int rpw = routes_per_warp(min(kRouteChunk, total - (int)blockIdx.x * kRouteChunk));
   pdl_trigger();
   pdl_wait();
-  for (int i = threadIdx.x; i < 2 * etot; i += blockDim.x) others[i] = 0;
+  for (int i = threadIdx.x; i < 2 * etot; i += blockDim.x) after[i] = 0;
   __syncthreads();
   int ex[kRouteSteps];
   float wt[kRouteSteps];                           // routing weight of each own route: fetched with the ids, before any store
@@ -447,13 +448,10 @@ __global__ void __launch_bounds__(kRouteThreads) k_route_fused(RouteView r, cons
       eo[step] = route_expert32(r, c * kRouteChunk + warp * kRoutesPerWarp + step * 32 + lane, total);
 #pragma unroll
     for (int step = 0; step < kRouteSteps; ++step)
-      if (eo[step] >= 0) {
-        atomicAdd(&others[eo[step]], 1);
-        if (c < (int)blockIdx.x) atomicAdd(&before[eo[step]], 1);
-      }
+      if (eo[step] >= 0) atomicAdd((c < (int)blockIdx.x ? before : after) + eo[step], 1);
   }
-  chunk_histogram(ex, etot, hist);                 // own chunk, per warp; its barriers also publish others/before
-  scan_experts<kRouteWarps>(etot, others, before, hist, writer, b);
+  chunk_histogram(ex, etot, hist);                 // own chunk, per warp; its barriers also publish after/before
+  scan_experts<kRouteWarps>(etot, after, before, hist, writer, b);
   int pos[kRouteSteps];
 #pragma unroll
   for (int step = 0; step < kRouteSteps; ++step) {
@@ -479,72 +477,66 @@ __global__ void __launch_bounds__(kRouteThreads) k_route_fused(RouteView r, cons
   }
 }
 
-// Route map AND permute of a decode-sized batch (at most kGatherMaxRoutes routes) in one launch: every block builds the
-// whole map for itself in shared memory (a few thousand integer operations), block 0 stores it, and the blocks share the
-// row copies, one warp per routed row. The step loops are rolled: a one-wave, latency-bound kernel pays for every
-// instruction-cache line it touches, and a decode batch takes one step.
-template <int NW>                                  // warps per block: 8 for a handful of routes, kRouteWarps otherwise
-__global__ void __launch_bounds__(NW * 32) k_route_gather(RouteView r, const float* __restrict__ scores, int etot, RouteMapBuffers b,
-                                                     GatherView gv) {
-  extern __shared__ int hist[];                    // [warps][etot] | zeros [etot] | zeros [etot] | expert, then row, of every route
-  constexpr int nw = NW;
-  int* zeros = hist + nw * etot;
-  int* s_pos = zeros + 2 * etot;
+// Route map AND permute of a batch of at most kGatherMaxRoutes routes in one launch. Block b owns the routes
+// [b * chunk, (b + 1) * chunk), at most 32 * OW of them, and reads the expert ids of ALL routes itself: shared-memory counters
+// of the routes before and after its own give the segment starts and its base inside each segment (counts do not depend on
+// the order of the additions, so every output is reproducible), and only its own routes need the stable ranking. Then its
+// warps copy its rows. Building the whole ranked map in every block instead costs eight dependent ranking rounds at 8192
+// routes and 32 warps' histograms to zero, sum and scan. Layer call at T = 1024, H = 7168, 256 experts (this launch took 37 us
+// of it): 249 -> 234 us; at 14 216 routes, H = 2048 (route map and permute were two launches, 28 us): 118 -> 110 us.
+template <int OW>                                  // warps that own routes
+__global__ void __launch_bounds__(kRouteThreads) k_route_gather(RouteView r, const float* __restrict__ scores, int etot, int chunk,
+                                                               RouteMapBuffers b, GatherView gv) {
+  extern __shared__ int hist[];                    // own routes [OW][etot] | routes after [etot] | before [etot] | own positions [OW * 32]
+  int* after = hist + OW * etot;
+  int* before = after + etot;
+  int* s_pos = before + etot;
   const int kk = r.K + r.S;
   const int total = (int)(r.T * kk);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const bool writer = blockIdx.x == 0;
-  const int rpw = routes_per_warp(total, nw), nsteps = rpw >> 5;
-  const int bits = expert_bits(etot);
+  const int lo = (int)blockIdx.x * chunk, hi = min(total, lo + chunk);
   pdl_trigger();
+  for (int i = threadIdx.x; i < (OW + 2) * etot; i += blockDim.x) hist[i] = 0;
+  __syncthreads();
   pdl_wait();
-  for (int i = threadIdx.x; i < (nw + 2) * etot; i += blockDim.x) hist[i] = 0;
+  const bool flat = r.S == 0 && r.id_stride == r.K && r.seg_len <= 0;      // route f's expert is ids[f]: no division
+  const int f_own = lo + warp * 32 + lane;
+  const int e_own = warp < OW && f_own < hi ? route_expert32(r, f_own, total) : -1;
 #pragma unroll 4
-  for (int step = 0; step < nsteps; ++step) {
-    const int f = warp * rpw + step * 32 + lane;
-    if (f < total) s_pos[f] = route_expert32(r, f, total);
-  }
-  __syncthreads();
-#pragma unroll 1
-  for (int step = 0; step < nsteps; ++step) {
-    const int f = warp * rpw + step * 32 + lane;
-    const int e = f < total ? s_pos[f] : -1;
-    if (!__any_sync(0xFFFFFFFFu, e >= 0)) continue;
-    const unsigned m = same_expert_lanes(e, bits);
-    if (e >= 0 && lane == (__ffs(m) - 1)) hist[warp * etot + e] += __popc(m);
-    __syncwarp();
-  }
-  __syncthreads();
-  scan_experts<NW>(etot, zeros, zeros + etot, hist, writer, b);
-#pragma unroll 1
-  for (int step = 0; step < nsteps; ++step) {
-    const int f = warp * rpw + step * 32 + lane;
-    const int e = f < total ? s_pos[f] : -1;
-    int at = -1;
-    if (__any_sync(0xFFFFFFFFu, e >= 0)) {
-      const unsigned m = same_expert_lanes(e, bits);
-      if (e >= 0) at = hist[warp * etot + e] + __popc(m & ((1u << lane) - 1u));
-      __syncwarp();
-      if (e >= 0 && lane == (__ffs(m) - 1)) hist[warp * etot + e] += __popc(m);
-      __syncwarp();
+  for (int f = threadIdx.x; f < total; f += blockDim.x) {
+    int e;
+    if (flat) {
+      e = r.ids[f] - r.expert_offset;
+      if (e >= r.E) e = -1;
+    } else {
+      e = route_expert32(r, f, total);
     }
-    if (f < total) {
-      s_pos[f] = at;
-      if (writer) {
-        b.row_of[f] = at;
-        if (at >= 0) {
-          const int t = f / kk, k = f - t * kk;
-          b.tok_of_row[at] = t;
-          b.weight_of_row[at] = (scores && k < r.K) ? scores[(int64_t)t * r.id_stride + k] : 1.0f;
-        }
+    if (e >= 0 && (f < lo || f >= hi)) atomicAdd((f < lo ? before : after) + e, 1);
+  }
+  unsigned same = 0;
+  if (warp < OW) {
+    same = same_expert_lanes(e_own, expert_bits(etot));
+    if (e_own >= 0 && lane == (__ffs(same) - 1)) hist[warp * etot + e_own] = __popc(same);
+  }
+  __syncthreads();
+  scan_experts<OW>(etot, after, before, hist, blockIdx.x == 0, b);
+  if (warp < OW) {
+    int at = -1;
+    if (e_own >= 0) at = hist[warp * etot + e_own] + __popc(same & ((1u << lane) - 1u));
+    s_pos[warp * 32 + lane] = at;
+    if (f_own < hi) {
+      b.row_of[f_own] = at;
+      if (at >= 0) {
+        const int t = f_own / kk, k = f_own - t * kk;
+        b.tok_of_row[at] = t;
+        b.weight_of_row[at] = (scores && k < r.K) ? scores[(int64_t)t * r.id_stride + k] : 1.0f;
       }
     }
   }
   __syncthreads();
-  const int warps = (int)gridDim.x * nw;
-  for (int f = (int)blockIdx.x * nw + warp; f < total; f += warps) {
-    const int at = s_pos[f];
-    if (at >= 0) gather_row(gv, f / kk, at, lane);
+  for (int i = warp; i < hi - lo; i += (int)(blockDim.x >> 5)) {
+    const int at = s_pos[i];
+    if (at >= 0) gather_row(gv, (lo + i) / kk, at, lane);
   }
 }
 
@@ -575,9 +567,15 @@ int launch_route_map(const int32_t* ids, const float* scores, int64_t id_stride,
   return (int)err;
 }
 
+// Blocks of the one-launch form: one row per warp while the SMs last.
+static int route_gather_blocks(int64_t total, int threads) {
+  const int64_t blocks = (total + threads / 32 - 1) / (threads / 32);
+  return (int)(blocks < sm_count() ? blocks : sm_count());
+}
+
 bool route_gather_fits(int64_t T, int K, int S, int E, int H) {
   const int64_t total = T * (K + S);
-  return total >= 1 && total <= kGatherMaxRoutes && sizeof(int) * ((kRouteWarps + 2) * (size_t)(E + S) + kGatherMaxRoutes) <= kRouteSmemMax &&
+  return total >= 1 && total <= kGatherMaxRoutes && total <= (int64_t)route_gather_blocks(total, kRouteThreads) * kGatherMaxChunk &&
          H % 256 == 0;
 }
 
@@ -589,17 +587,18 @@ int launch_route_gather(const int32_t* ids, const float* scores, int64_t id_stri
   RouteView r{ids, id_stride > 0 ? id_stride : K, T, K, S, E, expert_offset, seg_valid ? seg_len : 0, seg_valid};
   GatherView gv{(const uint8_t*)hid_q, (const uint8_t*)hid_sf, q_stride > 0 ? q_stride : (int64_t)(H / 2),
                 sf_stride > 0 ? sf_stride : (int64_t)(H / 16), H, (uint8_t*)a_q, (uint8_t*)a_sf};
-  // a handful of routes (one step of 8 warps): a small block, whose barriers and zeroing cost less (T = 1: 2 us per step)
+  // a handful of routes: a small block, whose barriers and zeroing cost less (T = 1: 2 us per step)
   const int threads = total <= 256 ? 256 : kRouteThreads;
-  int64_t blocks = (total + threads / 32 - 1) / (threads / 32);     // one row per warp while the SMs last
-  if (blocks > sm_count()) blocks = sm_count();
-  if (threads == 256)       // at most 256 routes: their positions need 1 KB, the whole block stays far below 48 KB
-    return (int)launch_chain(k_route_gather<8>, dim3((unsigned)blocks), dim3(256), sizeof(int) * ((8 + 2) * (size_t)etot + 256), st, r,
-                             scores, etot, b, gv);
-  static SmemOptIn opt_in;
-  if (int e = opt_in.ensure(k_route_gather<kRouteWarps>, kRouteSmemMax)) return e;
-  return (int)launch_chain(k_route_gather<kRouteWarps>, dim3((unsigned)blocks), dim3(kRouteThreads),
-                           sizeof(int) * ((kRouteWarps + 2) * (size_t)etot + kGatherMaxRoutes), st, r, scores, etot, b, gv);
+  const int blocks = route_gather_blocks(total, threads);
+  const int chunk = (int)((total + blocks - 1) / blocks);
+  auto go = [&](auto kern, int ow) {               // at most (8 + 2) x 1024 counters + 256 positions: 41 KB
+    return (int)launch_chain(kern, dim3((unsigned)((total + chunk - 1) / chunk)), dim3(threads),
+                             sizeof(int) * ((ow + 2) * (size_t)etot + 32 * (size_t)ow), st, r, scores, etot, chunk, b, gv);
+  };
+  if (chunk <= 32) return go(k_route_gather<1>, 1);
+  if (chunk <= 64) return go(k_route_gather<2>, 2);
+  if (chunk <= 128) return go(k_route_gather<4>, 4);
+  return go(k_route_gather<8>, 8);
 }
 
 // ----------------------------------------------------------------------------- allocation-free variant

@@ -68,6 +68,18 @@ def test_small_batch_map_rows_and_output(tokens, tma_gather):
     assert_layer_parity(got, o.moe_expected(p), f"T={tokens}")
 
 
+@pytest.mark.parametrize("tokens,experts,masked", [(4, 24, False), (5, 24, True), (592, 24, True), (593, 24, False), (1185, 260, True), (2047, 24, True),
+                                                   (2048, 24, False), (2049, 24, True)])
+def test_one_launch_map_at_the_edges_of_a_blocks_share(tokens, experts, masked):
+    """8 routes per token (7 routed + 1 shared): up to 32 routes one warp of a block owns routes, from 4737 (148 blocks of 32)
+    two, from 9473 four; 16384 routes are the last size of the one-launch form."""
+    from gpu_util import run_model
+    p = make_moe_case(400 + tokens, tokens, 256, 256, experts, 7, shared=1, routing="zipf", masked=masked)
+    got, _, model = run_model(p)
+    _check_map_and_rows(p, model)
+    assert_layer_parity(got, o.moe_expected(p), f"T={tokens}")
+
+
 def test_small_batch_hotspot_rows_stay_in_route_order():
     """Every token picks the same experts: each segment holds one row per token, in ascending token order."""
     from gpu_util import run_model
