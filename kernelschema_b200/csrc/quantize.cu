@@ -3,7 +3,7 @@
 // Follows, bit for bit, the reference input generator's quantize():
 //   moe/nvfp4_fused_moe/problem/input.py:53-71            (global scale 1)
 //   gemm/dense/bf16_nvfp4_gemm/problem/input.py:40-64     (global scale != 1)
-// One thread owns one 16-element block: two 128-bit loads, one 64-bit payload store, one scale byte.
+// One thread owns one 16-element block: 32 bytes loaded, one 64-bit payload store, a quarter of a scale word.
 // HBM-bound: 2 B read + 0.5625 B written per element.
 #include <math.h>
 
@@ -19,75 +19,164 @@ DEV size_t sf_tiled_offset(int64_t row, int64_t blk, int64_t chunks_per_row) {
          (size_t)(blk & 3);
 }
 
-// Quotients x / (stored * gs) without sixteen IEEE divisions per block. With d = RN(stored * gs) (what the reference
-// divides by), r = RN(1 / d), q0 = RN(x * r), the residual rem = x - q0 * d is exact in one fma (q0 is within 1.5 ulp of
-// x / d and x has only 8 significant bits), and q1 = RN(q0 + rem * r) is the correctly rounded quotient (Markstein's
-// residual correction with a correctly rounded reciprocal). The E2M1 code only depends on the side of seven thresholds
-// the quotient lies on, so a last-bit error could matter only when x / d is within an ulp of a threshold; the test suite
-// sweeps every bf16 value against every E4M3 scale x a set of global scales and compares the codes with true division.
+// Packed fp32 arithmetic: two IEEE operations per instruction and lane.
+DEV uint64_t pack_f32x2(uint32_t lo, uint32_t hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
+  return r;
+}
+DEV uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+DEV uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// RN(a / b) from r = RN(1 / b): Markstein's residual correction, twice. The first step brings the quotient within an ulp, the
+// second (whose residual is then exact in one fma) rounds it correctly.
+DEV float div_rn(float a, float b, float r) {
+  float q = __fmul_rn(a, r);
+  q = __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
+  return __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
+}
+
+// What a block of 16 divides by, for every E4M3 scale byte: d = RN(stored * gs) (the reference divides by that) and
+// -RN(1 / d). 128 entries in shared memory, filled once per thread block.
+struct ScaleRow {
+  float d, neg_r;
+};
+
+// One block of 16 bf16 values (eight words) -> its E4M3 scale byte and 16 E2M1 codes.
+//
+// Quotients x / (stored * gs) without sixteen IEEE divisions per block. With r = RN(1 / d), q0 = RN(x * r), the residual
+// rem = x - q0 * d is exact in one fma (q0 is within 1.5 ulp of x / d and x has only 8 significant bits), and
+// q1 = RN(q0 + rem * r) is the correctly rounded quotient (Markstein's residual correction with a correctly rounded
+// reciprocal). The E2M1 code only depends on the side of seven thresholds the quotient lies on, so a last-bit error could
+// matter only when x / d is within an ulp of a threshold; the test suite sweeps every bf16 value against every E4M3 scale x a
+// set of global scales and compares the codes with true division. The chain runs on -x and -r: -rem = q0 * d + (-x) and
+// q1 = (-rem) * (-r) + q0 round alike, and both zeros come out with the sign of x (they encode as 0 and 8).
 // EXACT_DIV selects IEEE division instead (global scales so small or large that the residual could leave the normal range).
 template <bool EXACT_DIV>
-__global__ void __launch_bounds__(256) k_quantize_nvfp4(const __nv_bfloat16* __restrict__ x, int64_t rows, int64_t cols,
-                                                        int64_t row_stride, float gs, uint8_t* __restrict__ payload,
-                                                        uint8_t* __restrict__ scales, int sf_layout) {
-  // One block walks rows, its threads walk the 16-element blocks of a row: no integer division anywhere.
-  const int blocks_per_row = (int)(cols >> 4);
-  pdl_trigger();
-  pdl_wait();
-  for (int64_t row = blockIdx.x; row < rows; row += gridDim.x)
-  for (int blk = threadIdx.x; blk < blocks_per_row; blk += blockDim.x) {
-    const uint4* src = reinterpret_cast<const uint4*>(x + row * row_stride + blk * 16);
-    uint4 raw[2];
-    raw[0] = __ldg(src);
-    raw[1] = __ldg(src + 1);
-    const uint32_t* w = reinterpret_cast<const uint32_t*>(raw);
-    float v[16];
+DEV uint32_t quantize_block(const uint32_t (&w)[8], float gs, float rgs, const ScaleRow* __restrict__ table, uint32_t (&packed)[2]) {
+  __nv_bfloat162 m = __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[0]));      // the largest magnitude, exact in bf16
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      v[2 * i] = __uint_as_float(w[i] << 16);
-      v[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
-    }
-    float peak = 0.f;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) peak = fmaxf(peak, fabsf(v[i]));
-    peak = fmaxf(peak, 9.5367431640625e-07f);                       // clamp_min(2^-20), before the global scale
-    float scale = __fdiv_rn(peak, 6.0f);
+  for (int i = 1; i < 8; ++i) m = __hmax2(m, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[i])));
+  float peak = fmaxf(__low2float(m), __high2float(m));
+  peak = fmaxf(peak, 9.5367431640625e-07f);                       // clamp_min(2^-20), before the global scale
+  float scale;
+  if (EXACT_DIV) {
+    scale = __fdiv_rn(peak, 6.0f);
     if (gs != 1.0f) scale = __fdiv_rn(scale, gs);
-    scale = fminf(fmaxf(scale, 0.001953125f), 448.0f);               // clamp(2^-9, 448)
-    const uint32_t sbyte = cvt_e4m3(scale);
-    const float d = __fmul_rn(e4m3_to_f32(sbyte), gs);               // the reference divides by stored * gs
-    uint32_t packed[2];
-    if (EXACT_DIV) {
+  } else {
+    // operands beyond 6144 * gs and 1024 * gs only ever give a scale that the clamp below turns into 448
+    scale = div_rn(fminf(peak, 6144.0f * gs), 6.0f, 1.0f / 6.0f);
+    scale = div_rn(scale, gs, rgs);
+  }
+  scale = fminf(fmaxf(scale, 0.001953125f), 448.0f);               // clamp(2^-9, 448)
+  const uint32_t sbyte = cvt_e4m3(scale);
+  if (EXACT_DIV) {
+    const float d = __fmul_rn(e4m3_to_f32(sbyte), gs);
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        uint32_t word = 0;
+    for (int h = 0; h < 2; ++h) {
+      float q[8];
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-          word |= cvt_e2m1x2(__fdiv_rn(v[8 * h + 2 * i], d), __fdiv_rn(v[8 * h + 2 * i + 1], d)) << (8 * i);
-        packed[h] = word;
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t u = w[4 * h + i];
+        q[2 * i] = __fdiv_rn(__uint_as_float(u << 16), d);
+        q[2 * i + 1] = __fdiv_rn(__uint_as_float(u & 0xFFFF0000u), d);
       }
-    } else {
-      const float r = __frcp_rn(d);
+      packed[h] = cvt_e2m1x8(q);
+    }
+  } else {
+    const ScaleRow row = table[sbyte];
+    const uint32_t nr = __float_as_uint(row.neg_r), db = __float_as_uint(row.d);
+    const uint64_t nr2 = pack_f32x2(nr, nr), d2 = pack_f32x2(db, db);
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        uint32_t word = 0;
+    for (int h = 0; h < 2; ++h) {
+      float q[8];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float a = v[8 * h + 2 * i], b = v[8 * h + 2 * i + 1];
-          float qa = a * r, qb = b * r;
-          qa = copysignf(fmaf(fmaf(-qa, d, a), r, qa), a);     // keep -0 and negative underflow: they encode as 8
-          qb = copysignf(fmaf(fmaf(-qb, d, b), r, qb), b);
-          word |= cvt_e2m1x2(qa, qb) << (8 * i);
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t u = w[4 * h + i];
+        const uint64_t nx = pack_f32x2(u * 65536u + 0x80000000u, (u & 0xFFFF0000u) ^ 0x80000000u);
+        const uint64_t q0 = mul_f32x2(nx, nr2);
+        const uint64_t q1 = fma_f32x2(fma_f32x2(q0, d2, nx), nr2, q0);
+        q[2 * i] = __uint_as_float((uint32_t)q1);
+        q[2 * i + 1] = __uint_as_float((uint32_t)(q1 >> 32));
+      }
+      packed[h] = cvt_e2m1x8(q);
+    }
+  }
+  return sbyte;
+}
+
+// A block of threads = rows_per_block rows x threads_per_row 16-element blocks (one integer division per thread); every
+// thread has the loads of kRowsInFlight rows out before it computes. It was bound by the issue rate (223 instructions per 16
+// elements at 71 % of the issue slots, 8192 x 7168 in 33 us): hence packed arithmetic, packed maxima, the table instead of a
+// reciprocal per block, corrected multiplications instead of two divisions, and one scale store per four threads.
+constexpr int kRowsInFlight = 2;
+
+template <bool EXACT_DIV, bool WIDE>      // WIDE: rows start on 32-byte boundaries, one 256-bit load per block
+__global__ void __launch_bounds__(256, 4) k_quantize_nvfp4(const __nv_bfloat16* __restrict__ x, int64_t rows, int blocks_per_row,
+                                                        int64_t row_stride, float gs, uint8_t* __restrict__ payload,
+                                                        uint8_t* __restrict__ scales, int sf_layout, int threads_per_row,
+                                                        int rows_per_block, int word_scales) {
+  __shared__ ScaleRow table[128];
+  pdl_trigger();
+  if (!EXACT_DIV) {
+    for (int i = threadIdx.x; i < 128; i += blockDim.x) {
+      const float d = __fmul_rn(e4m3_to_f32((uint32_t)i), gs);
+      table[i] = {d, -__frcp_rn(d)};
+    }
+    __syncthreads();
+  }
+  const float rgs = __frcp_rn(gs);
+  const int r = (int)threadIdx.x / threads_per_row;
+  const int blk0 = (int)threadIdx.x - r * threads_per_row;
+  const uint32_t quad = 0xFu << (threadIdx.x & 28);               // four neighbouring 16-element blocks of one row
+  if (r >= rows_per_block) return;
+  const int64_t step = (int64_t)gridDim.x * rows_per_block;
+  pdl_wait();
+  for (int64_t row0 = (int64_t)blockIdx.x * rows_per_block + r; row0 < rows; row0 += step * kRowsInFlight)
+    for (int blk = blk0; blk < blocks_per_row; blk += threads_per_row) {
+      uint32_t w[kRowsInFlight][8];
+#pragma unroll
+      for (int i = 0; i < kRowsInFlight; ++i) {
+        const int64_t row = row0 + i * step;
+        if (row >= rows) break;
+        const __nv_bfloat16* src = x + row * row_stride + blk * 16;
+        if (WIDE) {
+          asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                       : "=r"(w[i][0]), "=r"(w[i][1]), "=r"(w[i][2]), "=r"(w[i][3]), "=r"(w[i][4]), "=r"(w[i][5]), "=r"(w[i][6]),
+                         "=r"(w[i][7])
+                       : "l"(src));
+        } else {
+          const uint4 lo = __ldg(reinterpret_cast<const uint4*>(src)), hi = __ldg(reinterpret_cast<const uint4*>(src) + 1);
+          w[i][0] = lo.x; w[i][1] = lo.y; w[i][2] = lo.z; w[i][3] = lo.w;
+          w[i][4] = hi.x; w[i][5] = hi.y; w[i][6] = hi.z; w[i][7] = hi.w;
         }
-        packed[h] = word;
+      }
+#pragma unroll
+      for (int i = 0; i < kRowsInFlight; ++i) {
+        const int64_t row = row0 + i * step;
+        if (row >= rows) break;
+        uint32_t packed[2];
+        const uint32_t sbyte = quantize_block<EXACT_DIV>(w[i], gs, rgs, table, packed);
+        *reinterpret_cast<uint2*>(payload + row * ((int64_t)blocks_per_row * 8) + (int64_t)blk * 8) = make_uint2(packed[0], packed[1]);
+        const size_t at = sf_layout == 0 ? (size_t)(row * blocks_per_row + blk) : sf_tiled_offset(row, blk, blocks_per_row >> 2);
+        if (word_scales) {
+          uint32_t word = sbyte << (8 * (blk & 3));
+          word |= __shfl_xor_sync(quad, word, 1);
+          word |= __shfl_xor_sync(quad, word, 2);
+          if ((blk & 3) == 0) *reinterpret_cast<uint32_t*>(scales + at) = word;
+        } else {
+          scales[at] = (uint8_t)sbyte;
+        }
       }
     }
-    *reinterpret_cast<uint2*>(payload + row * (cols >> 1) + (int64_t)blk * 8) = make_uint2(packed[0], packed[1]);
-    if (sf_layout == 0)
-      scales[row * blocks_per_row + blk] = (uint8_t)sbyte;
-    else
-      scales[sf_tiled_offset(row, blk, cols >> 6)] = (uint8_t)sbyte;
-  }
 }
 
 // Row-major scale bytes [rows, cols/16] -> 128x4 tiles; rows beyond `rows` up to the next multiple of 128 become 0.
@@ -107,20 +196,25 @@ __global__ void k_sf_to_tiles(const uint8_t* __restrict__ src, int64_t rows, int
 int launch_quantize_nvfp4(const void* x, int64_t rows, int64_t cols, int64_t row_stride, float gs, void* payload, void* scales,
                           int sf_layout, cudaStream_t st) {
   if (rows == 0) return 0;
-  const int bpr = (int)(cols >> 4);
-  // threads = blocks per row rounded up to a warp, split into equal passes of at most 256 threads
+  const int bpr = (int)(cols >> 4);                       // a multiple of 4
+  // threads of a row: its 16-element blocks in equal passes of at most 256, a multiple of 4; short rows share a block
   const int passes = (bpr + 255) / 256;
-  int threads = ((bpr + passes - 1) / passes + 31) / 32 * 32;
-  if (threads > 256) threads = 256;
-  const int64_t resident = (int64_t)sm_count() * 32;
-  const int64_t blocks = rows < resident ? rows : resident;
+  const int tpr = ((bpr + passes - 1) / passes + 3) / 4 * 4;
+  const int rpb = 256 / tpr;
+  const int threads = (rpb * tpr + 31) / 32 * 32;
+  const int64_t resident = (int64_t)sm_count() * (1024 / threads);       // one wave at 64 registers a thread
+  const int64_t want = (rows + rpb - 1) / rpb;
+  const int64_t blocks = want < resident ? want : resident;
   // stored * gs stays a normal number with room for the residual of a bf16 numerator inside 2^-40 .. 2^40
   const bool fast = gs >= 0x1p-40f && gs <= 0x1p40f;
-  if (fast)
-    return (int)launch_chain(k_quantize_nvfp4<false>, dim3((unsigned)blocks), dim3(threads), 0, st, (const __nv_bfloat16*)x, rows, cols,
-                             row_stride, gs, (uint8_t*)payload, (uint8_t*)scales, sf_layout);
-  return (int)launch_chain(k_quantize_nvfp4<true>, dim3((unsigned)blocks), dim3(threads), 0, st, (const __nv_bfloat16*)x, rows, cols,
-                           row_stride, gs, (uint8_t*)payload, (uint8_t*)scales, sf_layout);
+  const bool wide = ((uintptr_t)x & 31) == 0 && row_stride % 16 == 0;
+  const int word_scales = ((uintptr_t)scales & 3) == 0;
+  auto go = [&](auto kern) {
+    return (int)launch_chain(kern, dim3((unsigned)blocks), dim3(threads), 0, st, (const __nv_bfloat16*)x, rows, bpr, row_stride, gs,
+                             (uint8_t*)payload, (uint8_t*)scales, sf_layout, tpr, rpb, word_scales);
+  };
+  if (!fast) return go(k_quantize_nvfp4<true, false>);
+  return wide ? go(k_quantize_nvfp4<false, true>) : go(k_quantize_nvfp4<false, false>);
 }
 
 int launch_sf_to_tiles(const void* src, int64_t rows, int64_t blocks_per_row, void* dst, cudaStream_t st) {

@@ -68,7 +68,9 @@ def nvfp4_quantize(x: torch.Tensor, global_scale: float = 1.0, tiled_scales: boo
     else:
         payload = torch.empty((rows, cols // 2), dtype=torch.uint8, device=x.device)
         if tiled_scales:
-            scales = torch.zeros(((rows + 127) // 128, cols // 64, 32, 16), dtype=torch.uint8, device=x.device)
+            scales = torch.empty(((rows + 127) // 128, cols // 64, 32, 16), dtype=torch.uint8, device=x.device)
+            if rows % 128:
+                scales[-1].zero_()           # the kernel writes every row it has; only a ragged last tile holds others
         else:
             scales = torch.empty((rows, cols // 16), dtype=torch.uint8, device=x.device)
     lib = _lib.load()

@@ -48,6 +48,25 @@ def test_quantize_matches_oracle(rows, cols, scale):
         assert np.array_equal(ks.scales_to_tiles(ks.nvfp4_quantize(x.cuda())[1]).cpu().numpy(), ref_t)
 
 
+@pytest.mark.parametrize("rows,cols,pad,offset", [(1, 64, 0, 0), (9999, 64, 0, 0), (300, 192, 8, 1), (9500, 320, 0, 0), (130, 4160, 8, 0),
+                                                  (4800, 4096, 16, 3)])
+def test_quantize_short_rows_odd_strides_and_scale_alignment(rows, cols, pad, offset):
+    """Several rows per block, two rows per thread in flight, rows that start on 16- but not 32-byte boundaries, and scale
+    buffers on odd addresses, in both layouts."""
+    import kernelschema_b200 as ks
+    x = torch.randn(rows, cols + pad, generator=torch.Generator().manual_seed(rows)).to(torch.bfloat16)
+    oq, os_ = o.quantize(x[:, :cols].float().numpy(), 16, 0.0021)
+    for tiled in (False, True):
+        n = (rows + 127) // 128 * (cols // 64) * 512 if tiled else rows * (cols // 16)
+        q = torch.empty((rows, cols // 2), dtype=torch.uint8, device="cuda")
+        s = torch.zeros(n + 16, dtype=torch.uint8, device="cuda")
+        ks.nvfp4_quantize(x.cuda()[:, :cols], 0.0021, tiled_scales=tiled, out=(q, s[offset:offset + n]))
+        assert np.array_equal(q.cpu().numpy(), oq)
+        want = o.block_scales(os_[None])[0] if tiled else os_
+        assert np.array_equal(s[offset:offset + n].cpu().numpy(), want.reshape(-1))
+        assert not s[:offset].any() and not s[offset + n:].any()
+
+
 def _torch_quantize_true_division(x, gs):
     """The reference quantize() (gemm/dense/bf16_nvfp4_gemm/problem/input.py:40-64) in torch ops on the device with
     tensor / tensor divisions only (IEEE round-to-nearest; tensor / python-scalar would multiply by a reciprocal)."""
