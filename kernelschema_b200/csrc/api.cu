@@ -64,7 +64,8 @@ struct b200moe_layer {
   uint8_t *a_q, *a_sf, *act_q, *act_sf;
   __nv_bfloat16* rout;
   int32_t* status;
-  CUtensorMap tm_a1, tm_a2, tm_b1, tm_b2;
+  ActMaps tm_a1, tm_a2;
+  CUtensorMap tm_b1, tm_b2;
   CUtensorMap tm_b1_narrow, tm_b2_narrow;
   CUtensorMap tm_hid;                                 // the caller's token rows as FC1's A operand (TMA gather), box {128, 1}
   const void* hid_ptr;
@@ -196,6 +197,12 @@ int check_args(const b200moe_layer* h, const b200moe_args* a) {
   return 0;
 }
 
+int make_act_maps(ActMaps* m, const void* base, uint64_t rows, uint64_t row_bytes) {
+  int rc = make_operand_map(&m->rows128, base, rows, row_bytes, 128);
+  if (!rc) rc = make_operand_map(&m->rows64, base, rows, row_bytes, 64);
+  return rc ? rc : make_operand_map(&m->rows16, base, rows, row_bytes, 16);
+}
+
 struct EpRun {
   EpPeers peers;
   const int32_t* ctrl;     // this rank's control block of the step's parity
@@ -300,10 +307,10 @@ int run_impl(b200moe_layer* h, const b200moe_args* a, cudaStream_t st, cudaEvent
       gp.tile_row0 = h->rm.pair_row0;
       gp.tile_rows = h->rm.pair_rows;
       gp.n_tiles_ptr = h->rm.totals + 3;
-      rc = launch_gemm_nvfp4_pair(kGemmFc1, h->tm_a1, h->tm_b1, h->tm_sfa1, h->tm_sfb1, gp,
+      rc = launch_gemm_nvfp4_pair(kGemmFc1, h->tm_a1.rows128, h->tm_b1, h->tm_sfa1, h->tm_sfb1, gp,
                                   (int)(items < h->n_clusters ? items : h->n_clusters), st);
     } else {
-      rc = launch_gemm_nvfp4(kGemmFc1, bn, gather_a ? h->tm_hid : h->tm_a1, bn == h->bn ? h->tm_b1 : h->tm_b1_narrow, g, grid, st);
+      rc = launch_gemm_nvfp4(kGemmFc1, bn, gather_a ? ActMaps{h->tm_hid, h->tm_hid, h->tm_hid} : h->tm_a1, bn == h->bn ? h->tm_b1 : h->tm_b1_narrow, g, grid, st);
     }
     if (rc) return cuda_fail(rc, "FC1");
   }
@@ -332,7 +339,7 @@ int run_impl(b200moe_layer* h, const b200moe_args* a, cudaStream_t st, cudaEvent
       gp.tile_row0 = h->rm.pair_row0;
       gp.tile_rows = h->rm.pair_rows;
       gp.n_tiles_ptr = h->rm.totals + 3;
-      rc = launch_gemm_nvfp4_pair(kGemmFc2, h->tm_a2, h->tm_b2, h->tm_sfa2, h->tm_sfb2, gp,
+      rc = launch_gemm_nvfp4_pair(kGemmFc2, h->tm_a2.rows128, h->tm_b2, h->tm_sfa2, h->tm_sfb2, gp,
                                   (int)(items < h->n_clusters ? items : h->n_clusters), st);
     } else {
       rc = launch_gemm_nvfp4(kGemmFc2, bn, h->tm_a2, bn == h->bn ? h->tm_b2 : h->tm_b2_narrow, g, grid, st);
@@ -451,7 +458,7 @@ int b200moe_gemm_nvfp4(const void* a_q, const void* a_sf, const void* b_q, const
   }
   const int64_t items = (int64_t)g.n_tiles_static * (n / bn);
   const int grid = (int)(items < sms ? items : sms);
-  return cuda_fail(launch_gemm_nvfp4(kGemmDense, bn, ta, tb, g, grid, (cudaStream_t)stream), "gemm");
+  return cuda_fail(launch_gemm_nvfp4(kGemmDense, bn, ActMaps{ta, ta, ta}, tb, g, grid, (cudaStream_t)stream), "gemm");
 }
 
 int64_t b200moe_gemm_bf16_nvfp4_workspace_bytes(int64_t m, int64_t n, int64_t k) {
@@ -537,8 +544,8 @@ int b200moe_create(const b200moe_config* cfg, b200moe_handle* out) {
     delete h;
     return cuda_fail((int)e, "create: workspace clear");
   }
-  rc = make_operand_map(&h->tm_a1, h->a_q, (uint64_t)p.row_capacity, cfg->hidden / 2, 128);
-  if (!rc) rc = make_operand_map(&h->tm_a2, h->act_q, (uint64_t)p.row_capacity, cfg->intermediate / 2, 128);
+  rc = make_act_maps(&h->tm_a1, h->a_q, (uint64_t)p.row_capacity, cfg->hidden / 2);
+  if (!rc) rc = make_act_maps(&h->tm_a2, h->act_q, (uint64_t)p.row_capacity, cfg->intermediate / 2);
   if (!rc) rc = make_sf_map(&h->tm_sfa1, h->a_sf, (uint64_t)p.row_capacity / 128 * (cfg->hidden / 64));
   if (!rc) rc = make_sf_map(&h->tm_sfa2, h->act_sf, (uint64_t)p.row_capacity / 128 * (cfg->intermediate / 64));
   h->n_clusters = h->sm_count / 2;

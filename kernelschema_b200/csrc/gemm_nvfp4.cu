@@ -75,6 +75,27 @@ DEV float tanh_fast(float x) {
   return y;
 }
 
+// Per-expert multipliers and activation parameters of one work item, fetched before its accumulator is waited for.
+struct EpiScale {
+  float up, gate, alpha, beta, limit, out;
+};
+template <int MODE>
+DEV EpiScale load_scales(const GemmParams& p, int e) {
+  EpiScale s = {1.0f, 1.0f, 1.0f, 0.0f, 0.0f, 1.0f};
+  if (MODE == kGemmFc1) {
+    if (p.scale_up) s.up = __ldg(p.scale_up + e);
+    if (p.scale_gate) s.gate = __ldg(p.scale_gate + e);
+    if (p.alpha) s.alpha = __ldg(p.alpha + e);
+    if (p.beta) s.beta = __ldg(p.beta + e);
+    if (p.limit) s.limit = __ldg(p.limit + e);
+  } else if (MODE == kGemmFc2) {
+    if (p.out_scale) s.out = __ldg(p.out_scale + e);
+  } else {
+    s.out = p.dense_alpha;
+  }
+  return s;
+}
+
 // Epilogue of EC (64 or 128) accumulator columns [col0, col0 + EC) of one tile for the calling warp's 32 TMEM lanes.
 // The values are pulled into registers first and `release` is called right after the last TMEM read, so the
 // accumulator buffer is free again after a few hundred cycles and the arithmetic, the requantisation and the global
@@ -82,7 +103,7 @@ DEV float tanh_fast(float x) {
 // scheduler: the activation + requantisation chain is latency-bound with two, which shows when the k-loop of a tile is
 // short (K <= 2048: 8 stages, about 4 us); with a long k-loop the eight-warp form (EC = 128) hides it and draws less power.
 template <int MODE, int EC, class Release>
-DEV void epilogue_cols(const GemmParams& p, uint32_t taddr, int e, size_t row, bool live, int col0, Release release) {
+DEV void epilogue_cols(const GemmParams& p, uint32_t taddr, const EpiScale& sc, size_t row, bool live, int col0, Release release) {
   constexpr int NCB = EC / 32;
   // a warp whose 32 rows are all padding (decode: a few routes per expert) neither reads the accumulator nor computes
   if (!__any_sync(0xFFFFFFFFu, live)) {
@@ -95,12 +116,8 @@ DEV void epilogue_cols(const GemmParams& p, uint32_t taddr, int e, size_t row, b
   tmem_ld_wait();
   release();
   if (MODE == kGemmFc1) {
-    const float s_up = p.scale_up ? p.scale_up[e] : 1.0f;
-    const float s_gate = p.scale_gate ? p.scale_gate[e] : 1.0f;
-    const float alpha = p.alpha ? p.alpha[e] : 1.0f;
-    const float beta = p.beta ? p.beta[e] : 0.0f;
+    const float alpha = sc.alpha, beta = sc.beta, limit = sc.limit;
     const bool clamp = p.limit != nullptr;
-    const float limit = clamp ? p.limit[e] : 0.f;
     uint2 packed[NCB];
     uint32_t sfword = 0;
 #pragma unroll
@@ -111,8 +128,8 @@ DEV void epilogue_cols(const GemmParams& p, uint32_t taddr, int e, size_t row, b
       for (int c = 0; c < 2; ++c)
 #pragma unroll
         for (int b = 0; b < 8; ++b) {
-          float up = v[cb][16 * c + b] * s_up;
-          float gate = v[cb][16 * c + 8 + b] * s_gate;
+          float up = v[cb][16 * c + b] * sc.up;
+          float gate = v[cb][16 * c + 8 + b] * sc.gate;
           if (clamp) {
             up = fminf(fmaxf(up, -limit), limit);
             gate = fminf(gate, limit);
@@ -130,13 +147,10 @@ DEV void epilogue_cols(const GemmParams& p, uint32_t taddr, int e, size_t row, b
       const uint32_t sb = cvt_e4m3(sfv);
       const float sff = e4m3_to_f32(sb);
       const float inv = sff > 0.f ? __frcp_rn(sff) : 0.f;
-      uint32_t w0 = 0, w1 = 0;
+      float q[2][8];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        w0 |= cvt_e2m1x2(act[2 * j] * inv, act[2 * j + 1] * inv) << (8 * j);
-        w1 |= cvt_e2m1x2(act[8 + 2 * j] * inv, act[8 + 2 * j + 1] * inv) << (8 * j);
-      }
-      packed[cb] = make_uint2(w0, w1);
+      for (int j = 0; j < 16; ++j) q[j >> 3][j & 7] = act[j] * inv;
+      packed[cb] = make_uint2(cvt_e2m1x8(q[0]), cvt_e2m1x8(q[1]));
       sfword |= sb << (8 * cb);
     }
     if (live) {
@@ -159,7 +173,7 @@ DEV void epilogue_cols(const GemmParams& p, uint32_t taddr, int e, size_t row, b
     }
   } else {
     if (!live) return;
-    const float oscale = (MODE == kGemmFc2) ? (p.out_scale ? p.out_scale[e] : 1.0f) : p.dense_alpha;
+    const float oscale = sc.out;
     const size_t orow = (MODE == kGemmFc2 && p.out_row_index) ? (size_t)p.out_row_index[row] : row;
     __nv_bfloat16* dst_row = p.out + orow * p.out_stride + col0;
 #pragma unroll
@@ -234,7 +248,7 @@ DEV void copier_loop(const GemmParams& p, uint32_t tmem, uint32_t s_sfa, uint32_
 
 template <int MODE, int BN, int EC>
 __global__ void __launch_bounds__(gemm_threads<BN, EC>(), 1)
-k_gemm_nvfp4(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const GemmParams p) {
+k_gemm_nvfp4(const __grid_constant__ ActMaps am, const __grid_constant__ CUtensorMap tm_b, const GemmParams p) {
   using C = GemmCfg<BN>;
   constexpr int kEpiWarps = 4 * BN / EC;
   extern __shared__ uint8_t smem_raw[];
@@ -265,7 +279,7 @@ k_gemm_nvfp4(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
       mbar_init(bar_acc_empty + 8 * b, kEpiWarps);
     }
     mbar_init_fence();
-    tma_prefetch_desc(&tm_a);
+    tma_prefetch_desc(&am.rows128);
     tma_prefetch_desc(&tm_b);
   }
   if (warp == 1) tmem_alloc<512>(s_tmem_slot);
@@ -324,7 +338,7 @@ k_gemm_nvfp4(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
           const uint32_t full = bar_full + 8 * s;
           if (lane == 0) mbar_expect_tx(full, stage_bytes);
           __syncwarp();
-          if (lane < nbox) tma_gather4(s_a + s * C::kABytes + 512u * lane, &tm_a, full, ks * 128, tok.x, tok.y, tok.z, tok.w);
+          if (lane < nbox) tma_gather4(s_a + s * C::kABytes + 512u * lane, &am.rows128, full, ks * 128, tok.x, tok.y, tok.z, tok.w);
           if (lane == 0) {
             tma_load_2d(s_b + s * C::kBBytes, &tm_b, full, ks * 128, brow0);
             bulk_load_1d(s_sfa + s * C::kSfaBytes, sfa_src + (size_t)ks * 4 * kSfChunk, 4 * kSfChunk, full);
@@ -341,28 +355,31 @@ k_gemm_nvfp4(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
       uint32_t s = 0, ph = 1;
       bool ok = true;
       // the tile-table entries of an item are fetched one item ahead, so their latency hides behind a whole k-loop
-      int mt_n = 0, e_n = 0, row0_n = 0;
-      if (blockIdx.x < total_items) {
-        mt_n = (int)(blockIdx.x / n_ntiles);
+      int mt_n = 0, e_n = 0, row0_n = 0, rows_n = kBM;
+      auto fetch = [&](long long item) {
+        mt_n = (int)(item / n_ntiles);
         e_n = p.tile_expert ? p.tile_expert[mt_n] : 0;
         row0_n = p.tile_row0 ? p.tile_row0[mt_n] : mt_n * kBM;
-      }
+        rows_n = p.tile_rows ? p.tile_rows[mt_n] : kBM;
+      };
+      if (blockIdx.x < total_items) fetch(blockIdx.x);
       for (long long item = blockIdx.x; ok && item < total_items; item += gridDim.x) {
         const int nt = (int)(item - (long long)mt_n * n_ntiles);
-        const int e = e_n, row0 = row0_n;
-        if (item + gridDim.x < total_items) {
-          mt_n = (int)((item + gridDim.x) / n_ntiles);
-          e_n = p.tile_expert ? p.tile_expert[mt_n] : 0;
-          row0_n = p.tile_row0 ? p.tile_row0[mt_n] : mt_n * kBM;
-        }
+        const int e = e_n, row0 = row0_n, rows = rows_n;
+        if (item + gridDim.x < total_items) fetch(item + gridDim.x);
+        // A tile with few rows fetches a box of 16 or 64: the rest of its slot keeps old bytes, whose products stay in rows
+        // that are never stored. (Of a decode batch's segments most rows are padding that somebody would have to read.)
+        const CUtensorMap* tm_a = rows <= 16 ? &am.rows16 : rows <= 64 ? &am.rows64 : &am.rows128;
+        const uint32_t a_rows = rows <= 16 ? 16u : rows <= 64 ? 64u : (uint32_t)kBM;
+        const uint32_t stage_bytes = C::kStageBytes - C::kABytes + a_rows * 128u;
         const int brow0 = e * p.N + nt * BN;
         const uint8_t* sfa_src = p.sfa + (size_t)(row0 >> 7) * chunks_per_row * kSfChunk;
         const uint8_t* sfb_src = p.sfb + (size_t)(brow0 >> 7) * chunks_per_row * kSfChunk;
         for (int ks = 0; ks < nk; ++ks) {
           if (!mbar_wait(bar_empty + 8 * s, ph)) { report(p.status, 101); ok = false; break; }
           const uint32_t full = bar_full + 8 * s;
-          mbar_expect_tx(full, C::kStageBytes);
-          tma_load_2d(s_a + s * C::kABytes, &tm_a, full, ks * 128, row0);
+          mbar_expect_tx(full, stage_bytes);
+          tma_load_2d(s_a + s * C::kABytes, tm_a, full, ks * 128, row0);
           tma_load_2d(s_b + s * C::kBBytes, &tm_b, full, ks * 128, brow0);
           bulk_load_1d(s_sfa + s * C::kSfaBytes, sfa_src + (size_t)ks * 4 * kSfChunk, 4 * kSfChunk, full);
 #pragma unroll
@@ -431,6 +448,7 @@ k_gemm_nvfp4(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
       const int e = p.tile_expert ? p.tile_expert[mt] : 0;
       const int row0 = p.tile_row0 ? p.tile_row0[mt] : mt * kBM;
       const int rows = p.tile_rows ? p.tile_rows[mt] : min(kBM, p.M - row0);
+      const EpiScale sc = load_scales<MODE>(p, e);
       const uint32_t buf = it % C::kAccBufs;
       int okw = 1;
       if (lane == 0) okw = mbar_wait(bar_acc_full + 8 * buf, (it / C::kAccBufs) & 1) ? 1 : 0;
@@ -438,7 +456,7 @@ k_gemm_nvfp4(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
       if (!okw) { if (lane == 0) report(p.status, 104); break; }
       tc_fence_after();
       const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + buf * BN + group * EC;
-      epilogue_cols<MODE, EC>(p, taddr, e, (size_t)row0 + r_in_tile, r_in_tile < rows, nt * BN + group * EC, [&]() {
+      epilogue_cols<MODE, EC>(p, taddr, sc, (size_t)row0 + r_in_tile, r_in_tile < rows, nt * BN + group * EC, [&]() {
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_acc_empty + 8 * buf);
@@ -627,13 +645,14 @@ k_gemm_nvfp4_pair(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       const int row0 = (p.tile_row0 ? p.tile_row0[mt] : mt * 256) + (int)rank * 128;
       const int pair_rows = p.tile_rows ? p.tile_rows[mt] : min(256, p.M - mt * 256);
       const int rows = min(128, max(0, pair_rows - (int)rank * 128));
+      const EpiScale sc = load_scales<MODE>(p, e);
       int okw = 1;
       if (lane == 0) okw = mbar_wait_cluster(bar_acc_full, it & 1) ? 1 : 0;
       okw = __shfl_sync(0xFFFFFFFFu, okw, 0);
       if (!okw) { if (lane == 0) report(p.status, 204); break; }
       tc_fence_after();
       const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + group * 64;
-      epilogue_cols<MODE, 64>(p, taddr, e, (size_t)row0 + r_in_tile, r_in_tile < rows, nt * BN + group * 64, [&]() {
+      epilogue_cols<MODE, 64>(p, taddr, sc, (size_t)row0 + r_in_tile, r_in_tile < rows, nt * BN + group * 64, [&]() {
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_remote(acc_empty_leader);
@@ -715,7 +734,7 @@ int launch_gemm_nvfp4_pair(int mode, const CUtensorMap& ta, const CUtensorMap& t
 }
 
 template <int MODE, int BN, int EC>
-static int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int grid, cudaStream_t st) {
+static int launch_one(const ActMaps& ta, const CUtensorMap& tb, const GemmParams& p, int grid, cudaStream_t st) {
   auto kern = k_gemm_nvfp4<MODE, BN, EC>;
   static SmemOptIn opt_in;
   if (int e = opt_in.ensure(kern, GemmCfg<BN>::kSmemBytes)) return e;
@@ -729,14 +748,14 @@ static int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const GemmPa
 static int epilogue_cols_for(int k, int64_t rows_hint) { return (k >= 4096 && (rows_hint == 0 || rows_hint > 8192)) ? 128 : 64; }
 
 template <int MODE>
-static int launch_mode(int bn, const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int grid, cudaStream_t st) {
+static int launch_mode(int bn, const ActMaps& ta, const CUtensorMap& tb, const GemmParams& p, int grid, cudaStream_t st) {
   const int ec = epilogue_cols_for(p.K, p.rows_hint);
   if (bn == 128) return ec == 64 ? launch_one<MODE, 128, 64>(ta, tb, p, grid, st) : launch_one<MODE, 128, 128>(ta, tb, p, grid, st);
   if (bn == 256) return ec == 64 ? launch_one<MODE, 256, 64>(ta, tb, p, grid, st) : launch_one<MODE, 256, 128>(ta, tb, p, grid, st);
   return 703;
 }
 
-int launch_gemm_nvfp4(int mode, int bn, const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int grid,
+int launch_gemm_nvfp4(int mode, int bn, const ActMaps& ta, const CUtensorMap& tb, const GemmParams& p, int grid,
                       cudaStream_t st) {
   if (grid <= 0) return 0;
   if (p.K % kStageK != 0 || p.N % bn != 0) return 702;

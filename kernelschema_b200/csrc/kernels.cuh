@@ -116,7 +116,7 @@ int launch_router_logits_small(const void* x, const void* w, int64_t T, int H, i
 // slots of each region hold a token (the receive buffer of the expert-parallel exchange); the rest count as unrouted.
 int launch_route_map(const int32_t* ids, const float* scores, int64_t id_stride, int64_t T, int K, int S, int E, int expert_offset,
                      RouteMapBuffers b, cudaStream_t st, int seg_len = 0, const int32_t* seg_valid = nullptr);
-// Route map and permute in ONE launch for batches of at most 8192 routes with row-major token scales (decode sizes):
+// Route map and permute in ONE launch for batches of at most 16384 routes with row-major token scales (decode sizes):
 // `route_gather_fits` says whether a call qualifies.
 bool route_gather_fits(int64_t T, int K, int S, int E, int H);
 int launch_route_gather(const int32_t* ids, const float* scores, int64_t id_stride, int64_t T, int K, int S, int E, int expert_offset,
@@ -166,7 +166,11 @@ int launch_finalize_ep(const void* rout, const int32_t* row_of, const float* wei
                        const EpPeers& peers, const int32_t* ctrl, int seg_len, cudaStream_t st);
 int launch_gemm_nvfp4_pair(int mode, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tsa, const CUtensorMap& tsb,
                            const GemmParams& p, int n_clusters, cudaStream_t st);
-int launch_gemm_nvfp4(int mode, int bn, const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int grid,
+// A-operand maps with 128-, 64- and 16-row boxes (dense and TMA-gathered launches use the first only).
+struct ActMaps {
+  CUtensorMap rows128, rows64, rows16;
+};
+int launch_gemm_nvfp4(int mode, int bn, const ActMaps& ta, const CUtensorMap& tb, const GemmParams& p, int grid,
                       cudaStream_t st);
 
 }  // namespace b200
