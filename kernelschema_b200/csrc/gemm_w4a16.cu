@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(256) k_w4a16_reduce(const float* __restrict__ 
 
 // Split-K plan for small M: enough CTAs per output tile to occupy the device; 1 = no split (no workspace needed).
 static int w4a16_splits(int64_t m, int64_t n, int64_t k, int sms) {
-  if (m > 128) return 1;
+  if (m > 128 || w4a16_decode_fits(m)) return 1;
   const int64_t tiles = n / 128, groups = k / 256;
   int64_t s = sms / tiles;
   if (s > 8) s = 8;
@@ -383,6 +383,7 @@ int launch_gemm_w4a16(const void* a, int64_t a_stride, const void* b_q, const vo
                       int64_t k, void* out, int64_t out_stride, void* workspace, int64_t workspace_bytes, int32_t* status,
                       cudaStream_t st) {
   if (m == 0) return 0;
+  if (w4a16_decode_fits(m)) return launch_gemm_w4a16_decode(a, a_stride, b_q, b_sf, alpha, m, n, k, out, out_stride, st);
   const int bn = (n % 256 == 0 && m > 128) ? 256 : 128;
   CUtensorMap ta;
   int rc = make_operand_map(&ta, a, (uint64_t)m, (uint64_t)k * 2, 256, (uint64_t)a_stride * 2);

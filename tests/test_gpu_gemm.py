@@ -153,6 +153,33 @@ def test_w4a16_matches_oracle(m, n, k, outliers):
     assert (o.bf16_bits(got) != o.bf16_bits(ref)).mean() <= 0.05
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 128, 256), (7, 384, 2304), (8, 4096, 12288), (9, 1024, 4096), (16, 8192, 512), (17, 256, 2048),
+                                   (31, 7168, 768), (32, 128, 12288)])
+def test_w4a16_decode_sizes_all_codes(m, n, k):
+    """A handful of tokens: every code and every scale byte (subnormal scales and the 0.5 code among them) in random places,
+    a strided A, and rows beyond M left alone. Sums of K products differ from the oracle's only by the order of the fp32
+    additions, so a bf16 step (2^-8) of the result plus 2^-20 of the sum of magnitudes bounds every element."""
+    import kernelschema_b200 as ks
+    rng = np.random.default_rng(m + n + k)
+    wide = torch.zeros((m, k + 8), dtype=torch.bfloat16, device="cuda")
+    a = o.bf16_round(rng.standard_normal((m, k), dtype=np.float32))
+    wide[:, :k] = _bf16_dev(a)
+    bq = rng.integers(0, 256, (n, k // 2), dtype=np.uint8)
+    bsf = rng.integers(0, 0x7F, (n, k // 16), dtype=np.uint8)
+    backing = torch.full((m + 2, n), -17.0, dtype=torch.bfloat16, device="cuda")
+    out = ks.mm_bf16_nvfp4(wide[:, :k], torch.from_numpy(bq).cuda(), torch.from_numpy(bsf).cuda(),
+                           torch.tensor([0.5], dtype=torch.float32, device="cuda"), out=backing[1:m + 1])
+    torch.cuda.synchronize()
+    assert (backing[0] == -17).all() and (backing[m + 1] == -17).all()
+    codes = np.array([0, 0.5, 1, 1.5, 2, 3, 4, 6, -0.0, -0.5, -1, -1.5, -2, -3, -4, -6], dtype=np.float64)
+    w = np.empty((n, k))
+    w[:, 0::2], w[:, 1::2] = codes[bq & 15], codes[bq >> 4]
+    scale = torch.arange(256, dtype=torch.int32).to(torch.uint8).view(torch.float8_e4m3fn).double().numpy()[bsf]
+    w *= np.repeat(scale, 16, axis=1)
+    ref, mag = 0.5 * a.astype(np.float64) @ w.T, 0.5 * np.abs(a).astype(np.float64) @ np.abs(w).T
+    assert (np.abs(out.float().cpu().numpy() - ref) <= np.abs(ref) / 256 + mag * 2.0 ** -20).all()
+
+
 def test_w4a16_strided_a_and_no_alpha():
     import kernelschema_b200 as ks
     a, bq, bsf = _w4a16_case(64, 128, 512, 7)
