@@ -112,16 +112,28 @@ int launch_router_logits_tc(const void* x, const void* w, int64_t T, int H, int 
 // memory. Returns -1 when the shape does not qualify (the caller then uses launch_router_logits_tc).
 int launch_router_logits_ksplit(const void* x, const void* w, int64_t T, int H, int E, float* logits, int32_t* status, cudaStream_t st);
 int launch_router_logits_small(const void* x, const void* w, int64_t T, int H, int E, float* logits, cudaStream_t st);   // T <= 16
+// Router logits and quantiser of T <= 8 contiguous token rows in one launch (row-major scales, global scale in quantize_fast's range).
+int launch_front_small(const void* x, const void* w, int64_t T, int H, int E, float* logits, float gs, void* payload, void* scales,
+                       cudaStream_t st);
 // seg_len > 0: the T token slots are regions of seg_len consecutive slots and only the first seg_valid[slot / seg_len]
 // slots of each region hold a token (the receive buffer of the expert-parallel exchange); the rest count as unrouted.
 int launch_route_map(const int32_t* ids, const float* scores, int64_t id_stride, int64_t T, int K, int S, int E, int expert_offset,
                      RouteMapBuffers b, cudaStream_t st, int seg_len = 0, const int32_t* seg_valid = nullptr);
 // Route map and permute in ONE launch for batches of at most 16384 routes with row-major token scales (decode sizes):
 // `route_gather_fits` says whether a call qualifies.
+// With `topk` the expert ids come from router logits inside the launch (T <= kTopkGatherTokens, E <= 256); `ids` / `scores` are
+// then unused and the selection is also stored to topk->ids / topk->weights.
+constexpr int kTopkGatherTokens = 8;
+struct TopkView {
+  const float* logits;
+  const float* bias;
+  int32_t* ids;
+  float* weights;
+};
 bool route_gather_fits(int64_t T, int K, int S, int E, int H);
 int launch_route_gather(const int32_t* ids, const float* scores, int64_t id_stride, int64_t T, int K, int S, int E, int expert_offset,
                         RouteMapBuffers b, const void* hid_q, const void* hid_sf, int64_t q_stride, int64_t sf_stride, int H, void* a_q,
-                        void* a_sf, cudaStream_t st, int seg_len = 0, const int32_t* seg_valid = nullptr);
+                        void* a_sf, cudaStream_t st, int seg_len = 0, const int32_t* seg_valid = nullptr, const TopkView* topk = nullptr);
 int launch_route_map_static(const int32_t* ids, const float* scores, int64_t T, int K, int S, int E, int expert_offset,
                             RouteMapBuffers b, cudaStream_t st);
 int launch_ep_visits(const int32_t* ids, int64_t T, int K, int experts_per_rank, int world, int32_t* rank_slots, cudaStream_t st);

@@ -9,6 +9,7 @@
 // No atomics: three passes (block histograms, scan, stable scatter).
 #include "kernels.cuh"
 #include "ptx.cuh"
+#include "topk.cuh"
 
 namespace b200 {
 
@@ -484,10 +485,14 @@ __global__ void __launch_bounds__(kRouteThreads) k_route_fused(RouteView r, cons
 // warps copy its rows. Building the whole ranked map in every block instead costs eight dependent ranking rounds at 8192
 // routes and 32 warps' histograms to zero, sum and scan. Layer call at T = 1024, H = 7168, 256 experts (this launch took 37 us
 // of it): 249 -> 234 us; at 14 216 routes, H = 2048 (route map and permute were two launches, 28 us): 118 -> 110 us.
-template <int OW>                                  // warps that own routes
-__global__ void __launch_bounds__(kRouteThreads) k_route_gather(RouteView r, const float* __restrict__ scores, int etot, int chunk,
-                                                               RouteMapBuffers b, GatherView gv) {
+// TOPK: a decode batch straight from router logits (one token per warp, at most 256 experts): every block selects the experts of
+// all tokens itself, block 0 stores them.
+template <int OW, bool TOPK>                       // OW = warps that own routes
+__global__ void __launch_bounds__(TOPK ? 256 : kRouteThreads) k_route_gather(RouteView r, const float* scores, int etot,
+                                                                            int chunk, RouteMapBuffers b, GatherView gv, TopkView tk) {
   extern __shared__ int hist[];                    // own routes [OW][etot] | routes after [etot] | before [etot] | own positions [OW * 32]
+  __shared__ int32_t s_ids[TOPK ? kTopkGatherTokens * 32 : 1];
+  __shared__ float s_wts[TOPK ? kTopkGatherTokens * 32 : 1];
   int* after = hist + OW * etot;
   int* before = after + etot;
   int* s_pos = before + etot;
@@ -499,6 +504,25 @@ __global__ void __launch_bounds__(kRouteThreads) k_route_gather(RouteView r, con
   for (int i = threadIdx.x; i < (OW + 2) * etot; i += blockDim.x) hist[i] = 0;
   __syncthreads();
   pdl_wait();
+  if (TOPK) {
+    if (warp < r.T) {
+      int id;
+      float w;
+      topk_token<8>(tk.logits + (int64_t)warp * r.E, tk.bias, r.E, r.K, lane, id, w);
+      if (lane < r.K) {
+        s_ids[warp * r.K + lane] = id;
+        s_wts[warp * r.K + lane] = w;
+        if (blockIdx.x == 0) {
+          tk.ids[warp * r.K + lane] = id;
+          tk.weights[warp * r.K + lane] = w;
+        }
+      }
+    }
+    __syncthreads();
+    r.ids = s_ids;
+    r.id_stride = r.K;
+    scores = s_wts;
+  }
   const bool flat = r.S == 0 && r.id_stride == r.K && r.seg_len <= 0;      // route f's expert is ids[f]: no division
   const int f_own = lo + warp * 32 + lane;
   const int e_own = warp < OW && f_own < hi ? route_expert32(r, f_own, total) : -1;
@@ -581,24 +605,27 @@ bool route_gather_fits(int64_t T, int K, int S, int E, int H) {
 
 int launch_route_gather(const int32_t* ids, const float* scores, int64_t id_stride, int64_t T, int K, int S, int E, int expert_offset,
                         RouteMapBuffers b, const void* hid_q, const void* hid_sf, int64_t q_stride, int64_t sf_stride, int H, void* a_q,
-                        void* a_sf, cudaStream_t st, int seg_len, const int32_t* seg_valid) {
+                        void* a_sf, cudaStream_t st, int seg_len, const int32_t* seg_valid, const TopkView* topk) {
   const int etot = E + S;
   const int64_t total = T * (K + S);
   RouteView r{ids, id_stride > 0 ? id_stride : K, T, K, S, E, expert_offset, seg_valid ? seg_len : 0, seg_valid};
   GatherView gv{(const uint8_t*)hid_q, (const uint8_t*)hid_sf, q_stride > 0 ? q_stride : (int64_t)(H / 2),
                 sf_stride > 0 ? sf_stride : (int64_t)(H / 16), H, (uint8_t*)a_q, (uint8_t*)a_sf};
   // a handful of routes: a small block, whose barriers and zeroing cost less (T = 1: 2 us per step)
-  const int threads = total <= 256 ? 256 : kRouteThreads;
+  if (topk && (T > kTopkGatherTokens || E > 256)) return 704;
+  const int threads = total <= 256 || topk ? 256 : kRouteThreads;
   const int blocks = route_gather_blocks(total, threads);
   const int chunk = (int)((total + blocks - 1) / blocks);
   auto go = [&](auto kern, int ow) {               // at most (8 + 2) x 1024 counters + 256 positions: 41 KB
     return (int)launch_chain(kern, dim3((unsigned)((total + chunk - 1) / chunk)), dim3(threads),
-                             sizeof(int) * ((ow + 2) * (size_t)etot + 32 * (size_t)ow), st, r, scores, etot, chunk, b, gv);
+                             sizeof(int) * ((ow + 2) * (size_t)etot + 32 * (size_t)ow), st, r, scores, etot, chunk, b, gv,
+                             topk ? *topk : TopkView{});
   };
-  if (chunk <= 32) return go(k_route_gather<1>, 1);
-  if (chunk <= 64) return go(k_route_gather<2>, 2);
-  if (chunk <= 128) return go(k_route_gather<4>, 4);
-  return go(k_route_gather<8>, 8);
+  if (topk) return go(k_route_gather<1, true>, 1);       // at most 8 x 64 routes over blocks of 8
+  if (chunk <= 32) return go(k_route_gather<1, false>, 1);
+  if (chunk <= 64) return go(k_route_gather<2, false>, 2);
+  if (chunk <= 128) return go(k_route_gather<4, false>, 4);
+  return go(k_route_gather<8, false>, 8);
 }
 
 // ----------------------------------------------------------------------------- allocation-free variant

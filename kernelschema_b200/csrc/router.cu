@@ -7,21 +7,11 @@
 // One warp per token; each lane keeps E/32 logits in registers.
 #include "kernels.cuh"
 #include "ptx.cuh"
+#include "quantize.cuh"
+#include "topk.cuh"
 
 namespace b200 {
 
-// fp32 -> unsigned key in the same order; -inf and NaN, which are never selected, become 0 (every other key is larger) and
-// both zeros share a key.
-DEV uint32_t logit_key(float x) {
-  if (!(x > -INFINITY)) return 0u;
-  const uint32_t u = __float_as_uint(x + 0.0f);
-  return u ^ (u >> 31 ? 0xFFFFFFFFu : 0x80000000u);
-}
-DEV float key_logit(uint32_t k) { return k ? __uint_as_float(k ^ (k >> 31 ? 0x80000000u : 0xFFFFFFFFu)) : -INFINITY; }
-
-// PL = logits kept per lane (experts <= 32 * PL); the loops are unrolled for the instantiated size only. The K selection rounds
-// are a serial chain, so each is two warp-wide reductions (largest key, then lowest expert that has it) instead of five
-// exchange steps of (value, index) pairs.
 template <int PL>
 __global__ void __launch_bounds__(256) k_route_topk(const float* __restrict__ logits, const float* __restrict__ bias, int64_t T,
                                                     int E, int K, int32_t* __restrict__ ids, float* __restrict__ weights) {
@@ -30,49 +20,12 @@ __global__ void __launch_bounds__(256) k_route_topk(const float* __restrict__ lo
   pdl_trigger();
   pdl_wait();
   if (tok >= T) return;
-  uint32_t v[PL];
-#pragma unroll
-  for (int i = 0; i < PL; ++i) {
-    const int e = i * 32 + lane;
-    float x = -INFINITY;
-    if (e < E) {
-      x = logits[tok * E + e];
-      if (bias) x = __fadd_rn(x, bias[e]);
-    }
-    v[i] = logit_key(x);
-  }
-  float sel = 0.f;      // lane k keeps the k-th selected logit
-  int sel_id = -1;
-  uint32_t mine = 0;    // largest key of this lane
-#pragma unroll
-  for (int i = 0; i < PL; ++i) mine = max(mine, v[i]);
-  for (int k = 0; k < K; ++k) {
-    const uint32_t best = __reduce_max_sync(0xFFFFFFFFu, mine);
-    uint32_t at = 0x7FFFFFFFu;
-    if (mine == best && best != 0u) {
-#pragma unroll
-      for (int i = PL - 1; i >= 0; --i)
-        if (v[i] == best) at = (uint32_t)(i * 32 + lane);
-    }
-    const int best_e = (int)__reduce_min_sync(0xFFFFFFFFu, at);
-    if (lane == k) { sel = key_logit(best); sel_id = best_e; }
-    if (at == (uint32_t)best_e && best != 0u) {      // the owner takes it out
-      mine = 0;
-#pragma unroll
-      for (int i = 0; i < PL; ++i) {
-        if (i * 32 + lane == best_e) v[i] = 0u;
-        mine = max(mine, v[i]);
-      }
-    }
-  }
-  const float top = __shfl_sync(0xFFFFFFFFu, sel, 0);
-  double ex = (lane < K) ? exp((double)sel - (double)top) : 0.0;
-  double sum = ex;
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, off);
+  int id;
+  float weight;
+  topk_token<PL>(logits + tok * E, bias, E, K, lane, id, weight);
   if (lane < K) {
-    ids[tok * K + lane] = sel_id;
-    weights[tok * K + lane] = (float)(ex / sum);
+    ids[tok * K + lane] = id;
+    weights[tok * K + lane] = weight;
   }
 }
 
@@ -124,14 +77,12 @@ __global__ void __launch_bounds__(256) k_router_logits(const __nv_bfloat16* __re
 // = 2 experts x 4 quarters of H (one warp each), every warp reads its part of the weight row once and keeps one fp32
 // accumulator per token; the four partial sums of an expert are added in a fixed order (reproducible).
 template <int TT>
-__global__ void __launch_bounds__(256) k_router_logits_small(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
-                                                             int T, int H, int E, float* __restrict__ logits) {
+DEV void logits_small(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, int T, int H, int E,
+                      float* __restrict__ logits) {
   __shared__ float part_sum[4][2][TT];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int el = warp >> 2, part = warp & 3;
   const int e = blockIdx.x * 2 + el;
-  pdl_trigger();
-  pdl_wait();
   float acc[TT];
 #pragma unroll
   for (int t = 0; t < TT; ++t) acc[t] = 0.f;
@@ -174,6 +125,49 @@ __global__ void __launch_bounds__(256) k_router_logits_small(const __nv_bfloat16
     const int eg = blockIdx.x * 2 + ee;
     if (t < T && eg < E) logits[(int64_t)t * E + eg] = ((part_sum[0][ee][t] + part_sum[1][ee][t]) + part_sum[2][ee][t]) + part_sum[3][ee][t];
   }
+}
+
+template <int TT>
+__global__ void __launch_bounds__(256) k_router_logits_small(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+                                                             int T, int H, int E, float* __restrict__ logits) {
+  pdl_trigger();
+  pdl_wait();
+  logits_small<TT>(x, w, T, H, E, logits);
+}
+
+// The two kernels that read a decode batch's tokens in one launch (at T = 1 a launch costs more than either): the first
+// (E + 1) / 2 blocks compute router logits, the others quantise one token each.
+__global__ void __launch_bounds__(256) k_front_small(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, int T, int H,
+                                                     int E, float* __restrict__ logits, float gs, uint8_t* __restrict__ payload,
+                                                     uint8_t* __restrict__ scales) {
+  __shared__ ScaleRow table[128];
+  pdl_trigger();
+  const int router_blocks = (E + 1) / 2;
+  if ((int)blockIdx.x < router_blocks) {
+    pdl_wait();
+    logits_small<8>(x, w, T, H, E, logits);
+    return;
+  }
+  fill_scale_table(table, gs);
+  __syncthreads();
+  pdl_wait();
+  const int64_t row = (int)blockIdx.x - router_blocks;
+  const float rgs = __frcp_rn(gs);
+  const int blocks_per_row = H >> 4;
+  for (int blk = threadIdx.x; blk < blocks_per_row; blk += blockDim.x) {
+    const uint4* src = reinterpret_cast<const uint4*>(x + row * H + blk * 16);
+    const uint4 lo = __ldg(src), hi = __ldg(src + 1);
+    const uint32_t v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+    uint32_t packed[2];
+    scales[row * blocks_per_row + blk] = (uint8_t)quantize_block<false>(v, gs, rgs, table, packed);
+    *reinterpret_cast<uint2*>(payload + row * (H >> 1) + (int64_t)blk * 8) = make_uint2(packed[0], packed[1]);
+  }
+}
+
+int launch_front_small(const void* x, const void* w, int64_t T, int H, int E, float* logits, float gs, void* payload, void* scales,
+                       cudaStream_t st) {
+  return (int)launch_chain(k_front_small, dim3((unsigned)((E + 1) / 2 + T)), dim3(256), 0, st, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
+                           (int)T, H, E, logits, gs, (uint8_t*)payload, (uint8_t*)scales);
 }
 
 int launch_router_logits_small(const void* x, const void* w, int64_t T, int H, int E, float* logits, cudaStream_t st) {

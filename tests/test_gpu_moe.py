@@ -283,6 +283,34 @@ def test_library_graph_cache_and_hot_call():
     cached.close()
 
 
+@pytest.mark.parametrize("t,h,e,k,s", [(1, 512, 16, 4, 0), (3, 512, 255, 10, 1), (8, 512, 256, 32, 2), (9, 512, 16, 4, 1), (8, 4608, 16, 4, 1),
+                                       (4, 8192, 17, 17, 0), (8, 256, 300, 3, 0)])
+def test_step_of_a_handful_of_tokens_equals_separate_calls(t, h, e, k, s):
+    """Up to eight tokens share a launch for router logits and quantiser (while T x H <= 32768) and select their experts inside
+    the route-map launch (up to 256 experts); both edges, and the forms beyond them."""
+    import kernelschema_b200 as ks
+    i = 256
+    gen = torch.Generator(device="cuda").manual_seed(t + h + e)
+    rand = lambda *shape: torch.randn(shape, device="cuda", generator=gen)
+    x, gate, bias, gs = rand(t, h).to(torch.bfloat16), (rand(e, h) * 0.05).to(torch.bfloat16), rand(e) * 0.1, 0.0021
+    bias[1] = float("-inf")                                  # never selected
+    w1, s1 = ks.nvfp4_quantize((rand((e + s) * 2 * i, h) * 0.02).to(torch.bfloat16), 1.0, tiled_scales=True)
+    w2, s2 = ks.nvfp4_quantize((rand((e + s) * h, i) * 0.02).to(torch.bfloat16), 1.0, tiled_scales=True)
+    w1, w2 = w1.view(e + s, 2 * i, h // 2), w2.view(e + s, h, i // 2)
+    s1, s2 = s1.view(e + s, 2 * i, h // 16), s2.view(e + s, h, i // 16)
+    hq, hs = ks.nvfp4_quantize(x, gs)
+    ids, wt = ks.route_topk(ks.router_logits(x, gate), k, bias)
+    want, out = torch.empty_like(x), torch.empty_like(x)
+    ref_layer = ks.MoELayer(h, i, e, k, t, num_shared_experts=s)
+    ref_layer.run(ids, wt, hq, hs.view(torch.uint8), w1, s1, w2, s2, want)
+    layer = ks.MoELayer(h, i, e, k, t, num_shared_experts=s)
+    layer.step(x, gate, bias, gs, w1, s1, w2, s2, out)
+    torch.cuda.synchronize()
+    got = layer.step_outputs(t)
+    assert torch.equal(got["ids"], ids) and torch.equal(got["weights"], wt)
+    assert torch.equal(out, want) and layer.status() == 0
+
+
 @pytest.mark.parametrize("t,graph", [(200, False), (200, True), (1, True), (16, True), (2500, False), (2500, True)])
 def test_whole_step_entry_equals_separate_calls(t, graph):
     """b200moe_step (bf16 tokens -> quantiser -> router logits -> top-k -> layer in one library call) against the same
