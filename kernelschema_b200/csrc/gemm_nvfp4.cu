@@ -69,6 +69,25 @@ DEV void report(int32_t* status, int code) {
 }
 
 DEV float sigmoid_fast(float x) { return __frcp_rn(1.0f + __expf(-x)); }
+DEV float ex2_fast(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+DEV float rcp_fast(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// Two sigmoids in packed arithmetic. One Newton-Raphson step brings the approximate reciprocal of d = 1 + e^-x to within an ulp
+// of the rounded one, without the range test and branch of a general reciprocal; an infinite d keeps its reciprocal of 0.
+DEV float2 sigmoid2(float2 x) {
+  const float2 u = mul2(x, make_float2(-1.442695041f, -1.442695041f));                   // -x / ln 2
+  const float2 d = add2(make_float2(ex2_fast(u.x), ex2_fast(u.y)), make_float2(1.0f, 1.0f));
+  const float2 r = make_float2(rcp_fast(d.x), rcp_fast(d.y));
+  const float2 e = fma2(make_float2(-fminf(d.x, 3e38f), -fminf(d.y, 3e38f)), r, make_float2(1.0f, 1.0f));
+  return fma2(r, e, r);
+}
 DEV float tanh_fast(float x) {
   float y;
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -117,30 +136,34 @@ DEV void epilogue_cols(const GemmParams& p, uint32_t taddr, const EpiScale& sc, 
   release();
   if (MODE == kGemmFc1) {
     const float alpha = sc.alpha, beta = sc.beta, limit = sc.limit;
-    const bool clamp = p.limit != nullptr;
+    const bool clamp = p.limit != nullptr, situ = p.act_type == 10;
     uint2 packed[NCB];
     uint32_t sfword = 0;
 #pragma unroll
     for (int cb = 0; cb < NCB; ++cb) {
       float act[16];
       float amax = 0.f;
+      // two neighbouring channels of a half at a time: up and gate of each sit in neighbouring registers
 #pragma unroll
       for (int c = 0; c < 2; ++c)
 #pragma unroll
-        for (int b = 0; b < 8; ++b) {
-          float up = v[cb][16 * c + b] * sc.up;
-          float gate = v[cb][16 * c + 8 + b] * sc.gate;
+        for (int b = 0; b < 8; b += 2) {
+          float2 up = mul2(make_float2(v[cb][16 * c + b], v[cb][16 * c + b + 1]), make_float2(sc.up, sc.up));
+          float2 gate = mul2(make_float2(v[cb][16 * c + 8 + b], v[cb][16 * c + 9 + b]), make_float2(sc.gate, sc.gate));
           if (clamp) {
-            up = fminf(fmaxf(up, -limit), limit);
-            gate = fminf(gate, limit);
+            up = make_float2(fminf(fmaxf(up.x, -limit), limit), fminf(fmaxf(up.y, -limit), limit));
+            gate = make_float2(fminf(gate.x, limit), fminf(gate.y, limit));
           }
-          float a;
-          if (p.act_type == 10)
-            a = alpha * tanh_fast(__fdividef(gate, alpha)) * sigmoid_fast(gate) * (beta * tanh_fast(__fdividef(up, beta)));
-          else
-            a = gate * sigmoid_fast(alpha * gate) * (up + beta);
-          act[2 * b + c] = a;
-          amax = fmaxf(amax, fabsf(a));
+          float2 a;
+          if (situ) {
+            a.x = alpha * tanh_fast(__fdividef(gate.x, alpha)) * sigmoid_fast(gate.x) * (beta * tanh_fast(__fdividef(up.x, beta)));
+            a.y = alpha * tanh_fast(__fdividef(gate.y, alpha)) * sigmoid_fast(gate.y) * (beta * tanh_fast(__fdividef(up.y, beta)));
+          } else {
+            a = mul2(mul2(gate, sigmoid2(mul2(gate, make_float2(alpha, alpha)))), add2(up, make_float2(beta, beta)));
+          }
+          act[2 * b + c] = a.x;
+          act[2 * b + 2 + c] = a.y;
+          amax = fmaxf(amax, fmaxf(fabsf(a.x), fabsf(a.y)));
         }
       // reference.py:40-42: sf = e4m3(clamp(amax * (1/6), 0, 448)); zero scale -> zero block
       const float sfv = fminf(amax * (1.0f / 6.0f), 448.0f);

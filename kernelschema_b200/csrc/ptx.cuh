@@ -242,6 +242,32 @@ DEV void mma_commit_pair(uint32_t bar) {
 }
 
 // ----------------------------------------------------------------------------- number formats
+// Packed fp32 arithmetic: two IEEE operations per instruction and lane.
+DEV uint64_t f32x2_bits(float2 a) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
+  return r;
+}
+DEV float2 f32x2_val(uint64_t a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+  return r;
+}
+DEV float2 mul2(float2 a, float2 b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f32x2_bits(a)), "l"(f32x2_bits(b)));
+  return f32x2_val(r);
+}
+DEV float2 add2(float2 a, float2 b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f32x2_bits(a)), "l"(f32x2_bits(b)));
+  return f32x2_val(r);
+}
+DEV float2 fma2(float2 a, float2 b, float2 c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(f32x2_bits(a)), "l"(f32x2_bits(b)), "l"(f32x2_bits(c)));
+  return f32x2_val(r);
+}
 // Two fp32 -> one byte of two E2M1 codes, round-to-nearest-even, saturating at 6; `lo` lands in the low nibble.
 DEV uint32_t cvt_e2m1x2(float lo, float hi) {
   uint32_t r;
