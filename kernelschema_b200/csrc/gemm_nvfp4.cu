@@ -14,14 +14,21 @@
 //        32-column block is exactly one 16-channel NVFP4 block of the intermediate activation;
 //   FC2: column 8a+b is output channel 4b+a.
 //
-// One CTA per SM, warp-specialised: TMA producer, MMA issuer, scale-factor copiers, epilogue warps (roles are listed
+// One CTA per SM, warp-specialised: TMA producer, MMA issuer, epilogue warps (roles are listed
 // at each kernel). Stage = 256 FP4 of K: A 16 KB, B BN*128 B, scale factors 2 KB per 128 rows.
 //
 // The tcgen05 and TMA instructions of a role are issued inside `if (elect_one())`, not `if (lane == 0)`: with elect.sync the
 // compiler knows that one thread runs the branch and keeps descriptors in uniform registers; with a lane test every issue
-// costs about 48 cycles (measured with an issue-only loop). A 128 x 256 stage needs 12 scale-factor copies + 4 MMAs (512
-// tensor cycles), spread over kCopiers warps beside the MMA thread. 8192^3, lane test -> elect.sync: CTA-pair kernel
+// costs about 48 cycles (measured with an issue-only loop), and a 128 x 256 stage needs 12 scale-factor copies + 4 MMAs (512
+// tensor cycles). 8192^3, lane test -> elect.sync: CTA-pair kernel
 // 356 -> 223 us (one thread issues for two SMs), 128 x 128 tiles 279 -> 266 us, 128 x 256 tiles 231 -> 227 us.
+//
+// With a long k-loop and enough rows the stage ring is bound by its round trip (TMA latency, hand-over, MMA, commit; about
+// 1.5 us over four stages), not by issue: there the MMA thread copies a stage's scale factors itself, in order before its MMAs,
+// because copier warps between TMA and MMA cost a barrier hop per stage (8192^3 222 -> 207 us without them, 203 us with no scale
+// copies at all; DeepSeek-V3 FC1 at T = 8192 1030 -> 978 us). A batch that streams weights, or a short k-loop, drains stages that
+// are already there at the issue rate, and two copier warps beside the MMA thread are faster (Qwen3 FC1 T = 64 43.4 us against
+// 45.4, T = 16384 183 against 187; T = 1 23.4 us a step against 24.3).
 #include "kernels.cuh"
 #include "ptx.cuh"
 
@@ -30,8 +37,7 @@ namespace b200 {
 constexpr int kBM = 128;
 constexpr int kStageK = 256;             // FP4 elements of K per pipeline stage (128 payload bytes per row)
 constexpr int kSfChunk = 512;            // bytes of one (128 rows x 64 K) scale-factor chunk
-constexpr int kCopiers = 2;              // warps that issue the scale-factor copies of a stage, round-robin (a third would make
-                                         // 13 or 21 warps: one more warp on an SM sub-partition costs the epilogue its registers)
+constexpr int kPairCopiers = 2;          // CTA-pair kernel: warps that issue the scale-factor copies of a stage, round-robin
 
 template <int BN>
 struct GemmCfg {
@@ -45,7 +51,7 @@ struct GemmCfg {
   static constexpr int kSfCols = 16 + 16 * (BN / 128);          // TMEM columns of one scale-factor buffer
   static constexpr int kSfBase = kAccBufs * BN;                  // first scale-factor column
   static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*alignment slack*/ + 256 /*barriers*/;
-  // one TMEM scale-factor buffer per pipeline stage: a copier can run as far ahead of the MMA thread as the stage ring lets it
+  // one TMEM scale-factor buffer per pipeline stage
   static_assert(kSfBase + kStages * kSfCols <= 512, "TMEM budget");
   static constexpr int kSfCopies = 4 + 4 * (BN / 128);           // tcgen05.cp per stage
 };
@@ -227,13 +233,13 @@ DEV void epilogue_cols(const GemmParams& p, uint32_t taddr, const EpiScale& sc, 
   }
 }
 
-// Warp roles: 0 = TMA producer, 1 = TMEM owner + MMA issuer, 2 .. 1 + kCopiers = scale-factor copiers (shared memory ->
-// TMEM), then 4 * BN/EC epilogue warps; epilogue warp w owns TMEM lane quadrant w & 3 and the EC-column group
-// (w - kFirstEpiWarp) / 4.
-constexpr int kFirstEpiWarp = 2 + kCopiers;
+// Warp roles: 0 = TMA producer, 1 = TMEM owner + issuer of the MMAs (and of the scale copies), then kGemmCopiers scale copiers,
+// then 4 * BN/EC epilogue warps; epilogue warp w owns TMEM lane quadrant w & 3 and an EC-column group.
+template <int EC>
+constexpr int kGemmCopiers = EC == 64 ? 2 : 0;
 // any four consecutive warps own the four TMEM lane quadrants (quadrant = warp & 3), so the epilogue groups may start anywhere
 template <int BN, int EC>
-constexpr int gemm_threads() { return 32 * (kFirstEpiWarp + 4 * BN / EC); }
+constexpr int gemm_threads() { return 32 * (2 + kGemmCopiers<EC> + 4 * BN / EC); }
 
 // Scale-factor copy j of a stage (j < 4: A scales of k-block j; then B scales, 128-row half h, k-block q) from the
 // stage's shared-memory slots into its TMEM buffer.
@@ -248,7 +254,7 @@ DEV void sf_copy(int j, uint32_t sf_t, uint32_t sfa_lo, uint32_t sfb_lo) {
   }
 }
 
-// The scale-factor copies of copier warp C: copies C, C + kCopiers, C + 2 * kCopiers, ... of every stage.
+// The scale-factor copies of copier warp C of two: every second copy of every stage.
 template <int BN, int C>
 DEV void copier_loop(const GemmParams& p, uint32_t tmem, uint32_t s_sfa, uint32_t s_sfb, uint32_t bar_full, uint32_t bar_sf,
                      long long total_items, int nk) {
@@ -262,7 +268,7 @@ DEV void copier_loop(const GemmParams& p, uint32_t tmem, uint32_t s_sfa, uint32_
       const uint32_t sf_t = tmem + Cfg::kSfBase + s * Cfg::kSfCols;
       const uint32_t sfa_lo = sfa_lo0 + s * (Cfg::kSfaBytes >> 4), sfb_lo = sfb_lo0 + s * (Cfg::kSfbBytes >> 4);
 #pragma unroll
-      for (int j = C; j < Cfg::kSfCopies; j += kCopiers) sf_copy<BN>(j, sf_t, sfa_lo, sfb_lo);
+      for (int j = C; j < Cfg::kSfCopies; j += 2) sf_copy<BN>(j, sf_t, sfa_lo, sfb_lo);
       mma_commit(bar_sf + 8 * s);                      // arrives once this thread's copies have landed
       if (++s == Cfg::kStages) { s = 0; ph ^= 1; }
     }
@@ -274,6 +280,7 @@ __global__ void __launch_bounds__(gemm_threads<BN, EC>(), 1)
 k_gemm_nvfp4(const __grid_constant__ ActMaps am, const __grid_constant__ CUtensorMap tm_b, const GemmParams p) {
   using C = GemmCfg<BN>;
   constexpr int kEpiWarps = 4 * BN / EC;
+  constexpr int kCopiers = kGemmCopiers<EC>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t s_a = smem_base;
@@ -282,7 +289,7 @@ k_gemm_nvfp4(const __grid_constant__ ActMaps am, const __grid_constant__ CUtenso
   const uint32_t s_sfb = s_sfa + C::kStages * C::kSfaBytes;
   const uint32_t s_bar = s_sfb + C::kStages * C::kSfbBytes;
   const uint32_t bar_full = s_bar;                              // [kStages] TMA bytes landed
-  const uint32_t bar_sf = bar_full + 8 * C::kStages;            // [kStages] scale factors of the stage are in TMEM (all copiers)
+  const uint32_t bar_sf = bar_full + 8 * C::kStages;            // [kStages] the copiers' scale factors are in TMEM (kCopiers > 0)
   const uint32_t bar_empty = bar_sf + 8 * C::kStages;           // [kStages] MMAs of the stage retired
   const uint32_t bar_acc_full = bar_empty + 8 * C::kStages;     // [kAccBufs]
   const uint32_t bar_acc_empty = bar_acc_full + 8 * C::kAccBufs;
@@ -294,7 +301,7 @@ k_gemm_nvfp4(const __grid_constant__ ActMaps am, const __grid_constant__ CUtenso
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::kStages; ++s) {
       mbar_init(bar_full + 8 * s, 1);
-      mbar_init(bar_sf + 8 * s, kCopiers);
+      if (kCopiers > 0) mbar_init(bar_sf + 8 * s, kCopiers);
       mbar_init(bar_empty + 8 * s, 1);
     }
     for (int b = 0; b < C::kAccBufs; ++b) {
@@ -415,39 +422,39 @@ k_gemm_nvfp4(const __grid_constant__ ActMaps am, const __grid_constant__ CUtenso
       // this CTA has asked for its last bytes: the next kernel of the stream may start its prologue under our tail
       pdl_trigger();
     }
-  } else if (warp >= 2 && warp < kFirstEpiWarp) {
-    // ------------------------------------------------------------------ scale-factor copiers: shared memory -> TMEM
-    if (elect_one()) {
-      if (warp == 2) copier_loop<BN, 0>(p, tmem, s_sfa, s_sfb, bar_full, bar_sf, total_items, nk);
-      else if (warp == 3) copier_loop<BN, 1 % kCopiers>(p, tmem, s_sfa, s_sfb, bar_full, bar_sf, total_items, nk);
-      else copier_loop<BN, 2 % kCopiers>(p, tmem, s_sfa, s_sfb, bar_full, bar_sf, total_items, nk);
-    }
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer
+    // ------------------------------------------------------------------ issuer: scale-factor copies, then the MMAs
     if (elect_one()) {
-      // One thread feeds the tensor pipe with four instructions per stage: everything is 32-bit, the stage ring is
-      // walked with counters and the shared-memory descriptors are base + stage * stride.
+      // One thread feeds the tensor pipe: everything is 32-bit, the stage ring is walked with counters and the shared-memory
+      // descriptors are base + stage * stride.
       constexpr uint32_t idesc = make_idesc_nvf4(kBM, BN);
       constexpr uint32_t kHiOp = (1024u >> 4) | (1u << 14) | (2u << 29);   // SBO 1024, version 1, SWIZZLE_128B
       const uint32_t a_lo0 = ((s_a >> 4) & 0x3FFF) | (1u << 16), b_lo0 = ((s_b >> 4) & 0x3FFF) | (1u << 16);
+      const uint32_t sfa_lo0 = (s_sfa >> 4) & 0x3FFF, sfb_lo0 = (s_sfb >> 4) & 0x3FFF;
       uint32_t s = 0, ph = 0, it = 0;
       bool ok = true;
       PROBE_DECL
       for (long long item = blockIdx.x; ok && item < total_items; item += gridDim.x, ++it) {
         const uint32_t buf = it % C::kAccBufs;
-        PROBE_T(pr_a)
-        if (!mbar_wait(bar_acc_empty + 8 * buf, ((it / C::kAccBufs) & 1) ^ 1)) { report(p.status, 102); break; }
-        PROBE_ADD(pr_acc, pr_a)
-        tc_fence_after();
         const uint32_t acc = tmem + buf * BN;
         for (int ks = 0; ks < nk; ++ks) {
-          // the copiers waited for the stage's TMA bytes before they copied: their barrier covers the operands too
           PROBE_T(pr_b)
-          if (!mbar_wait(bar_sf + 8 * s, ph)) { report(p.status, 103); ok = false; break; }
+          // the copiers waited for the stage's TMA bytes before they copied: their barrier covers the operands too
+          if (!mbar_wait((kCopiers > 0 ? bar_sf : bar_full) + 8 * s, ph)) { report(p.status, 103); ok = false; break; }
           PROBE_ADD(pr_sf, pr_b)
           tc_fence_after();
           const uint32_t sf_t = tmem + C::kSfBase + s * C::kSfCols;
           const uint32_t a_lo = a_lo0 + s * (C::kABytes >> 4), b_lo = b_lo0 + s * (C::kBBytes >> 4);
+          if constexpr (kCopiers == 0) {
+#pragma unroll
+            for (int j = 0; j < C::kSfCopies; ++j) sf_copy<BN>(j, sf_t, sfa_lo0 + s * (C::kSfaBytes >> 4), sfb_lo0 + s * (C::kSfbBytes >> 4));
+          }
+          if (ks == 0) {                               // the scale factors do not need the accumulator
+            PROBE_T(pr_a)
+            if (!mbar_wait(bar_acc_empty + 8 * buf, ((it / C::kAccBufs) & 1) ^ 1)) { report(p.status, 102); ok = false; break; }
+            PROBE_ADD(pr_acc, pr_a)
+            tc_fence_after();
+          }
           mma_nvf4(acc, ((uint64_t)kHiOp << 32) | a_lo, ((uint64_t)kHiOp << 32) | b_lo, idesc, sf_t, sf_t + 16, ks ? 1u : 0u);
 #pragma unroll
           for (int q = 1; q < 4; ++q)
@@ -460,18 +467,32 @@ k_gemm_nvfp4(const __grid_constant__ ActMaps am, const __grid_constant__ CUtenso
       }
       PROBE_STORE
     }
+  } else if (kCopiers > 0 && warp < 2 + kCopiers) {
+    if (elect_one()) {
+      if (warp == 2) copier_loop<BN, 0>(p, tmem, s_sfa, s_sfb, bar_full, bar_sf, total_items, nk);
+      else copier_loop<BN, 1>(p, tmem, s_sfa, s_sfb, bar_full, bar_sf, total_items, nk);
+    }
   } else {
     // ------------------------------------------------------------------ epilogue
     const int quad = warp & 3;
-    const int group = (warp - kFirstEpiWarp) >> 2;   // which EC accumulator columns
+    const int group = (warp - 2 - kCopiers) >> 2;   // which EC accumulator columns
     const int r_in_tile = quad * 32 + lane;
     uint32_t it = 0;
+    // table entries and scales of an item are fetched while the one before it is worked on
+    int mt_n = 0, e_n = 0, row0_n = 0, rows_n = 0;
+    auto fetch = [&](long long item) {
+      mt_n = (int)(item / n_ntiles);
+      e_n = p.tile_expert ? p.tile_expert[mt_n] : 0;
+      row0_n = p.tile_row0 ? p.tile_row0[mt_n] : mt_n * kBM;
+      rows_n = p.tile_rows ? p.tile_rows[mt_n] : min(kBM, p.M - row0_n);
+    };
+    if (blockIdx.x < total_items) fetch(blockIdx.x);
+    EpiScale sc = load_scales<MODE>(p, e_n);
     for (long long item = blockIdx.x; item < total_items; item += gridDim.x, ++it) {
-      const int mt = (int)(item / n_ntiles), nt = (int)(item % n_ntiles);
-      const int e = p.tile_expert ? p.tile_expert[mt] : 0;
-      const int row0 = p.tile_row0 ? p.tile_row0[mt] : mt * kBM;
-      const int rows = p.tile_rows ? p.tile_rows[mt] : min(kBM, p.M - row0);
-      const EpiScale sc = load_scales<MODE>(p, e);
+      const int nt = (int)(item - (long long)mt_n * n_ntiles);
+      const int e = e_n, row0 = row0_n, rows = rows_n;
+      const bool more = item + gridDim.x < total_items;
+      if (more) fetch(item + gridDim.x);
       const uint32_t buf = it % C::kAccBufs;
       int okw = 1;
       if (lane == 0) okw = mbar_wait(bar_acc_full + 8 * buf, (it / C::kAccBufs) & 1) ? 1 : 0;
@@ -484,6 +505,7 @@ k_gemm_nvfp4(const __grid_constant__ ActMaps am, const __grid_constant__ CUtenso
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_acc_empty + 8 * buf);
       });
+      if (more && e_n != e) sc = load_scales<MODE>(p, e_n);
     }
   }
   tc_fence_before();
@@ -500,7 +522,7 @@ k_gemm_nvfp4(const __grid_constant__ ActMaps am, const __grid_constant__ CUtenso
 // single-CTA tile. Work item = (pair of consecutive 128-row m-tiles of one expert, 256 weight rows).
 // Barriers: `full` lives in the leader (2 producer arrivals + both CTAs' TMA bytes); `empty` and `acc_full` exist
 // in both CTAs and are signalled by the leader's tcgen05.commit to both; `acc_empty` lives in the leader and
-// collects the 32 epilogue warps of the pair. The scale-factor copies are issued by kCopiers warps of the leader, half
+// collects the 32 epilogue warps of the pair. The scale-factor copies are issued by kPairCopiers warps of the leader, half
 // of a stage's twelve each (one tcgen05.cp.cta_group::2 copies in both CTAs, each from its own shared memory).
 struct PairCfg {
   static constexpr int kStages = 5;
@@ -515,7 +537,8 @@ struct PairCfg {
   static_assert(kSfBase + kStages * kSfCols <= 512, "TMEM budget: one scale-factor buffer per stage");
 };
 
-constexpr int kPairThreads = 32 * (kFirstEpiWarp + 16);    // TMA, MMA, scale-factor copiers, 16 epilogue warps
+constexpr int kPairEpiWarp = 2 + kPairCopiers;
+constexpr int kPairThreads = 32 * (kPairEpiWarp + 16);     // TMA, MMA, scale-factor copiers, 16 epilogue warps
 
 template <int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
@@ -545,7 +568,7 @@ k_gemm_nvfp4_pair(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::kStages; ++s) {
       mbar_init(bar_full + 8 * s, 2);
-      mbar_init(bar_sf + 8 * s, kCopiers);
+      mbar_init(bar_sf + 8 * s, kPairCopiers);
       mbar_init(bar_empty + 8 * s, 1);
     }
     mbar_init(bar_acc_full, 1);
@@ -595,7 +618,7 @@ k_gemm_nvfp4_pair(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       }
       pdl_trigger();
     }
-  } else if (warp >= 2 && warp < kFirstEpiWarp) {
+  } else if (warp >= 2 && warp < kPairEpiWarp) {
     // ------------------------------------------------------------------ scale-factor copiers (leader; every copy acts on both CTAs)
     if (leader && elect_one()) {
       constexpr uint32_t kHiSf = (128u >> 4) | (1u << 14);
@@ -609,7 +632,7 @@ k_gemm_nvfp4_pair(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
           tc_fence_after();
           const uint32_t sf_t = tmem + C::kSfBase + s * C::kSfCols;
           const uint32_t sfa_lo = sfa_lo0 + s * (C::kSfaBytes >> 4), sfb_lo = sfb_lo0 + s * (C::kSfbBytes >> 4);
-          for (int j = j0; j < 12; j += kCopiers) {    // copy j of the stage: 0..3 A scales, then B scales (half h, k-block q)
+          for (int j = j0; j < 12; j += kPairCopiers) {    // copy j of the stage: 0..3 A scales, then B scales (half h, k-block q)
             if (j < 4) {
               tmem_cp_sf_pair(sf_t + 4 * j, ((uint64_t)kHiSf << 32) | (sfa_lo + j * (kSfChunk >> 4)));
             } else {
@@ -658,7 +681,7 @@ k_gemm_nvfp4_pair(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   } else {
     // ------------------------------------------------------------------ epilogue (both CTAs: own 128 rows x 256 columns)
     const int quad = warp & 3;
-    const int group = (warp - kFirstEpiWarp) >> 2;
+    const int group = (warp - kPairEpiWarp) >> 2;
     const int r_in_tile = quad * 32 + lane;
     const uint32_t acc_empty_leader = map_to_cta(bar_acc_empty, 0);
     uint32_t it = 0;
@@ -764,17 +787,17 @@ static int launch_one(const ActMaps& ta, const CUtensorMap& tb, const GemmParams
   return (int)launch_chain(kern, dim3(grid), dim3(gemm_threads<BN, EC>()), GemmCfg<BN>::kSmemBytes, st, ta, tb, p);
 }
 
-// Epilogue columns per warp. Eight warps x 128 columns win only when the k-loop is long AND the GEMM is tensor-bound
-// (DeepSeek-V3 FC1 at T = 8192: 1-2 %). With a short k-loop the eight-warp epilogue is not hidden, and a batch that merely
-// streams its weights (rows_hint: at most that many rows of A) wants its accumulator back as early as possible:
-// T = 128 over 128 experts at K = 4096 takes 137 us per step with 16 x 64 against 151 us.
-static int epilogue_cols_for(int k, int64_t rows_hint) { return (k >= 4096 && (rows_hint == 0 || rows_hint > 8192)) ? 128 : 64; }
+// The form for tensor-bound launches with a long k-loop: eight epilogue warps x 128 columns (hidden by the loop, less power) and
+// in-line scale copies. rows_hint is the most rows of A the launch can hold; the rows of a layer are spread over its experts, so a
+// layer becomes tensor-bound at many more of them than a dense product. Everything else takes 16 warps x 64 columns, which
+// keeps up with a short k-loop and gives a weight-streaming batch its accumulator back early (T = 128 over 128 experts at
+// K = 4096: 137 us per step against 151).
+static bool long_loop_form(int mode, int k, int64_t rows_hint) { return k >= 4096 && rows_hint >= (mode == kGemmDense ? 2048 : 32768); }
 
 template <int MODE>
 static int launch_mode(int bn, const ActMaps& ta, const CUtensorMap& tb, const GemmParams& p, int grid, cudaStream_t st) {
-  const int ec = epilogue_cols_for(p.K, p.rows_hint);
-  if (bn == 128) return ec == 64 ? launch_one<MODE, 128, 64>(ta, tb, p, grid, st) : launch_one<MODE, 128, 128>(ta, tb, p, grid, st);
-  if (bn == 256) return ec == 64 ? launch_one<MODE, 256, 64>(ta, tb, p, grid, st) : launch_one<MODE, 256, 128>(ta, tb, p, grid, st);
+  if (bn == 128) return launch_one<MODE, 128, 64>(ta, tb, p, grid, st);
+  if (bn == 256) return long_loop_form(MODE, p.K, p.rows_hint) ? launch_one<MODE, 256, 128>(ta, tb, p, grid, st) : launch_one<MODE, 256, 64>(ta, tb, p, grid, st);
   return 703;
 }
 
