@@ -297,7 +297,14 @@ int run_impl(b200moe_layer* h, const b200moe_args* a, cudaStream_t st, cudaEvent
   const int64_t worst_tiles = routes / 128 + (routes < h->etot ? routes : (int64_t)h->etot);
   auto tile_n_for = [&](int n_cols) {
     if (h->bn != 256 || c.tile_n != 0) return h->bn;
-    return worst_tiles * (n_cols / 256) * 2 <= h->sm_count ? 128 : 256;
+    if (worst_tiles * (n_cols / 256) * 2 <= h->sm_count) return 128;
+    // A batch with few rows per expert (one m-tile each) streams weights, and its time goes in whole waves of items: 128-wide
+    // tiles when they fill their last wave better (768 items of 256 columns are 5.2 waves of 148 SMs: FC1 of 128 experts x 1536
+    // columns 86 -> 82 us at T = 100, K = 4096). With more rows the narrow tile's extra A traffic costs more than that.
+    if (routes > 64 * (int64_t)h->etot) return 256;
+    const int64_t wide = (routes < h->etot ? routes : (int64_t)h->etot) * (n_cols / 256);
+    const auto fill = [&](int64_t items) { return (double)items / (double)((items + h->sm_count - 1) / h->sm_count * h->sm_count); };
+    return fill(2 * wide) > 1.03 * fill(wide) ? 128 : 256;
   };
   {
     const int bn = tile_n_for(g.N);
