@@ -9,16 +9,22 @@
 //
 // Tile: 256 rows of A (two 128-row accumulators) x BN weight rows, K in steps of 64; one decoded weight tile feeds two
 // MMAs. The kernel is bound by shared-memory bandwidth (per k-step the tile's A and decoded B are written once and read
-// by the MMAs), so the wide form BN = 256 is the default when N allows it: 160 KB of shared-memory traffic per
+// by the MMAs), so the wide form BN = 256 is taken when N allows it: 160 KB of shared-memory traffic per
 // 256 x 256 x 64 step against 112 KB per 256 x 128 x 64 step. Its two 256-column accumulators fill the 512 TMEM columns,
-// so the epilogue of a tile (a few microseconds) is not overlapped; BN = 128 (N % 256 != 0, or M <= 128 where more,
-// narrower tiles keep more SMs busy) alternates between two accumulator pairs.
+// so the epilogue of a tile (a few microseconds) is not overlapped; BN = 128 (N % 256 != 0) alternates between two
+// accumulator pairs.
 // Warp roles: 0 = TMA producer of A (bf16, 128-byte swizzle); 1 = TMEM owner + MMA issuer; then BN/32 decoder warps, one
-// thread per weight row of the tile: it reads the row's 128-byte line (256 weights) and 16 scale bytes with plain loads,
-// one k-group ahead, expands them with byte permutes and one bf16 multiply per pair, and writes bf16 into shared memory
+// thread per weight row of the tile. In the wide form a warp loads its 32 rows' lines (128 bytes = 256 weights each) one k-group ahead, four
+// rows per instruction, and turns them to a row per lane in a shared-memory patch of its own: loaded row by row, an
+// instruction touches 32 lines, and those passes through the L1 pipe compete with the operand traffic (8192 x 4096 x 12288:
+// 734 us, 554 with no weight loads at all). A thread expands its row with byte permutes and one bf16 multiply per pair, and
+// writes bf16 into shared memory
 // in the layout a 128-byte-swizzled TMA load would have produced (16-byte chunk c of row r at
 // r * 128 + ((c ^ (r & 7)) * 16)), then fence.proxy.async + mbarrier arrive; the last 8 warps = epilogue.
 // Every wait is bounded and reports through the status word.
+//
+// The tiles of a last, partly filled wave are split along K (fp32 partial tiles, added in split order by k_w4a16_reduce) as long
+// as that fills the idle SMs; a problem with fewer tiles than SMs is all tail.
 #include "kernels.cuh"
 #include "ptx.cuh"
 
@@ -33,8 +39,11 @@ struct WCfg {
   static constexpr int kStages = BN == 256 ? 3 : 4;
   static constexpr int kABytes = 256 * 128;                // 256 rows x 64 bf16
   static constexpr int kBBytes = BN * 128;                 // BN weight rows x 64 bf16
-  static constexpr int kSmem = kStages * (kABytes + kBBytes) + 1024 + 256;
   static constexpr int kDecWarps = BN / 32;                // one decoder thread per weight row
+  static constexpr bool kPatch = BN == 256;                // weights through a patch: the narrow form has few, short tiles to
+                                                           // hide the extra trip behind (M = 128, N = 2048, K = 4096: 13.8 -> 15.7 us)
+  static constexpr int kPatchBytes = kPatch ? 32 * 128 : 0;   // per decoder warp
+  static constexpr int kSmem = kStages * (kABytes + kBBytes) + kDecWarps * kPatchBytes + 1024 + 256;
   static constexpr int kEpiWarp0 = 2 + kDecWarps;          // first epilogue warp: 2 mod 4, so warp & 3 walks the lane quadrants
   static constexpr int kThreads = 32 * (kEpiWarp0 + 8);
   static constexpr int kAccBufs = 256 / BN;                // pairs of accumulators that fit the 512 TMEM columns
@@ -48,8 +57,9 @@ struct W4A16Params {
   int64_t out_stride;
   int M, N, K;
   int32_t* status;
-  // split-K (small M only): `splits` CTAs share one output tile, each reduces `groups_per_split` k-groups of 256 and
-  // writes fp32 partial sums to partial[split][M][N]; k_w4a16_reduce adds them in split order. splits == 1: no workspace.
+  // Tiles from `full_tiles` on are shared by `splits` CTAs, each of which reduces `groups_per_split` k-groups of 256 and writes
+  // fp32 sums to partial[split][tile - full_tiles][256][BN]. splits == 1: no workspace, full_tiles = all tiles.
+  int full_tiles, tail_tiles;
   int splits;
   int groups_per_split;
   float* partial;
@@ -105,15 +115,14 @@ DEV void decode_half_stage(const uint32_t* w, uint32_t sf2, uint32_t dst, uint32
 }
 
 // BN accumulator columns of the calling warp's 32 lanes -> alpha * x as bf16 at out[row, col0 ...], 64 columns at a
-// time; `release` is called right after the last TMEM read. A warp without live rows only releases.
+// time, or as fp32 at `partial_row`; `release` is called right after the last TMEM read. A warp without live rows only releases.
 template <int BN, class Release>
-DEV void store_cols(const W4A16Params& p, uint32_t taddr, int row, bool live, int col0, float alpha, int split, Release release) {
+DEV void store_cols(const W4A16Params& p, uint32_t taddr, int row, bool live, int col0, float alpha, float* partial_row, Release release) {
   if (!__any_sync(0xFFFFFFFFu, live)) {
     release();
     return;
   }
-  if (BN == 128 && p.splits > 1) {                   // fp32 partial sums of this split; alpha and the rounding come in the reduce
-    float* dst = p.partial + ((size_t)split * p.M + row) * p.N + col0;
+  if (partial_row) {                                 // alpha and the rounding come in the reduce
 #pragma unroll
     for (int pass = 0; pass < BN / 32; ++pass) {
       float v[32];
@@ -122,7 +131,8 @@ DEV void store_cols(const W4A16Params& p, uint32_t taddr, int row, bool live, in
       if (pass == BN / 32 - 1) release();
       if (live) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) reinterpret_cast<float4*>(dst + pass * 32)[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+        for (int j = 0; j < 8; ++j)
+          reinterpret_cast<float4*>(partial_row + pass * 32)[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
       }
     }
     return;
@@ -162,7 +172,8 @@ k_gemm_w4a16(const __grid_constant__ CUtensorMap tm_a, const W4A16Params p) {
   using C = WCfg<BN>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t s_a = base, s_b = s_a + C::kStages * C::kABytes, s_bar = s_b + C::kStages * C::kBBytes;
+  const uint32_t s_a = base, s_b = s_a + C::kStages * C::kABytes, s_patch = s_b + C::kStages * C::kBBytes;
+  const uint32_t s_bar = s_patch + C::kDecWarps * C::kPatchBytes;
   const uint32_t bar_full_a = s_bar;                         // [stages] TMA bytes of A landed
   const uint32_t bar_full_b = bar_full_a + 8 * C::kStages;   // [stages] the decoder warps wrote their rows
   const uint32_t bar_empty = bar_full_b + 8 * C::kStages;    // [stages] MMAs of the stage retired
@@ -192,15 +203,15 @@ k_gemm_w4a16(const __grid_constant__ CUtensorMap tm_a, const W4A16Params p) {
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(s_slot));
   pdl_wait();
 
-  const int n_mt = (p.M + 255) >> 8;        // 256-row tiles of A
   const int n_nt = p.N / BN;                // BN-row tiles of the weights
   const int groups = p.K >> 8;              // k-groups of 256 weights = one 128-byte line per weight row
-  // item = (tile, split), split fastest; tile = (mt, nt), n fastest: the CTAs of a wave share A's rows and sweep the
-  // weights (L2-resident). A split covers k-groups [g0, g1).
-  const int total_items = n_mt * n_nt * p.splits;
-  auto item_tile = [&](int item) { return item / p.splits; };
-  auto item_g0 = [&](int item) { return (item % p.splits) * p.groups_per_split; };
-  auto item_g1 = [&](int item) { return min(groups, (item % p.splits + 1) * p.groups_per_split); };
+  // items: the whole tiles, then (tail tile, split) with the split fastest; tile = (mt, nt), n fastest: the CTAs of a wave share
+  // A's rows and sweep the weights (L2-resident). A split covers k-groups [g0, g1).
+  const int total_items = p.full_tiles + p.tail_tiles * p.splits;
+  auto item_tile = [&](int item) { return item < p.full_tiles ? item : p.full_tiles + (item - p.full_tiles) / p.splits; };
+  auto item_split = [&](int item) { return item < p.full_tiles ? -1 : (item - p.full_tiles) % p.splits; };
+  auto item_g0 = [&](int item) { return max(item_split(item), 0) * p.groups_per_split; };
+  auto item_g1 = [&](int item) { return item < p.full_tiles ? groups : min(groups, (item_split(item) + 1) * p.groups_per_split); };
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer of A
@@ -260,37 +271,62 @@ k_gemm_w4a16(const __grid_constant__ CUtensorMap tm_a, const W4A16Params p) {
     bool ok = true;
     uint4 nxt[8];
     uint4 nxt_sf;
+    const uint32_t patch = s_patch + (uint32_t)(warp - 2) * C::kPatchBytes;
+    // one k-group of the warp's rows: through the patch lane -> row 4i + lane / 8, 16-byte piece lane % 8, else each lane its own
+    // row; and the scales of the lane's own row
     auto fetch = [&](int item, int g) {
-      const int nt = item_tile(item) % n_nt;
-      const size_t row = (size_t)nt * BN + r;
-      const uint4* q = reinterpret_cast<const uint4*>(p.b_q + row * (size_t)(p.K >> 1)) + (size_t)g * 8;
+      const size_t row0 = (size_t)(item_tile(item) % n_nt) * BN + (r & ~31);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) nxt[i] = __ldg(q + i);
-      nxt_sf = __ldg(reinterpret_cast<const uint4*>(p.b_sf + row * (size_t)(p.K >> 4)) + g);
+      for (int i = 0; i < 8; ++i) {
+        const int row = C::kPatch ? 4 * i + (lane >> 3) : lane, piece = C::kPatch ? lane & 7 : i;
+        nxt[i] = __ldg(reinterpret_cast<const uint4*>(p.b_q + (row0 + row) * (size_t)(p.K >> 1)) + (size_t)g * 8 + piece);
+      }
+      nxt_sf = __ldg(reinterpret_cast<const uint4*>(p.b_sf + (row0 + lane) * (size_t)(p.K >> 4)) + g);
     };
     if ((int)blockIdx.x < total_items) fetch(blockIdx.x, item_g0(blockIdx.x));
     for (int item = blockIdx.x; ok && item < total_items; item += gridDim.x) {
       const int g1 = item_g1(item);
       for (int g = item_g0(item); ok && g < g1; ++g) {
-        uint32_t cur[32];
-        uint32_t cur_sf[4];
+        uint32_t line[C::kPatch ? 1 : 32];
+        if constexpr (!C::kPatch) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          cur[4 * i] = nxt[i].x; cur[4 * i + 1] = nxt[i].y; cur[4 * i + 2] = nxt[i].z; cur[4 * i + 3] = nxt[i].w;
+          for (int i = 0; i < 8; ++i) {
+            line[4 * i] = nxt[i].x; line[4 * i + 1] = nxt[i].y; line[4 * i + 2] = nxt[i].z; line[4 * i + 3] = nxt[i].w;
+          }
         }
-        cur_sf[0] = nxt_sf.x; cur_sf[1] = nxt_sf.y; cur_sf[2] = nxt_sf.z; cur_sf[3] = nxt_sf.w;
-        // next line: the following k-group of this item, or the first of this CTA's next item
+        if (C::kPatch) __syncwarp();                        // the previous group has been read out of the patch
+#pragma unroll
+        for (int i = 0; C::kPatch && i < 8; ++i) {
+          const uint32_t pr = 4 * i + (lane >> 3);
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(patch + pr * 128u + ((((uint32_t)lane & 7) ^ (pr & 7)) << 4)),
+                       "r"(nxt[i].x), "r"(nxt[i].y), "r"(nxt[i].z), "r"(nxt[i].w)
+                       : "memory");
+        }
+        if (C::kPatch) __syncwarp();
+        const uint32_t cur_sf[4] = {nxt_sf.x, nxt_sf.y, nxt_sf.z, nxt_sf.w};
+        // next lines: the following k-group of this item, or the first of this CTA's next item
         if (g + 1 < g1) fetch(item, g + 1);
         else if (item + (int)gridDim.x < total_items) fetch(item + gridDim.x, item_g0(item + gridDim.x));
 #pragma unroll
         for (int q = 0; q < 4; ++q) {                       // the four 64-wide k-steps of the group
+          uint32_t cur[8];
+          if constexpr (!C::kPatch) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) cur[i] = line[8 * q + i];
+          }
+#pragma unroll
+          for (int c = 0; C::kPatch && c < 2; ++c)
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(cur[4 * c]), "=r"(cur[4 * c + 1]), "=r"(cur[4 * c + 2]), "=r"(cur[4 * c + 3])
+                         : "r"(patch + (uint32_t)lane * 128u + (((uint32_t)(2 * q + c) ^ sw) << 4))
+                         : "memory");
           int okw = 1;
           if (lane == 0) okw = mbar_wait(bar_empty + 8 * s, ph) ? 1 : 0;
           okw = __shfl_sync(0xFFFFFFFFu, okw, 0);
           if (!okw) { if (lane == 0 && p.status) atomicCAS(p.status, 0, 125); ok = false; break; }
           const uint32_t dst = s_b + s * C::kBBytes + row_off;
-          decode_half_stage(cur + 8 * q, cur_sf[q], dst, sw, 0);
-          decode_half_stage(cur + 8 * q + 4, cur_sf[q] >> 16, dst, sw, 4);
+          decode_half_stage(cur, cur_sf[q], dst, sw, 0);
+          decode_half_stage(cur + 4, cur_sf[q] >> 16, dst, sw, 4);
           fence_async_proxy();                              // generic-proxy writes -> visible to the tensor core's reads
           __syncwarp();
           if (lane == 0) mbar_arrive(bar_full_b + 8 * s);
@@ -316,7 +352,11 @@ k_gemm_w4a16(const __grid_constant__ CUtensorMap tm_a, const W4A16Params p) {
       const int row = mt * 256 + half * 128 + quad * 32 + lane;
       const bool live = row < p.M;
       const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + buf * 2 * BN + half * BN;
-      store_cols<BN>(p, taddr, row, live, nt * BN, alpha, item % p.splits, [&]() {
+      const int split = item_split(item);
+      float* partial_row = split < 0 || p.splits == 1 ? nullptr
+                                                      : p.partial + (((size_t)split * p.tail_tiles + (tile - p.full_tiles)) * 256 +
+                                                                     (half * 128 + quad * 32 + lane)) * BN;
+      store_cols<BN>(p, taddr, row, live, nt * BN, alpha, partial_row, [&]() {
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_acc_empty + 8 * buf);
@@ -331,51 +371,64 @@ k_gemm_w4a16(const __grid_constant__ CUtensorMap tm_a, const W4A16Params p) {
   }
 }
 
-// out[m, n] = bf16(alpha * sum over splits of partial[s][m][n]), splits added in ascending order (reproducible).
-__global__ void __launch_bounds__(256) k_w4a16_reduce(const float* __restrict__ partial, const float* __restrict__ alpha_ptr, int splits,
-                                                      int64_t M, int64_t N, __nv_bfloat16* __restrict__ out, int64_t out_stride) {
+// Tail tiles: out = bf16(alpha * sum over splits of partial[s][tile]), splits added in ascending order (reproducible).
+__global__ void __launch_bounds__(256) k_w4a16_reduce(const W4A16Params p, int bn) {
   pdl_trigger();
   pdl_wait();
-  const float alpha = alpha_ptr ? *alpha_ptr : 1.0f;
-  const int64_t quads = M * N / 4;
+  const float alpha = p.alpha ? *p.alpha : 1.0f;
+  const int n_nt = p.N / bn, tile_quads = min(p.M, 256) * bn / 4;     // groups of four columns of a tile's rows
+  const int64_t quads = (int64_t)p.tail_tiles * tile_quads;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < quads; i += (int64_t)gridDim.x * blockDim.x) {
-    float4 acc = reinterpret_cast<const float4*>(partial)[i];
-    for (int s = 1; s < splits; ++s) {
-      const float4 v = reinterpret_cast<const float4*>(partial + (size_t)s * M * N)[i];
+    const int t = (int)(i / tile_quads), tile = p.full_tiles + t, at = (int)(i - (int64_t)t * tile_quads) * 4;
+    const int row = tile / n_nt * 256 + at / bn, col = tile % n_nt * bn + at % bn;
+    if (row >= p.M) continue;
+    const float* src = p.partial + (size_t)t * 256 * bn + at;
+    float4 acc = *reinterpret_cast<const float4*>(src);
+    for (int s = 1; s < p.splits; ++s) {
+      const float4 v = *reinterpret_cast<const float4*>(src + (size_t)s * p.tail_tiles * 256 * bn);
       acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
     }
-    const int64_t m = (i * 4) / N, n = (i * 4) % N;
     const __nv_bfloat162 lo = __floats2bfloat162_rn(acc.x * alpha, acc.y * alpha), hi = __floats2bfloat162_rn(acc.z * alpha, acc.w * alpha);
     uint2 o;
     o.x = *reinterpret_cast<const uint32_t*>(&lo);
     o.y = *reinterpret_cast<const uint32_t*>(&hi);
-    *reinterpret_cast<uint2*>(out + m * out_stride + n) = o;
+    *reinterpret_cast<uint2*>(p.out + (size_t)row * p.out_stride + col) = o;
   }
 }
 
 }  // namespace
 
-// Split-K plan for small M: enough CTAs per output tile to occupy the device; 1 = no split (no workspace needed).
-static int w4a16_splits(int64_t m, int64_t n, int64_t k, int sms) {
-  if (m > 128 || w4a16_decode_fits(m)) return 1;
-  const int64_t tiles = n / 128, groups = k / 256;
-  int64_t s = sms / tiles;
+// Tile width and split of the last wave. The tiles left over after whole waves are shared by as many CTAs as the SMs hold (at most
+// eight, at least one k-group each). Behind whole waves that pays for its partial tiles and the second launch (about 15 us) only
+// when a tile is long: from 16 k-groups on.
+struct W4A16Plan {
+  int bn, full_tiles, tail_tiles, splits;
+};
+static W4A16Plan w4a16_plan(int64_t m, int64_t n, int64_t k, int sms) {
+  W4A16Plan pl;
+  // up to 128 rows half of a wide tile's accumulators idle: it pays when the tiles are many and long (M = 64, N = 4096,
+  // K = 12288: 31 us against 36 us; N = 2048, K = 4096: 16 against 12)
+  pl.bn = n % 256 == 0 && (m > 128 || (n >= 4096 && k >= 8192)) ? 256 : 128;
+  const int64_t tiles = (m + 255) / 256 * (n / pl.bn), groups = k / 256, tail = tiles % sms;
+  int64_t s = tail ? sms / tail : 1;
   if (s > 8) s = 8;
   if (s > groups) s = groups;
-  return s < 2 ? 1 : (int)s;
+  if (s < 2 || w4a16_decode_fits(m) || (tiles > tail && groups < 16)) s = 1;
+  pl.splits = (int)s;
+  pl.tail_tiles = s > 1 ? (int)tail : 0;
+  pl.full_tiles = (int)(tiles - pl.tail_tiles);
+  return pl;
 }
+static int64_t w4a16_partial_bytes(const W4A16Plan& pl) { return (int64_t)pl.splits * pl.tail_tiles * 256 * pl.bn * 4; }
 
-int64_t gemm_w4a16_workspace_bytes(int64_t m, int64_t n, int64_t k) {
-  const int s = w4a16_splits(m, n, k, sm_count());
-  return s > 1 ? (int64_t)s * m * n * 4 : 0;
-}
+int64_t gemm_w4a16_workspace_bytes(int64_t m, int64_t n, int64_t k) { return w4a16_partial_bytes(w4a16_plan(m, n, k, sm_count())); }
 
 template <int BN>
 static int launch_w4a16(const CUtensorMap& ta, const W4A16Params& p, int sms, cudaStream_t st) {
   auto kern = k_gemm_w4a16<BN>;
   static SmemOptIn opt_in;
   if (int e = opt_in.ensure(kern, WCfg<BN>::kSmem)) return e;
-  const int64_t items = (int64_t)((p.M + 255) / 256) * (p.N / BN) * p.splits;
+  const int64_t items = (int64_t)p.full_tiles + (int64_t)p.tail_tiles * p.splits;
   return (int)launch_chain(kern, dim3((unsigned)(items < sms ? items : sms)), dim3(WCfg<BN>::kThreads), WCfg<BN>::kSmem, st, ta, p);
 }
 
@@ -384,11 +437,12 @@ int launch_gemm_w4a16(const void* a, int64_t a_stride, const void* b_q, const vo
                       cudaStream_t st) {
   if (m == 0) return 0;
   if (w4a16_decode_fits(m)) return launch_gemm_w4a16_decode(a, a_stride, b_q, b_sf, alpha, m, n, k, out, out_stride, st);
-  const int bn = (n % 256 == 0 && m > 128) ? 256 : 128;
+  const int sms = sm_count();
+  W4A16Plan pl = w4a16_plan(m, n, k, sms);
+  const int bn = pl.bn;
   CUtensorMap ta;
   int rc = make_operand_map(&ta, a, (uint64_t)m, (uint64_t)k * 2, 256, (uint64_t)a_stride * 2);
   if (rc) return rc;
-  const int sms = sm_count();
   W4A16Params p;
   p.b_q = (const uint8_t*)b_q;
   p.b_sf = (const uint8_t*)b_sf;
@@ -399,21 +453,20 @@ int launch_gemm_w4a16(const void* a, int64_t a_stride, const void* b_q, const vo
   p.N = (int)n;
   p.K = (int)k;
   p.status = status;
-  p.splits = 1;
-  p.groups_per_split = (int)(k / 256);
-  p.partial = nullptr;
-  const int want = w4a16_splits(m, n, k, sms);
-  if (bn == 128 && want > 1 && workspace && workspace_bytes >= (int64_t)want * m * n * 4) {
-    p.groups_per_split = (int)((k / 256 + want - 1) / want);
-    p.splits = (int)((k / 256 + p.groups_per_split - 1) / p.groups_per_split);      // no empty split
-    p.partial = (float*)workspace;
+  p.partial = (float*)workspace;
+  if (pl.splits > 1 && (!workspace || workspace_bytes < w4a16_partial_bytes(pl))) {      // no room for partial tiles: nothing is split
+    pl.full_tiles += pl.tail_tiles;
+    pl.tail_tiles = 0;
+    pl.splits = 1;
   }
+  p.groups_per_split = (int)((k / 256 + pl.splits - 1) / pl.splits);
+  p.splits = (int)((k / 256 + p.groups_per_split - 1) / p.groups_per_split);              // no empty split
+  p.full_tiles = pl.full_tiles;
+  p.tail_tiles = pl.tail_tiles;
   rc = bn == 256 ? launch_w4a16<256>(ta, p, sms, st) : launch_w4a16<128>(ta, p, sms, st);
   if (rc || p.splits == 1) return rc;
-  const int64_t quads = m * n / 4;
-  const int64_t blocks = (quads + 255) / 256;
-  return (int)launch_chain(k_w4a16_reduce, dim3((unsigned)(blocks < (int64_t)sms * 8 ? blocks : (int64_t)sms * 8)), dim3(256), 0, st, (const float*)p.partial,
-                           alpha, p.splits, m, n, (__nv_bfloat16*)out, out_stride);
+  const int64_t blocks = ((int64_t)p.tail_tiles * (m < 256 ? m : 256) * (bn / 4) + 255) / 256;
+  return (int)launch_chain(k_w4a16_reduce, dim3((unsigned)(blocks < (int64_t)sms * 8 ? blocks : (int64_t)sms * 8)), dim3(256), 0, st, p, bn);
 }
 
 }  // namespace b200

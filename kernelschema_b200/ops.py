@@ -68,9 +68,9 @@ def nvfp4_quantize(x: torch.Tensor, global_scale: float = 1.0, tiled_scales: boo
     else:
         payload = torch.empty((rows, cols // 2), dtype=torch.uint8, device=x.device)
         if tiled_scales:
-            scales = torch.empty(((rows + 127) // 128, cols // 64, 32, 16), dtype=torch.uint8, device=x.device)
-            if rows % 128:
-                scales[-1].zero_()           # the kernel writes every row it has; only a ragged last tile holds others
+            # the kernel writes every row it has; only a ragged last tile holds others
+            alloc = torch.zeros if rows % 128 else torch.empty
+            scales = alloc(((rows + 127) // 128, cols // 64, 32, 16), dtype=torch.uint8, device=x.device)
         else:
             scales = torch.empty((rows, cols // 16), dtype=torch.uint8, device=x.device)
     lib = _lib.load()
@@ -140,9 +140,6 @@ def mm_nvfp4(a_q, a_sf_tiled, b_q, b_sf_tiled, alpha: float = 1.0, out: torch.Te
     return out
 
 
-_W4A16_WORKSPACE: dict = {}     # device index -> fp32 split-K scratch, grown on demand (small M only)
-
-
 def mm_bf16_nvfp4(a: torch.Tensor, b: torch.Tensor, b_descale: torch.Tensor, alpha: torch.Tensor | None = None,
                   out: torch.Tensor | None = None, status: torch.Tensor | None = None, split_k: bool = True) -> torch.Tensor:
     """out[M, N] = bf16(alpha * a @ decode(b)^T): bf16 activations [M, K] (not quantised), NVFP4 weights uint8 [N, K/2] with
@@ -165,12 +162,8 @@ def mm_bf16_nvfp4(a: torch.Tensor, b: torch.Tensor, b_descale: torch.Tensor, alp
     ws = None
     need = int(lib.b200moe_gemm_bf16_nvfp4_workspace_bytes(m, n, k)) if split_k else 0
     if need:
-        # one scratch buffer per device, reused by later calls on the same stream order (calls on different streams
-        # that may overlap should pass split_k=False or run on one stream)
-        dev = a.device.index
-        ws = _W4A16_WORKSPACE.get(dev)
-        if ws is None or ws.numel() < need:
-            ws = _W4A16_WORKSPACE[dev] = torch.empty(need, dtype=torch.uint8, device=a.device)
+        # from the caching allocator per call: ordered with the current stream, so calls on other streams and threads keep apart
+        ws = torch.empty(need, dtype=torch.uint8, device=a.device)
     _lib.check(lib.b200moe_gemm_bf16_nvfp4(a.data_ptr(), a.stride(0), b.data_ptr(), b_descale.data_ptr(), _ptr(alpha), out.data_ptr(),
                                            m, n, k, out.stride(0), _ptr(ws), need, _ptr(status), _stream()),
                "b200moe_gemm_bf16_nvfp4")

@@ -191,6 +191,29 @@ def test_w4a16_strided_a_and_no_alpha():
     assert r["rel_l2"] <= 1e-3, r
 
 
+@pytest.mark.parametrize("m,n,k", [(33, 4096, 8192), (128, 4096, 8192), (129, 256, 256), (300, 1024, 1280), (513, 4096, 4096), (2600, 4096, 4096),
+                                   (3000, 3328, 4352)])
+def test_w4a16_split_last_wave(m, n, k):
+    """Problems of fewer tiles than SMs, and a last wave behind whole ones (2600 x 4096: 176 tiles, 28 of them split on 148 SMs):
+    the same sums with and without the workspace up to the order of the fp32 additions, rows beyond M left alone."""
+    import kernelschema_b200 as ks
+    gen = torch.Generator(device="cuda").manual_seed(m + n)
+    a = torch.randn(m, k, device="cuda", generator=gen).to(torch.bfloat16)
+    bq, bsf = ks.nvfp4_quantize((torch.randn(n, k, device="cuda", generator=gen) * k ** -0.5).to(torch.bfloat16), 1.0)
+    alpha = torch.tensor([1.25], dtype=torch.float32, device="cuda")
+    backing = torch.full((m + 2, n), -17.0, dtype=torch.bfloat16, device="cuda")
+    y = ks.mm_bf16_nvfp4(a, bq, bsf.view(torch.uint8), alpha, out=backing[1:m + 1])
+    plain = ks.mm_bf16_nvfp4(a, bq, bsf.view(torch.uint8), alpha, split_k=False)
+    torch.cuda.synchronize()
+    assert (backing[0] == -17).all() and (backing[m + 1] == -17).all()
+    codes = torch.tensor([0, .5, 1, 1.5, 2, 3, 4, 6, 0, -.5, -1, -1.5, -2, -3, -4, -6], device="cuda", dtype=torch.float64)
+    w = torch.stack((codes[(bq & 15).long()], codes[(bq >> 4).long()]), -1).view(n, k)
+    w = (w.view(n, k // 16, 16) * bsf.view(torch.float8_e4m3fn).double()[..., None]).view(n, k)
+    ref, mag = 1.25 * a.double() @ w.T, 1.25 * a.double().abs() @ w.abs().T
+    for got in (y, plain):          # one bf16 rounding, and 2^-20 of the magnitudes for the fp32 sums
+        assert ((got.double() - ref).abs() <= ref.abs() / 256 + mag * 2.0 ** -20).all()
+
+
 def test_w4a16_linearity_full_size():
     """Size-independent properties at a reference shape (M 8192, N 4096, K 2048): doubling A doubles the output exactly,
     and a row of A gives the same output row whatever tile it sits in."""

@@ -283,6 +283,25 @@ def test_library_graph_cache_and_hot_call():
     cached.close()
 
 
+@pytest.mark.parametrize("rows", [1, 15, 16, 17, 63, 64, 65, 127, 128, 129, 144, 192, 193])
+def test_segments_at_the_edges_of_the_fetched_boxes(rows):
+    """An m-tile of up to 16 or 64 rows fetches a box of that height. One expert holds `rows` rows, the others one or none, on
+    top of a workspace full of another batch's rows."""
+    from gpu_util import run_model
+    e, t = 9, max(rows, 3)
+    p = make_moe_case(70 + rows, t, 512, 512, e, 1)
+    big = make_moe_case(69, 700, 512, 512, e, 1)
+    big["gemm1_weights"], big["gemm1_weights_scale"] = p["gemm1_weights"], p["gemm1_weights_scale"]
+    big["gemm2_weights"], big["gemm2_weights_scale"] = p["gemm2_weights"], p["gemm2_weights_scale"]
+    ids = np.full((t, 1), -1, np.int32)
+    ids[:rows] = 4
+    ids[rows:rows + 2] = 8
+    p["topk_ids"] = (ids, np.where(ids >= 0, np.float32(0.75), np.float32(0)))
+    _, _, model = run_model(big)
+    got, _, _ = run_model(p, model)
+    assert_layer_parity(got, o.moe_expected(p), f"rows={rows}")
+
+
 @pytest.mark.parametrize("t,h,e,k,s", [(1, 512, 16, 4, 0), (3, 512, 255, 10, 1), (8, 512, 256, 32, 2), (9, 512, 16, 4, 1), (8, 4608, 16, 4, 1),
                                        (4, 8192, 17, 17, 0), (8, 256, 300, 3, 0)])
 def test_step_of_a_handful_of_tokens_equals_separate_calls(t, h, e, k, s):
