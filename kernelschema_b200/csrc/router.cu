@@ -200,7 +200,7 @@ k_router_logits_tc(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
   const uint32_t s_a = base, s_b = s_a + kLgStages * kLgABytes, s_bar = s_b + kLgStages * kLgBBytes;
   const uint32_t bar_full = s_bar, bar_empty = s_bar + 8 * kLgStages, bar_acc_full = bar_empty + 8 * kLgStages,
                  bar_acc_empty = bar_acc_full + 16, s_slot = bar_acc_empty + 16;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kLgStages; ++s) { mbar_init(bar_full + 8 * s, 1); mbar_init(bar_empty + 8 * s, 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(bar_acc_full + 8 * b, 1); mbar_init(bar_acc_empty + 8 * b, 4); }
@@ -218,7 +218,7 @@ k_router_logits_tc(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
   const int nk = H >> 6;
   const uint32_t stage_bytes = kLgABytes + (uint32_t)e_pad * 128;
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t g = 0;
       bool ok = true;
       for (int tile = blockIdx.x; ok && tile < n_tiles; tile += gridDim.x)
@@ -231,7 +231,7 @@ k_router_logits_tc(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
         }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = make_idesc_bf16(128, e_pad);
       uint32_t g = 0, it = 0;
       bool ok = true;
@@ -328,7 +328,7 @@ k_router_logits_ksplit(const __grid_constant__ CUtensorMap tm_x, const __grid_co
   const uint32_t s_a = base, s_b = s_a + kLkStages * kLkABytes, s_bar = s_b + kLkStages * kLkBBytes;
   const uint32_t bar_full = s_bar, bar_empty = s_bar + 8 * kLkStages, bar_acc_full = bar_empty + 8 * kLkStages, s_slot = bar_acc_full + 8;
   const uint32_t s_part = s_a;                    // after the k-loop: this block's partial tile, [e_slice][128] floats
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform(), lane = threadIdx.x & 31;
   const int k_split = (int)gridDim.z;
   const uint32_t rank = cluster_ctarank();        // == blockIdx.z: the cluster spans z
   const int tile = (int)blockIdx.x, e0 = (int)blockIdx.y * e_slice;
@@ -348,7 +348,7 @@ k_router_logits_ksplit(const __grid_constant__ CUtensorMap tm_x, const __grid_co
   const int steps = (H >> 6) / k_split, ks0 = (int)rank * steps;
   const uint32_t stage_bytes = kLkABytes + (uint32_t)e_slice * 128;
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       for (int i = 0; i < steps; ++i) {
         const uint32_t s = i % kLkStages;
         if (!mbar_wait(bar_empty + 8 * s, ((i / kLkStages) & 1) ^ 1)) { if (status) atomicCAS(status, 0, 115); break; }
@@ -359,7 +359,7 @@ k_router_logits_ksplit(const __grid_constant__ CUtensorMap tm_x, const __grid_co
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = make_idesc_bf16(128, e_slice);
       bool ok = true;
       for (int i = 0; i < steps; ++i) {
