@@ -196,10 +196,12 @@ def make_step(wl, L, world, device, tokens=None):
             return out, ids_view[:x.shape[0]]
 
         step.front = front
-        # quantiser, router logits, top-k + the layer: route map and permute are one kernel up to 8192 routes, the route map
-        # alone is one kernel up to 16384 routes and three above; then FC1, FC2 and the combine
+        # quantiser, router logits, top-k (up to eight tokens: the first two in one kernel while T x H <= 32768, the selection
+        # inside the route map) + the layer: route map and permute are one kernel up to 16384 routes, above that the route map
+        # is two kernels up to 262144 and three beyond; then FC1, FC2 and the combine
         routes = t * (k + s)
-        return step, layer, 3 + (4 if routes <= 8192 else 5 if routes <= 16384 else 7)
+        front_launches = 3 if t > 8 else 2 if t * h > 32768 else 1
+        return step, layer, front_launches + (4 if routes <= 16384 else 6 if routes <= 262144 else 7)
     from kernelschema_b200.ep import ExpertParallelMoE
     ep = ExpertParallelMoE(h, i, e, k, t, num_shared_experts=s)
 

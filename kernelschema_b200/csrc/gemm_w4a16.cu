@@ -376,12 +376,10 @@ __global__ void __launch_bounds__(256) k_w4a16_reduce(const W4A16Params p, int b
   pdl_trigger();
   pdl_wait();
   const float alpha = p.alpha ? *p.alpha : 1.0f;
-  const int n_nt = p.N / bn, tile_quads = min(p.M, 256) * bn / 4;     // groups of four columns of a tile's rows
-  const int64_t quads = (int64_t)p.tail_tiles * tile_quads;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < quads; i += (int64_t)gridDim.x * blockDim.x) {
-    const int t = (int)(i / tile_quads), tile = p.full_tiles + t, at = (int)(i - (int64_t)t * tile_quads) * 4;
-    const int row = tile / n_nt * 256 + at / bn, col = tile % n_nt * bn + at % bn;
-    if (row >= p.M) continue;
+  const int at = ((int)blockIdx.x * (int)blockDim.x + (int)threadIdx.x) * 4;             // four columns of a tile's row
+  const int t = (int)blockIdx.y, tile = p.full_tiles + t, n_nt = p.N / bn;
+  const int row = tile / n_nt * 256 + at / bn, col = tile % n_nt * bn + at % bn;
+  if (at < min(p.M, 256) * bn && row < p.M) {
     const float* src = p.partial + (size_t)t * 256 * bn + at;
     float4 acc = *reinterpret_cast<const float4*>(src);
     for (int s = 1; s < p.splits; ++s) {
@@ -465,8 +463,8 @@ int launch_gemm_w4a16(const void* a, int64_t a_stride, const void* b_q, const vo
   p.tail_tiles = pl.tail_tiles;
   rc = bn == 256 ? launch_w4a16<256>(ta, p, sms, st) : launch_w4a16<128>(ta, p, sms, st);
   if (rc || p.splits == 1) return rc;
-  const int64_t blocks = ((int64_t)p.tail_tiles * (m < 256 ? m : 256) * (bn / 4) + 255) / 256;
-  return (int)launch_chain(k_w4a16_reduce, dim3((unsigned)(blocks < (int64_t)sms * 8 ? blocks : (int64_t)sms * 8)), dim3(256), 0, st, p, bn);
+  const int64_t quads = (m < 256 ? m : 256) * (bn / 4);
+  return (int)launch_chain(k_w4a16_reduce, dim3((unsigned)((quads + 255) / 256), (unsigned)p.tail_tiles), dim3(256), 0, st, p, bn);
 }
 
 }  // namespace b200

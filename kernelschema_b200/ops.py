@@ -140,6 +140,24 @@ def mm_nvfp4(a_q, a_sf_tiled, b_q, b_sf_tiled, alpha: float = 1.0, out: torch.Te
     return out
 
 
+_W4A16_WORKSPACE: dict = {}     # (device index, stream) -> split-K scratch
+
+
+def _w4a16_workspace(device: torch.device, stream: int, need: int) -> torch.Tensor:
+    """Scratch of the current stream: calls on one stream follow one another, calls on different streams never share. At most
+    eight streams keep one; a buffer that is let go returns to the caching allocator of its own stream. While the stream is being
+    captured the buffer belongs to the graph's pool instead, so that a replay never sees a buffer that has been replaced."""
+    if torch.cuda.is_current_stream_capturing():
+        return torch.empty(need, dtype=torch.uint8, device=device)
+    key = (device.index, stream)
+    ws = _W4A16_WORKSPACE.get(key)
+    if ws is None or ws.numel() < need:
+        if ws is None and len(_W4A16_WORKSPACE) >= 8:
+            _W4A16_WORKSPACE.pop(next(iter(_W4A16_WORKSPACE)), None)
+        ws = _W4A16_WORKSPACE[key] = torch.empty(need, dtype=torch.uint8, device=device)
+    return ws
+
+
 def mm_bf16_nvfp4(a: torch.Tensor, b: torch.Tensor, b_descale: torch.Tensor, alpha: torch.Tensor | None = None,
                   out: torch.Tensor | None = None, status: torch.Tensor | None = None, split_k: bool = True) -> torch.Tensor:
     """out[M, N] = bf16(alpha * a @ decode(b)^T): bf16 activations [M, K] (not quantised), NVFP4 weights uint8 [N, K/2] with
@@ -159,13 +177,12 @@ def mm_bf16_nvfp4(a: torch.Tensor, b: torch.Tensor, b_descale: torch.Tensor, alp
     if out.dtype != torch.bfloat16 or out.shape != (m, n) or out.stride(1) != 1:
         raise ValueError("out must be bf16 [M, N] with unit column stride")
     lib = _lib.load()
-    ws = None
+    ws, stream = None, _stream()
     need = int(lib.b200moe_gemm_bf16_nvfp4_workspace_bytes(m, n, k)) if split_k else 0
     if need:
-        # from the caching allocator per call: ordered with the current stream, so calls on other streams and threads keep apart
-        ws = torch.empty(need, dtype=torch.uint8, device=a.device)
+        ws = _w4a16_workspace(a.device, stream, need)
     _lib.check(lib.b200moe_gemm_bf16_nvfp4(a.data_ptr(), a.stride(0), b.data_ptr(), b_descale.data_ptr(), _ptr(alpha), out.data_ptr(),
-                                           m, n, k, out.stride(0), _ptr(ws), need, _ptr(status), _stream()),
+                                           m, n, k, out.stride(0), _ptr(ws), need, _ptr(status), stream),
                "b200moe_gemm_bf16_nvfp4")
     return out
 

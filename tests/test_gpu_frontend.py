@@ -243,3 +243,21 @@ def test_route_map_all_invalid():
     assert ws["totals"].cpu().tolist() == [0, 0, 0, 0]
     assert bool((ws["row_of"][:64] == -1).all())
     layer.close()
+
+
+@pytest.mark.parametrize("t,e,k", [(4096, 128, 8), (4097, 256, 8), (4099, 200, 3), (5002, 8, 8), (4098, 33, 1)])
+def test_topk_four_tokens_per_warp_equals_one(t, e, k):
+    """From 4096 tokens on a warp takes four tokens (K <= 8): the same ids and the same weight bits as slices below that size, with
+    ties, both zeros, NaN and rows that have fewer selectable logits than K."""
+    import kernelschema_b200 as ks
+    gen = torch.Generator(device="cuda").manual_seed(t + e)
+    logits = torch.randn(t, e, device="cuda", generator=gen)
+    logits[::5] = torch.round(logits[::5])                   # ties, among them +0 and -0
+    logits[3::7, ::3] = float("nan")
+    logits[2::11, 1:] = float("-inf")
+    bias = torch.randn(e, device="cuda", generator=gen)
+    for b in (None, bias):
+        ids, w = ks.route_topk(logits, k, b)
+        for t0 in range(0, t, 4000):
+            i1, w1 = ks.route_topk(logits[t0:t0 + 4000], k, b)
+            assert torch.equal(ids[t0:t0 + 4000], i1) and torch.equal(w[t0:t0 + 4000].view(torch.int32), w1.view(torch.int32))

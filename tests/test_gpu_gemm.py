@@ -191,6 +191,20 @@ def test_w4a16_strided_a_and_no_alpha():
     assert r["rel_l2"] <= 1e-3, r
 
 
+@pytest.mark.parametrize("m,n,k", [(2047, 2048, 4096), (2048, 2048, 4096), (2049, 1024, 4352), (2048, 2048, 3840)])
+def test_dense_both_sides_of_the_long_loop_form(m, n, k):
+    """K >= 4096 and M >= 2048 copies the scale factors in line with eight epilogue warps, other launches use copier warps:
+    the same bits as 128-wide tiles on both sides of each limit (same products, same order along K)."""
+    import kernelschema_b200 as ks
+    gen = torch.Generator(device="cuda").manual_seed(m + k)
+    aq, asf = ks.nvfp4_quantize(torch.randn(m, k, device="cuda", generator=gen).to(torch.bfloat16), tiled_scales=True)
+    bq, bsf = ks.nvfp4_quantize(torch.randn(n, k, device="cuda", generator=gen).to(torch.bfloat16), tiled_scales=True)
+    wide = ks.mm_nvfp4(aq, asf, bq, bsf, tile_n=256)
+    narrow = ks.mm_nvfp4(aq, asf, bq, bsf, tile_n=128)
+    torch.cuda.synchronize()
+    assert torch.equal(wide, narrow) and wide.float().abs().mean() > 1
+
+
 @pytest.mark.parametrize("m,n,k", [(33, 4096, 8192), (128, 4096, 8192), (129, 256, 256), (300, 1024, 1280), (513, 4096, 4096), (2600, 4096, 4096),
                                    (3000, 3328, 4352)])
 def test_w4a16_split_last_wave(m, n, k):
@@ -212,6 +226,35 @@ def test_w4a16_split_last_wave(m, n, k):
     ref, mag = 1.25 * a.double() @ w.T, 1.25 * a.double().abs() @ w.abs().T
     for got in (y, plain):          # one bf16 rounding, and 2^-20 of the magnitudes for the fp32 sums
         assert ((got.double() - ref).abs() <= ref.abs() / 256 + mag * 2.0 ** -20).all()
+
+
+def test_w4a16_split_on_two_streams_and_in_a_graph():
+    """Calls on different streams keep apart (each stream its own scratch), and a captured call still gives its result after
+    larger calls have replaced the stream's scratch."""
+    import kernelschema_b200 as ks
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    m, n, k = 300, 2048, 4096
+    a = [torch.randn(m, k, device="cuda", generator=gen).to(torch.bfloat16) for _ in range(2)]
+    bq, bsf = ks.nvfp4_quantize((torch.randn(n, k, device="cuda", generator=gen) * k ** -0.5).to(torch.bfloat16), 1.0)
+    bsf = bsf.view(torch.uint8)
+    want = [ks.mm_bf16_nvfp4(x, bq, bsf) for x in a]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    outs = [[torch.empty_like(want[0]) for _ in range(20)] for _ in range(2)]
+    for r in range(20):
+        for i, st in enumerate(streams):
+            with torch.cuda.stream(st):
+                ks.mm_bf16_nvfp4(a[i], bq, bsf, out=outs[i][r])
+    torch.cuda.synchronize()
+    assert all(torch.equal(outs[i][r], want[i]) for i in range(2) for r in range(20))
+    out = torch.empty_like(want[0])
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ks.mm_bf16_nvfp4(a[0], bq, bsf, out=out)
+    ks.mm_bf16_nvfp4(torch.cat((a[0], a[1], a[0])), bq, bsf)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want[0])
 
 
 def test_w4a16_linearity_full_size():
