@@ -6,7 +6,8 @@
 // schema_wiki/.../nvfp4_fused_moe/root.yaml:172-197), with one tightening: the position of a route
 // inside its expert segment is its rank in ascending flat index t*K+k (the reference leaves that
 // order arbitrary), so every integer output is reproducible and can be compared bit for bit.
-// No atomics: three passes (block histograms, scan, stable scatter).
+// No global atomics. One launch for small builds (with the permute, where that applies), histograms + scan-and-scatter for
+// larger ones, a scan launch of its own beyond kHistMaxBlocks chunks.
 #include "kernels.cuh"
 #include "ptx.cuh"
 #include "topk.cuh"
