@@ -888,7 +888,7 @@ static int step_impl(b200moe_layer* h, const b200moe_step_args* a, cudaStream_t 
   // inside the route-map launch (Qwen3, T = 1: seven launches to five, 27.5 -> 26.3 us).
   const bool one_front = c.top_k > 0 && router_small_wins(T, c.hidden, c.num_experts) && T <= 8 && a->x_stride == c.hidden &&
                          quantize_fast(a->activation_global_scale);
-  const bool topk_in_map = c.top_k > 0 && T <= kTopkGatherTokens && c.num_experts <= 256 && (int64_t)T * h->kk <= 1024 &&
+  const bool topk_in_map = c.top_k > 0 && route_gather_topk_fits(T, c.top_k, c.num_shared_experts, c.num_experts, sm_count()) &&
                            route_gather_fits(T, c.top_k, c.num_shared_experts, c.num_experts, c.hidden);
   int rc = 0, rc_router = 0;
   const char* where = "step: quantise";

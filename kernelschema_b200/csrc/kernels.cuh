@@ -121,9 +121,21 @@ int launch_route_map(const int32_t* ids, const float* scores, int64_t id_stride,
                      RouteMapBuffers b, cudaStream_t st, int seg_len = 0, const int32_t* seg_valid = nullptr);
 // Route map and permute in ONE launch for batches of at most 16384 routes with row-major token scales (decode sizes):
 // `route_gather_fits` says whether a call qualifies.
-// With `topk` the expert ids come from router logits inside the launch (T <= kTopkGatherTokens, E <= 256); `ids` / `scores` are
-// then unused and the selection is also stored to topk->ids / topk->weights.
+// With `topk` the expert ids come from router logits inside the launch (`route_gather_topk_fits` says whether a call qualifies);
+// `ids` / `scores` are then unused and the selection is also stored to topk->ids / topk->weights.
 constexpr int kTopkGatherTokens = 8;
+constexpr int kTopkGatherThreads = 256;
+// Routes that a block of the one-launch form owns: one row per warp while the SMs last.
+inline int route_gather_chunk(int64_t total, int threads, int sms) {
+  const int64_t want = (total + threads / 32 - 1) / (threads / 32), blocks = want < sms ? want : sms;
+  return (int)((total + blocks - 1) / blocks);
+}
+// One token per warp, at most 8 experts per lane, and one warp that owns a block's routes: at most 32 of them.
+inline bool route_gather_topk_fits(int64_t T, int K, int S, int E, int sms) {
+  const int64_t total = T * (K + S);
+  return T >= 1 && T <= kTopkGatherTokens && K >= 1 && K <= 32 && E <= 256 && total <= 1024 &&
+         route_gather_chunk(total, kTopkGatherThreads, sms) <= 32;
+}
 struct TopkView {
   const float* logits;
   const float* bias;

@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(kRouteThreads) k_route_scatter(RouteView r, co
 constexpr int kFusedMaxBlocks = 8;
 constexpr int kHistMaxBlocks = 128;              // beyond, every block reading every count costs more than the scan launch
 constexpr int kGatherMaxRoutes = 16384;          // the fused form that also permutes the rows
-constexpr int kGatherMaxChunk = 256;             // routes a block of it may own (8 warps)
+constexpr int kGatherMaxChunk = 256;             // routes a block of it may own (8 warps); 32 where it selects the experts itself
 
 // The permute of one routed row from inside the route-map kernel (small batches): payload with 16-byte vectors, the row's
 // scale words straight into the 128x4-tiled image. Scales of padding rows are left as they are: the GEMMs neither store
@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(kRouteThreads) k_route_fused(RouteView r, cons
 // TOPK: a decode batch straight from router logits (one token per warp, at most 256 experts): every block selects the experts of
 // all tokens itself, block 0 stores them.
 template <int OW, bool TOPK>                       // OW = warps that own routes
-__global__ void __launch_bounds__(TOPK ? 256 : kRouteThreads) k_route_gather(RouteView r, const float* scores, int etot,
+__global__ void __launch_bounds__(TOPK ? kTopkGatherThreads : kRouteThreads) k_route_gather(RouteView r, const float* scores, int etot,
                                                                             int chunk, RouteMapBuffers b, GatherView gv, TopkView tk) {
   extern __shared__ int hist[];                    // own routes [OW][etot] | routes after [etot] | before [etot] | own positions [OW * 32]
   __shared__ int32_t s_ids[TOPK ? kTopkGatherTokens * 32 : 1];
@@ -610,16 +610,9 @@ int launch_route_map(const int32_t* ids, const float* scores, int64_t id_stride,
   return (int)err;
 }
 
-// Blocks of the one-launch form: one row per warp while the SMs last.
-static int route_gather_blocks(int64_t total, int threads) {
-  const int64_t blocks = (total + threads / 32 - 1) / (threads / 32);
-  return (int)(blocks < sm_count() ? blocks : sm_count());
-}
-
 bool route_gather_fits(int64_t T, int K, int S, int E, int H) {
   const int64_t total = T * (K + S);
-  return total >= 1 && total <= kGatherMaxRoutes && total <= (int64_t)route_gather_blocks(total, kRouteThreads) * kGatherMaxChunk &&
-         H % 256 == 0;
+  return total >= 1 && total <= kGatherMaxRoutes && route_gather_chunk(total, kRouteThreads, sm_count()) <= kGatherMaxChunk && H % 256 == 0;
 }
 
 int launch_route_gather(const int32_t* ids, const float* scores, int64_t id_stride, int64_t T, int K, int S, int E, int expert_offset,
@@ -631,16 +624,15 @@ int launch_route_gather(const int32_t* ids, const float* scores, int64_t id_stri
   GatherView gv{(const uint8_t*)hid_q, (const uint8_t*)hid_sf, q_stride > 0 ? q_stride : (int64_t)(H / 2),
                 sf_stride > 0 ? sf_stride : (int64_t)(H / 16), H, (uint8_t*)a_q, (uint8_t*)a_sf};
   // a handful of routes: a small block, whose barriers and zeroing cost less (T = 1: 2 us per step)
-  if (topk && (T > kTopkGatherTokens || E > 256)) return 704;
-  const int threads = total <= 256 || topk ? 256 : kRouteThreads;
-  const int blocks = route_gather_blocks(total, threads);
-  const int chunk = (int)((total + blocks - 1) / blocks);
+  if (topk && !route_gather_topk_fits(T, K, S, E, sm_count())) return 704;
+  const int threads = total <= 256 || topk ? kTopkGatherThreads : kRouteThreads;
+  const int chunk = route_gather_chunk(total, threads, sm_count());
   auto go = [&](auto kern, int ow) {               // at most (8 + 2) x 1024 counters + 256 positions: 41 KB
     return (int)launch_chain(kern, dim3((unsigned)((total + chunk - 1) / chunk)), dim3(threads),
                              sizeof(int) * ((ow + 2) * (size_t)etot + 32 * (size_t)ow), st, r, scores, etot, chunk, b, gv,
                              topk ? *topk : TopkView{});
   };
-  if (topk) return go(k_route_gather<1, true>, 1);       // at most 8 x 64 routes over blocks of 8
+  if (topk) return go(k_route_gather<1, true>, 1);
   if (chunk <= 32) return go(k_route_gather<1, false>, 1);
   if (chunk <= 64) return go(k_route_gather<2, false>, 2);
   if (chunk <= 128) return go(k_route_gather<4, false>, 4);
