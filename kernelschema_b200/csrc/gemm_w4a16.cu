@@ -23,8 +23,9 @@
 // r * 128 + ((c ^ (r & 7)) * 16)), then fence.proxy.async + mbarrier arrive; the last 8 warps = epilogue.
 // Every wait is bounded and reports through the status word.
 //
-// The tiles of a last, partly filled wave are split along K (fp32 partial tiles, added in split order by k_w4a16_reduce) as long
-// as that fills the idle SMs; a problem with fewer tiles than SMs is all tail.
+// Up to 128 rows the tiles of a last, partly filled wave are split along K (fp32 partial tiles, added in split order by
+// k_w4a16_reduce) as long as that fills the idle SMs; a problem with fewer tiles than SMs is all tail. From 129 rows on nothing is
+// split: every element is one sum in ascending k, whatever tile and batch its row sits in.
 #include "kernels.cuh"
 #include "ptx.cuh"
 
@@ -58,7 +59,7 @@ struct W4A16Params {
   int M, N, K;
   int32_t* status;
   // Tiles from `full_tiles` on are shared by `splits` CTAs, each of which reduces `groups_per_split` k-groups of 256 and writes
-  // fp32 sums to partial[split][tile - full_tiles][256][BN]. splits == 1: no workspace, full_tiles = all tiles.
+  // fp32 sums to partial[split][tile - full_tiles][M][BN] (M <= 128: one row tile). splits == 1: no workspace, full_tiles = all.
   int full_tiles, tail_tiles;
   int splits;
   int groups_per_split;
@@ -354,8 +355,7 @@ k_gemm_w4a16(const __grid_constant__ CUtensorMap tm_a, const W4A16Params p) {
       const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + buf * 2 * BN + half * BN;
       const int split = item_split(item);
       float* partial_row = split < 0 || p.splits == 1 ? nullptr
-                                                      : p.partial + (((size_t)split * p.tail_tiles + (tile - p.full_tiles)) * 256 +
-                                                                     (half * 128 + quad * 32 + lane)) * BN;
+                                                      : p.partial + (((size_t)split * p.tail_tiles + (tile - p.full_tiles)) * p.M + row) * BN;
       store_cols<BN>(p, taddr, row, live, nt * BN, alpha, partial_row, [&]() {
         tc_fence_before();
         __syncwarp();
@@ -377,13 +377,13 @@ __global__ void __launch_bounds__(256) k_w4a16_reduce(const W4A16Params p, int b
   pdl_wait();
   const float alpha = p.alpha ? *p.alpha : 1.0f;
   const int at = ((int)blockIdx.x * (int)blockDim.x + (int)threadIdx.x) * 4;             // four columns of a tile's row
-  const int t = (int)blockIdx.y, tile = p.full_tiles + t, n_nt = p.N / bn;
-  const int row = tile / n_nt * 256 + at / bn, col = tile % n_nt * bn + at % bn;
-  if (at < min(p.M, 256) * bn && row < p.M) {
-    const float* src = p.partial + (size_t)t * 256 * bn + at;
+  const int t = (int)blockIdx.y;
+  const int row = at / bn, col = (p.full_tiles + t) * bn + at % bn;
+  if (row < p.M) {
+    const float* src = p.partial + (size_t)t * p.M * bn + at;
     float4 acc = *reinterpret_cast<const float4*>(src);
     for (int s = 1; s < p.splits; ++s) {
-      const float4 v = *reinterpret_cast<const float4*>(src + (size_t)s * p.tail_tiles * 256 * bn);
+      const float4 v = *reinterpret_cast<const float4*>(src + (size_t)s * p.tail_tiles * p.M * bn);
       acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
     }
     const __nv_bfloat162 lo = __floats2bfloat162_rn(acc.x * alpha, acc.y * alpha), hi = __floats2bfloat162_rn(acc.z * alpha, acc.w * alpha);
@@ -396,9 +396,12 @@ __global__ void __launch_bounds__(256) k_w4a16_reduce(const W4A16Params p, int b
 
 }  // namespace
 
-// Tile width and split of the last wave. The tiles left over after whole waves are shared by as many CTAs as the SMs hold (at most
-// eight, at least one k-group each). Behind whole waves that pays for its partial tiles and the second launch (about 15 us) only
-// when a tile is long: from 16 k-groups on.
+// Tile width and, up to 128 rows, the split of the last wave. The tiles left over after whole waves are shared by as many CTAs as
+// the SMs hold (at most eight, at least one k-group each). Behind whole waves that pays for its partial tiles and the second launch
+// only when a tile is long: from 16 k-groups on. The plan of a batch of 33 to 128 rows does not depend on its rows, so a row has
+// one value in all of them. Above, which tiles end up in the last wave depends on the batch: a split there would give a row other
+// last bits at another position, so there is none (that gives up time: 300 x 4096 x 4096 37 us
+// with a split, 61 without).
 struct W4A16Plan {
   int bn, full_tiles, tail_tiles, splits;
 };
@@ -411,15 +414,15 @@ static W4A16Plan w4a16_plan(int64_t m, int64_t n, int64_t k, int sms) {
   int64_t s = tail ? sms / tail : 1;
   if (s > 8) s = 8;
   if (s > groups) s = groups;
-  if (s < 2 || w4a16_decode_fits(m) || (tiles > tail && groups < 16)) s = 1;
+  if (s < 2 || m > 128 || w4a16_decode_fits(m) || (tiles > tail && groups < 16)) s = 1;
   pl.splits = (int)s;
   pl.tail_tiles = s > 1 ? (int)tail : 0;
   pl.full_tiles = (int)(tiles - pl.tail_tiles);
   return pl;
 }
-static int64_t w4a16_partial_bytes(const W4A16Plan& pl) { return (int64_t)pl.splits * pl.tail_tiles * 256 * pl.bn * 4; }
+static int64_t w4a16_partial_bytes(const W4A16Plan& pl, int64_t m) { return (int64_t)pl.splits * pl.tail_tiles * m * pl.bn * 4; }
 
-int64_t gemm_w4a16_workspace_bytes(int64_t m, int64_t n, int64_t k) { return w4a16_partial_bytes(w4a16_plan(m, n, k, sm_count())); }
+int64_t gemm_w4a16_workspace_bytes(int64_t m, int64_t n, int64_t k) { return w4a16_partial_bytes(w4a16_plan(m, n, k, sm_count()), m); }
 
 template <int BN>
 static int launch_w4a16(const CUtensorMap& ta, const W4A16Params& p, int sms, cudaStream_t st) {
@@ -452,7 +455,7 @@ int launch_gemm_w4a16(const void* a, int64_t a_stride, const void* b_q, const vo
   p.K = (int)k;
   p.status = status;
   p.partial = (float*)workspace;
-  if (pl.splits > 1 && (!workspace || workspace_bytes < w4a16_partial_bytes(pl))) {      // no room for partial tiles: nothing is split
+  if (pl.splits > 1 && (!workspace || workspace_bytes < w4a16_partial_bytes(pl, m))) {      // no room for partial tiles: nothing is split
     pl.full_tiles += pl.tail_tiles;
     pl.tail_tiles = 0;
     pl.splits = 1;
@@ -463,7 +466,7 @@ int launch_gemm_w4a16(const void* a, int64_t a_stride, const void* b_q, const vo
   p.tail_tiles = pl.tail_tiles;
   rc = bn == 256 ? launch_w4a16<256>(ta, p, sms, st) : launch_w4a16<128>(ta, p, sms, st);
   if (rc || p.splits == 1) return rc;
-  const int64_t quads = (m < 256 ? m : 256) * (bn / 4);
+  const int64_t quads = m * (bn / 4);
   return (int)launch_chain(k_w4a16_reduce, dim3((unsigned)((quads + 255) / 256), (unsigned)p.tail_tiles), dim3(256), 0, st, p, bn);
 }
 

@@ -206,10 +206,11 @@ def test_dense_both_sides_of_the_long_loop_form(m, n, k):
 
 
 @pytest.mark.parametrize("m,n,k", [(33, 4096, 8192), (128, 4096, 8192), (129, 256, 256), (300, 1024, 1280), (513, 4096, 4096), (2600, 4096, 4096),
-                                   (3000, 3328, 4352)])
+                                   (3000, 3328, 4352), (77, 20480, 4096), (40, 640, 2304), (128, 45056, 8192)])
 def test_w4a16_split_last_wave(m, n, k):
-    """Problems of fewer tiles than SMs, and a last wave behind whole ones (2600 x 4096: 176 tiles, 28 of them split on 148 SMs):
-    the same sums with and without the workspace up to the order of the fp32 additions, rows beyond M left alone."""
+    """Up to 128 rows: problems of fewer tiles than SMs, and a last wave behind whole ones (20480 columns: 160 tiles, 12 of them split
+    on 148 SMs; 45056: 176 wide tiles, 28 split). More rows: never split. The same sums with and without the workspace up to the
+    order of the fp32 additions, rows beyond M left alone."""
     import kernelschema_b200 as ks
     gen = torch.Generator(device="cuda").manual_seed(m + n)
     a = torch.randn(m, k, device="cuda", generator=gen).to(torch.bfloat16)
@@ -233,7 +234,7 @@ def test_w4a16_split_on_two_streams_and_in_a_graph():
     larger calls have replaced the stream's scratch."""
     import kernelschema_b200 as ks
     gen = torch.Generator(device="cuda").manual_seed(9)
-    m, n, k = 300, 2048, 4096
+    m, n, k = 60, 2048, 4096
     a = [torch.randn(m, k, device="cuda", generator=gen).to(torch.bfloat16) for _ in range(2)]
     bq, bsf = ks.nvfp4_quantize((torch.randn(n, k, device="cuda", generator=gen) * k ** -0.5).to(torch.bfloat16), 1.0)
     bsf = bsf.view(torch.uint8)
@@ -251,10 +252,30 @@ def test_w4a16_split_on_two_streams_and_in_a_graph():
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph):
         ks.mm_bf16_nvfp4(a[0], bq, bsf, out=out)
-    ks.mm_bf16_nvfp4(torch.cat((a[0], a[1], a[0])), bq, bsf)
+    ks.mm_bf16_nvfp4(torch.cat((a[0], a[1])), bq, bsf)
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(out, want[0])
+
+
+@pytest.mark.parametrize("n,k,sizes", [(4096, 4096, (129, 300, 1111, 2600)), (3328, 4352, (200, 3000)), (1152, 8192, (150, 1300)),
+                                       (4096, 8192, (33, 64, 65, 128)), (20480, 4096, (40, 128)), (1024, 4096, (1, 8, 9, 17, 32))])
+def test_w4a16_a_row_has_one_value(n, k, sizes):
+    """A row gives the same bits at any position and in any batch of 1..32, of 33..128 and of more than 128 rows: long K, fewer
+    tiles than SMs as well as a partly filled last wave behind whole ones. Above 128 rows the split changes nothing."""
+    import kernelschema_b200 as ks
+    gen = torch.Generator(device="cuda").manual_seed(n + k)
+    m = sizes[-1]
+    a = torch.randn(m, k, device="cuda", generator=gen).to(torch.bfloat16)
+    bq, bsf = ks.nvfp4_quantize((torch.randn(n, k, device="cuda", generator=gen) * k ** -0.5).to(torch.bfloat16), 1.0)
+    bsf = bsf.view(torch.uint8)
+    y = ks.mm_bf16_nvfp4(a, bq, bsf)
+    perm = torch.randperm(m, device="cuda", generator=gen)
+    assert torch.equal(ks.mm_bf16_nvfp4(a[perm].contiguous(), bq, bsf), y[perm])
+    for t in sizes:
+        assert torch.equal(ks.mm_bf16_nvfp4(a[m - t:], bq, bsf), y[m - t:]), t
+    if m > 128:
+        assert torch.equal(ks.mm_bf16_nvfp4(a, bq, bsf, split_k=False), y)
 
 
 def test_w4a16_linearity_full_size():
