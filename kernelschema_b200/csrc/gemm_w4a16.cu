@@ -400,21 +400,23 @@ __global__ void __launch_bounds__(256) k_w4a16_reduce(const W4A16Params p, int b
 // the SMs hold (at most eight, at least one k-group each). Behind whole waves that pays for its partial tiles and the second launch
 // only when a tile is long: from 16 k-groups on. The plan of a batch of 33 to 128 rows does not depend on its rows, so a row has
 // one value in all of them. Above, which tiles end up in the last wave depends on the batch: a split there would give a row other
-// last bits at another position, so there is none (that gives up time: 300 x 4096 x 4096 37 us
-// with a split, 61 without).
+// last bits at another position, so there is none (that gives up time: 8192 x 4096 x 12288 710 us with a split, 769 without;
+// 300 x 4096 x 4096 39 and 62). `room`: the caller has a workspace for the partial tiles.
 struct W4A16Plan {
   int bn, full_tiles, tail_tiles, splits;
 };
-static W4A16Plan w4a16_plan(int64_t m, int64_t n, int64_t k, int sms) {
+static W4A16Plan w4a16_plan(int64_t m, int64_t n, int64_t k, int sms, bool room) {
   W4A16Plan pl;
-  // up to 128 rows half of a wide tile's accumulators idle: it pays when the tiles are many and long (M = 64, N = 4096,
-  // K = 12288: 31 us against 36 us; N = 2048, K = 4096: 16 against 12)
-  pl.bn = n % 256 == 0 && (m > 128 || (n >= 4096 && k >= 8192)) ? 256 : 128;
+  // Up to 128 rows half of a wide tile's accumulators idle: it pays when the tiles are long and fill the device, by their number
+  // (M = 64, N = 25600, K = 8192: 120 us against 158) or by a split that there is room for (M = 64, N = 4096, K = 12288: 31 us against
+  // 36; N = 2048, K = 4096: 16 against 12). A split that falls away leaves half as many CTAs as narrow tiles do (M = 64, N = 4096,
+  // K = 8192: 116 us against 81; M = 128, N = 8192, K = 12288: 179 against 120).
+  pl.bn = n % 256 == 0 && (m > 128 || (room && n >= 4096 && k >= 8192)) ? 256 : 128;
   const int64_t tiles = (m + 255) / 256 * (n / pl.bn), groups = k / 256, tail = tiles % sms;
   int64_t s = tail ? sms / tail : 1;
   if (s > 8) s = 8;
   if (s > groups) s = groups;
-  if (s < 2 || m > 128 || w4a16_decode_fits(m) || (tiles > tail && groups < 16)) s = 1;
+  if (s < 2 || !room || m > 128 || w4a16_decode_fits(m) || (tiles > tail && groups < 16)) s = 1;
   pl.splits = (int)s;
   pl.tail_tiles = s > 1 ? (int)tail : 0;
   pl.full_tiles = (int)(tiles - pl.tail_tiles);
@@ -422,7 +424,7 @@ static W4A16Plan w4a16_plan(int64_t m, int64_t n, int64_t k, int sms) {
 }
 static int64_t w4a16_partial_bytes(const W4A16Plan& pl, int64_t m) { return (int64_t)pl.splits * pl.tail_tiles * m * pl.bn * 4; }
 
-int64_t gemm_w4a16_workspace_bytes(int64_t m, int64_t n, int64_t k) { return w4a16_partial_bytes(w4a16_plan(m, n, k, sm_count()), m); }
+int64_t gemm_w4a16_workspace_bytes(int64_t m, int64_t n, int64_t k) { return w4a16_partial_bytes(w4a16_plan(m, n, k, sm_count(), true), m); }
 
 template <int BN>
 static int launch_w4a16(const CUtensorMap& ta, const W4A16Params& p, int sms, cudaStream_t st) {
@@ -439,7 +441,8 @@ int launch_gemm_w4a16(const void* a, int64_t a_stride, const void* b_q, const vo
   if (m == 0) return 0;
   if (w4a16_decode_fits(m)) return launch_gemm_w4a16_decode(a, a_stride, b_q, b_sf, alpha, m, n, k, out, out_stride, st);
   const int sms = sm_count();
-  W4A16Plan pl = w4a16_plan(m, n, k, sms);
+  W4A16Plan pl = w4a16_plan(m, n, k, sms, true);
+  if (pl.splits > 1 && (!workspace || workspace_bytes < w4a16_partial_bytes(pl, m))) pl = w4a16_plan(m, n, k, sms, false);
   const int bn = pl.bn;
   CUtensorMap ta;
   int rc = make_operand_map(&ta, a, (uint64_t)m, (uint64_t)k * 2, 256, (uint64_t)a_stride * 2);
@@ -455,11 +458,6 @@ int launch_gemm_w4a16(const void* a, int64_t a_stride, const void* b_q, const vo
   p.K = (int)k;
   p.status = status;
   p.partial = (float*)workspace;
-  if (pl.splits > 1 && (!workspace || workspace_bytes < w4a16_partial_bytes(pl, m))) {      // no room for partial tiles: nothing is split
-    pl.full_tiles += pl.tail_tiles;
-    pl.tail_tiles = 0;
-    pl.splits = 1;
-  }
   p.groups_per_split = (int)((k / 256 + pl.splits - 1) / pl.splits);
   p.splits = (int)((k / 256 + p.groups_per_split - 1) / p.groups_per_split);              // no empty split
   p.full_tiles = pl.full_tiles;
