@@ -496,7 +496,7 @@ int b200moe_gemm_bf16_nvfp4(const void* a, int64_t a_stride, const void* b_q, co
     return fail(769, "gemm_bf16_nvfp4: out must be 32-byte aligned, out_stride >= N and a multiple of 16");
   if (workspace && ((uintptr_t)workspace & 15)) return fail(769, "gemm_bf16_nvfp4: workspace must be 16-byte aligned");
   return cuda_fail(launch_gemm_w4a16(a, a_stride, b_q, b_descale, alpha, m, n, k, out, out_stride, workspace,
-                                     workspace ? workspace_bytes : 0, status, (cudaStream_t)stream),
+                                     workspace || workspace_bytes < 0 ? workspace_bytes : 0, status, (cudaStream_t)stream),
                    "gemm_bf16_nvfp4");
 }
 

@@ -439,7 +439,8 @@ int launch_gemm_w4a16(const void* a, int64_t a_stride, const void* b_q, const vo
                       int64_t k, void* out, int64_t out_stride, void* workspace, int64_t workspace_bytes, int32_t* status,
                       cudaStream_t st) {
   if (m == 0) return 0;
-  if (w4a16_decode_fits(m)) return launch_gemm_w4a16_decode(a, a_stride, b_q, b_sf, alpha, m, n, k, out, out_stride, st);
+  // workspace_bytes < 0: one sum in ascending k per element at every size, so the tile kernel, unsplit
+  if (workspace_bytes >= 0 && w4a16_decode_fits(m)) return launch_gemm_w4a16_decode(a, a_stride, b_q, b_sf, alpha, m, n, k, out, out_stride, st);
   const int sms = sm_count();
   W4A16Plan pl = w4a16_plan(m, n, k, sms, true);
   if (pl.splits > 1 && (!workspace || workspace_bytes < w4a16_partial_bytes(pl, m))) pl = w4a16_plan(m, n, k, sms, false);

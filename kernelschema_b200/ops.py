@@ -162,7 +162,9 @@ def mm_bf16_nvfp4(a: torch.Tensor, b: torch.Tensor, b_descale: torch.Tensor, alp
                   out: torch.Tensor | None = None, status: torch.Tensor | None = None, split_k: bool = True) -> torch.Tensor:
     """out[M, N] = bf16(alpha * a @ decode(b)^T): bf16 activations [M, K] (not quantised), NVFP4 weights uint8 [N, K/2] with
     row-major E4M3 scales [N, K/16], alpha a 1-element fp32 device tensor or None (the dense operator's contract,
-    gemm/dense/bf16_nvfp4_gemm/problem/reference.py:10-15)."""
+    gemm/dense/bf16_nvfp4_gemm/problem/reference.py:10-15). A row of ``a`` gives the same bits in all batches of 1..32, of 33..128
+    and of more than 128 rows; between the three the order of the additions along K differs. ``split_k=False`` gives it the
+    same bits in every batch (slow for few rows)."""
     _need_cuda(a, b, b_descale, out, alpha)
     if a.dtype != torch.bfloat16 or a.dim() != 2 or a.stride(1) != 1:
         raise ValueError("a must be a bf16 matrix with unit column stride")
@@ -178,8 +180,8 @@ def mm_bf16_nvfp4(a: torch.Tensor, b: torch.Tensor, b_descale: torch.Tensor, alp
         raise ValueError("out must be bf16 [M, N] with unit column stride")
     lib = _lib.load()
     ws, stream = None, _stream()
-    need = int(lib.b200moe_gemm_bf16_nvfp4_workspace_bytes(m, n, k)) if split_k else 0
-    if need:
+    need = int(lib.b200moe_gemm_bf16_nvfp4_workspace_bytes(m, n, k)) if split_k else -1
+    if need > 0:
         ws = _w4a16_workspace(a.device, stream, need)
     _lib.check(lib.b200moe_gemm_bf16_nvfp4(a.data_ptr(), a.stride(0), b.data_ptr(), b_descale.data_ptr(), _ptr(alpha), out.data_ptr(),
                                            m, n, k, out.stride(0), _ptr(ws), need, _ptr(status), stream),

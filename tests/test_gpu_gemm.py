@@ -262,7 +262,8 @@ def test_w4a16_split_on_two_streams_and_in_a_graph():
                                        (4096, 8192, (33, 64, 65, 128)), (20480, 4096, (40, 128)), (1024, 4096, (1, 8, 9, 17, 32))])
 def test_w4a16_a_row_has_one_value(n, k, sizes):
     """A row gives the same bits at any position and in any batch of 1..32, of 33..128 and of more than 128 rows: long K, fewer
-    tiles than SMs as well as a partly filled last wave behind whole ones. Above 128 rows the split changes nothing."""
+    tiles than SMs as well as a partly filled last wave behind whole ones. With split_k=False the bits are those of more than 128
+    rows at every size."""
     import kernelschema_b200 as ks
     gen = torch.Generator(device="cuda").manual_seed(n + k)
     m = sizes[-1]
@@ -274,8 +275,11 @@ def test_w4a16_a_row_has_one_value(n, k, sizes):
     assert torch.equal(ks.mm_bf16_nvfp4(a[perm].contiguous(), bq, bsf), y[perm])
     for t in sizes:
         assert torch.equal(ks.mm_bf16_nvfp4(a[m - t:], bq, bsf), y[m - t:]), t
-    if m > 128:
-        assert torch.equal(ks.mm_bf16_nvfp4(a, bq, bsf, split_k=False), y)
+    # without a split the three ranges agree as well
+    plain = ks.mm_bf16_nvfp4(a.repeat(200 // m + 1, 1)[:max(m, 200)], bq, bsf)
+    for t in (1, 8, 16, 17, 32, 33, 128, *sizes):
+        if t <= m:
+            assert torch.equal(ks.mm_bf16_nvfp4(a[:t], bq, bsf, split_k=False), plain[:t]), t
 
 
 def test_w4a16_linearity_full_size():
