@@ -15,7 +15,7 @@
 // contiguous bytes; fetched by the fragments' own addresses a load touches 32 lines), kept in fragment order.
 //
 // Split: 8 warps of a block take the units of K in turn, and a cluster of C blocks splits K further while (N / 64) * C blocks
-// fit two per SM. Partial sums meet in shared memory, then in distributed shared memory, each time in a fixed order
+// are resident at once: two per SM up to 16 tokens, one above (255 registers). Partial sums meet in shared memory, then in distributed shared memory, each time in a fixed order
 // (reproducible, no workspace, one launch).
 #include "kernels.cuh"
 #include "ptx.cuh"
@@ -64,8 +64,12 @@ constexpr int dec_smem_bytes() {
   return x > part ? x : part;
 }
 
+// Blocks an SM holds: the fragments of 32 tokens take 255 registers a thread.
 template <int NT>
-__global__ void __launch_bounds__(32 * kDecWarps, NT <= 2 ? 2 : 1)
+constexpr int dec_blocks_per_sm() { return NT <= 2 ? 2 : 1; }
+
+template <int NT>
+__global__ void __launch_bounds__(32 * kDecWarps, dec_blocks_per_sm<NT>())
 k_gemm_w4a16_decode(const __nv_bfloat16* __restrict__ a, int64_t a_stride, const uint8_t* __restrict__ b_q,
                     const uint8_t* __restrict__ b_sf, const float* __restrict__ alpha_ptr, __nv_bfloat16* __restrict__ out,
                     int64_t out_stride, int M, int K, int split) {
@@ -197,7 +201,13 @@ k_gemm_w4a16_decode(const __nv_bfloat16* __restrict__ a, int64_t a_stride, const
 
 template <int NT>
 int launch_nt(const void* a, int64_t a_stride, const void* b_q, const void* b_sf, const float* alpha, int64_t m, int64_t n, int64_t k,
-              void* out, int64_t out_stride, int split, cudaStream_t st) {
+              void* out, int64_t out_stride, cudaStream_t st) {
+  // Blocks per row tile: double while all are resident at once and the added blocks would have K to work on. Counting two per SM
+  // for 32 tokens, of which one is resident, made two uneven waves of clusters (32 x 2048 x 7168 22.4 us against 12.4 with one,
+  // 32 x 8192 x 12288 56.7 against 50.5; 32 x 7168 x 18432, whose 112 tiles are one short wave, 78.7 against 83.5).
+  const int64_t tiles = n / kDecRows, units = k / kDecUnit, slots = (int64_t)sm_count() * dec_blocks_per_sm<NT>();
+  int split = 1;
+  while (split < 8 && tiles * split * 2 <= slots && units > (int64_t)split * kDecWarps) split *= 2;
   static SmemOptIn opt_in;
   if (int e = opt_in.ensure(k_gemm_w4a16_decode<NT>, dec_smem_bytes<NT>())) return e;
   cudaLaunchConfig_t cfg = {};
@@ -224,13 +234,9 @@ bool w4a16_decode_fits(int64_t m) { return m <= kW4A16DecodeMaxM; }
 
 int launch_gemm_w4a16_decode(const void* a, int64_t a_stride, const void* b_q, const void* b_sf, const float* alpha, int64_t m,
                              int64_t n, int64_t k, void* out, int64_t out_stride, cudaStream_t st) {
-  // blocks per row tile: double while two blocks per SM still hold the grid and the added blocks would have K to work on
-  const int64_t tiles = n / kDecRows, units = k / kDecUnit, slots = (int64_t)sm_count() * 2;
-  int split = 1;
-  while (split < 8 && tiles * split * 2 <= slots && units > (int64_t)split * kDecWarps) split *= 2;
-  if (m <= 8) return launch_nt<1>(a, a_stride, b_q, b_sf, alpha, m, n, k, out, out_stride, split, st);
-  if (m <= 16) return launch_nt<2>(a, a_stride, b_q, b_sf, alpha, m, n, k, out, out_stride, split, st);
-  return launch_nt<4>(a, a_stride, b_q, b_sf, alpha, m, n, k, out, out_stride, split, st);
+  if (m <= 8) return launch_nt<1>(a, a_stride, b_q, b_sf, alpha, m, n, k, out, out_stride, st);
+  if (m <= 16) return launch_nt<2>(a, a_stride, b_q, b_sf, alpha, m, n, k, out, out_stride, st);
+  return launch_nt<4>(a, a_stride, b_q, b_sf, alpha, m, n, k, out, out_stride, st);
 }
 
 }  // namespace b200

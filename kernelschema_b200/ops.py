@@ -162,8 +162,8 @@ def mm_bf16_nvfp4(a: torch.Tensor, b: torch.Tensor, b_descale: torch.Tensor, alp
                   out: torch.Tensor | None = None, status: torch.Tensor | None = None, split_k: bool = True) -> torch.Tensor:
     """out[M, N] = bf16(alpha * a @ decode(b)^T): bf16 activations [M, K] (not quantised), NVFP4 weights uint8 [N, K/2] with
     row-major E4M3 scales [N, K/16], alpha a 1-element fp32 device tensor or None (the dense operator's contract,
-    gemm/dense/bf16_nvfp4_gemm/problem/reference.py:10-15). A row of ``a`` gives the same bits in all batches of 1..32, of 33..128
-    and of more than 128 rows; between the three the order of the additions along K differs. ``split_k=False`` gives it the
+    gemm/dense/bf16_nvfp4_gemm/problem/reference.py:10-15). A row of ``a`` gives the same bits in all batches of 1..16, 17..32,
+    33..128 and more than 128 rows; between these ranges the order of the additions along K differs. ``split_k=False`` gives it the
     same bits in every batch (slow for few rows)."""
     _need_cuda(a, b, b_descale, out, alpha)
     if a.dtype != torch.bfloat16 or a.dim() != 2 or a.stride(1) != 1:
