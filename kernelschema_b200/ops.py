@@ -3,6 +3,7 @@ computation runs in libb200moe.so and a missing library or a non-CUDA tensor is 
 from __future__ import annotations
 
 import ctypes as C
+import threading
 
 import torch
 
@@ -140,21 +141,26 @@ def mm_nvfp4(a_q, a_sf_tiled, b_q, b_sf_tiled, alpha: float = 1.0, out: torch.Te
     return out
 
 
-_W4A16_WORKSPACE: dict = {}     # (device index, stream) -> split-K scratch
+_W4A16_WORKSPACE = threading.local()     # .kept: (device index, stream) -> split-K scratch of the calling thread
 
 
 def _w4a16_workspace(device: torch.device, stream: int, need: int) -> torch.Tensor:
-    """Scratch of the current stream: calls on one stream follow one another, calls on different streams never share. At most
-    eight streams keep one; a buffer that is let go returns to the caching allocator of its own stream. While the stream is being
-    captured the buffer belongs to the graph's pool instead, so that a replay never sees a buffer that has been replaced."""
+    """Scratch of this thread's calls on the current stream. A call is two launches (partial sums, their reduction); another thread
+    may launch between the two on the same stream, so threads never share a buffer, and neither do streams. A thread keeps at
+    most eight; a buffer that is let go, by a ninth stream or at the thread's end, returns to the caching allocator of its own
+    stream. While the stream is being captured the buffer belongs to the graph's pool instead, so that a replay never sees a
+    buffer that has been replaced."""
     if torch.cuda.is_current_stream_capturing():
         return torch.empty(need, dtype=torch.uint8, device=device)
+    kept = getattr(_W4A16_WORKSPACE, "kept", None)
+    if kept is None:
+        kept = _W4A16_WORKSPACE.kept = {}
     key = (device.index, stream)
-    ws = _W4A16_WORKSPACE.get(key)
+    ws = kept.get(key)
     if ws is None or ws.numel() < need:
-        if ws is None and len(_W4A16_WORKSPACE) >= 8:
-            _W4A16_WORKSPACE.pop(next(iter(_W4A16_WORKSPACE)), None)
-        ws = _W4A16_WORKSPACE[key] = torch.empty(need, dtype=torch.uint8, device=device)
+        if ws is None and len(kept) >= 8:
+            del kept[next(iter(kept))]
+        ws = kept[key] = torch.empty(need, dtype=torch.uint8, device=device)
     return ws
 
 

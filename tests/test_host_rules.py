@@ -1,6 +1,8 @@
 """CPU-only checks of the host rules that size launches: a small program includes the launch header and walks every form a rule accepts."""
 import os
 import subprocess
+import sys
+import threading
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
@@ -38,3 +40,37 @@ def test_selection_inside_the_route_map_owns_at_most_one_warp_of_routes(tmp_path
   printf("%d %d", widest, full);
   return 0;""")
     assert int(widest) == 32 and int(full) == 1
+
+
+def test_split_k_scratch_of_many_threads(monkeypatch):
+    """Threads that use more streams than a thread keeps scratch for: every call gets a buffer that no other thread holds, nothing
+    raises while buffers are replaced, and each thread keeps at most eight."""
+    import torch
+    from kernelschema_b200 import ops
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    held, errors, kept = [set() for _ in range(12)], [], [0] * 12
+    done = threading.Barrier(12)
+
+    def work(i):
+        try:
+            for j in range(1500):
+                ws = ops._w4a16_workspace(torch.device("cpu"), (i + j * 5) % 24, 64 + (j % 3) * 64)
+                assert ws.numel() >= 64 + (j % 3) * 64
+            mine = ops._W4A16_WORKSPACE.kept
+            held[i], kept[i] = {w.data_ptr() for w in mine.values()}, len(mine)
+        except Exception as exc:
+            errors.append(repr(exc))
+        done.wait(60)                                   # the buffers of all threads are alive at the same time
+
+    interval = sys.getswitchinterval()
+    sys.setswitchinterval(1e-6)
+    try:
+        threads = [threading.Thread(target=work, args=(i,)) for i in range(12)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+    finally:
+        sys.setswitchinterval(interval)
+    assert not errors, errors
+    assert max(kept) <= 8 and len(set().union(*held)) == sum(kept)
