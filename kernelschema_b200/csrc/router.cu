@@ -12,47 +12,23 @@
 
 namespace b200 {
 
-// QUAD: four tokens per warp (K <= 8). Their softmaxes share one pass of the fp64 chain, eight lanes each, which is most of a
-// token's time; the sums add in the same order as with a token per warp, so the weights are the same bits.
-template <int PL, bool QUAD>
+// Bound by the selection's serial chain in every warp, hidden by as many warps as an SM holds. Four tokens per warp, with their
+// softmaxes in one pass of the fp64 chain, quarter those warps: E = 256, T = 8192 24.5 us against 12.7, T = 65536 93.7 against 70.8;
+// E = 128, T = 4096 8.6 against 5.6, T = 65536 44.3 against 45.0.
+template <int PL>
 __global__ void __launch_bounds__(256) k_route_topk(const float* __restrict__ logits, const float* __restrict__ bias, int64_t T,
                                                     int E, int K, int32_t* __restrict__ ids, float* __restrict__ weights) {
   const int lane = threadIdx.x & 31;
-  const int64_t tok = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (QUAD ? 4 : 1);
+  const int64_t tok = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   pdl_trigger();
   pdl_wait();
   if (tok >= T) return;
   int id;
   float weight;
-  if (!QUAD) {
-    topk_token<PL>(logits + tok * E, bias, E, K, lane, id, weight);
-    if (lane < K) {
-      ids[tok * K + lane] = id;
-      weights[tok * K + lane] = weight;
-    }
-    return;
-  }
-  float sel = 0.f;
-  id = -1;
-  uint32_t v[4][PL];
-#pragma unroll
-  for (int j = 0; j < 4; ++j)
-    if (tok + j < T) load_keys<PL>(logits + (tok + j) * E, bias, E, lane, v[j]);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    if (tok + j >= T) break;
-    float s;
-    int e;
-    topk_select<PL>(v[j], K, lane, s, e);
-    s = __shfl_sync(0xFFFFFFFFu, s, lane & 7);
-    e = __shfl_sync(0xFFFFFFFFu, e, lane & 7);
-    if ((lane >> 3) == j) { sel = s; id = e; }
-  }
-  weight = softmax_lanes<8>(sel, K, lane);
-  const int64_t mine = tok + (lane >> 3);
-  if (mine < T && (lane & 7) < K) {
-    ids[mine * K + (lane & 7)] = id;
-    weights[mine * K + (lane & 7)] = weight;
+  topk_token<PL>(logits + tok * E, bias, E, K, lane, id, weight);
+  if (lane < K) {
+    ids[tok * K + lane] = id;
+    weights[tok * K + lane] = weight;
   }
 }
 
@@ -495,18 +471,15 @@ int launch_router_logits_ksplit(const void* x, const void* w, int64_t T, int H, 
 int launch_route_topk(const float* logits, const float* bias, int64_t T, int E, int K, int32_t* ids, float* weights,
                       cudaStream_t st) {
   if (T == 0) return 0;
-  // From a few waves of warps on, four tokens per warp; below, a token's latency counts and the device has room.
-  const bool quad = K <= 8 && E <= 256 && T >= 4096;
-  const unsigned blocks = (unsigned)((T + (quad ? 31 : 7)) / (quad ? 32 : 8));
+  const unsigned blocks = (unsigned)((T + 7) / 8);
   const int per_lane = (E + 31) / 32;
   auto go = [&](auto kern) { return (int)launch_chain(kern, dim3(blocks), dim3(256), 0, st, logits, bias, T, E, K, ids, weights); };
-  if (quad) return per_lane <= 4 ? go(k_route_topk<4, true>) : go(k_route_topk<8, true>);
-  if (per_lane <= 1) return go(k_route_topk<1, false>);
-  if (per_lane <= 2) return go(k_route_topk<2, false>);
-  if (per_lane <= 4) return go(k_route_topk<4, false>);
-  if (per_lane <= 8) return go(k_route_topk<8, false>);
-  if (per_lane <= 16) return go(k_route_topk<16, false>);
-  return go(k_route_topk<32, false>);
+  if (per_lane <= 1) return go(k_route_topk<1>);
+  if (per_lane <= 2) return go(k_route_topk<2>);
+  if (per_lane <= 4) return go(k_route_topk<4>);
+  if (per_lane <= 8) return go(k_route_topk<8>);
+  if (per_lane <= 16) return go(k_route_topk<16>);
+  return go(k_route_topk<32>);
 }
 
 int launch_router_logits(const void* x, const void* w, int64_t T, int H, int E, float* logits, cudaStream_t st) {

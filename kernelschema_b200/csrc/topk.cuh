@@ -67,14 +67,13 @@ DEV void load_keys(const float* __restrict__ logits, const float* __restrict__ b
   }
 }
 
-// Softmax over the selected logits in fp64: groups of WIDTH lanes, of which the first K hold a logit, the largest first.
-template <int WIDTH>
+// Softmax over the selected logits in fp64: the first K lanes hold a logit, the largest first.
 DEV float softmax_lanes(float sel, int K, int lane) {
-  const float top = __shfl_sync(0xFFFFFFFFu, sel, lane & ~(WIDTH - 1));
-  double ex = ((lane & (WIDTH - 1)) < K) ? exp((double)sel - (double)top) : 0.0;
+  const float top = __shfl_sync(0xFFFFFFFFu, sel, 0);
+  double ex = lane < K ? exp((double)sel - (double)top) : 0.0;
   double sum = ex;
 #pragma unroll
-  for (int off = WIDTH / 2; off > 0; off >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, off);
+  for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, off);
   return (float)(ex / sum);
 }
 
@@ -85,7 +84,7 @@ DEV void topk_token(const float* __restrict__ logits, const float* __restrict__ 
   load_keys<PL>(logits, bias, E, lane, v);
   float sel;
   topk_select<PL>(v, K, lane, sel, id);
-  weight = softmax_lanes<32>(sel, K, lane);
+  weight = softmax_lanes(sel, K, lane);
 }
 
 }  // namespace b200

@@ -246,8 +246,8 @@ def test_route_map_all_invalid():
 
 
 @pytest.mark.parametrize("t,e,k", [(4096, 128, 8), (4097, 256, 8), (4099, 200, 3), (5002, 8, 8), (4098, 33, 1)])
-def test_topk_four_tokens_per_warp_equals_one(t, e, k):
-    """From 4096 tokens on a warp takes four tokens (K <= 8): the same ids and the same weight bits as slices below that size, with
+def test_topk_of_a_batch_equals_its_slices(t, e, k):
+    """The same ids and the same weight bits in a large batch as in slices of it, with
     ties, both zeros, NaN and rows that have fewer selectable logits than K."""
     import kernelschema_b200 as ks
     gen = torch.Generator(device="cuda").manual_seed(t + e)
