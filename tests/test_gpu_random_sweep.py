@@ -1,6 +1,6 @@
 """Seeded sweep over small layer geometries against the oracle: expert counts from 1 to 300, 1 to 12 slots per token
-(routed + shared: the combine pass batches eight slots at a time), batches from 1 to 700 tokens (the one-launch route map +
-permute up to 8192 routes, the one-block route map up to 16384, the three-kernel build above), masked routes, Zipf and
+(routed + shared: the combine pass batches eight slots at a time), batches from 1 to 2100 tokens (the one-launch route map +
+permute up to 16384 routes, the two-launch map above), masked routes, Zipf and
 uniform routing, both activation types. Integer tables bit for bit, outputs by the reference's acceptance rule."""
 import numpy as np
 import pytest
@@ -23,8 +23,8 @@ def _cases():
         if e > 64 and t > 300:
             t = 300
         out.append((n, t, h, i, e, k, s, str(rng.choice(["uniform", "zipf"])), bool(rng.integers(0, 2)), int(rng.choice([3, 10]))))
-    out.append((100, 2100, 256, 256, 8, 8, 1, "zipf", True, 3))      # 18 900 routes: hist / scan / scatter kernels
-    out.append((101, 1200, 256, 256, 24, 8, 0, "uniform", False, 3))  # 9 600 routes: the one-block route map, five blocks
+    out.append((100, 2100, 256, 256, 8, 8, 1, "zipf", True, 3))      # 18 900 routes: histograms + scan-and-scatter
+    out.append((101, 1200, 256, 256, 24, 8, 0, "uniform", False, 3))  # 9 600 routes: one launch, blocks of 65 routes
     return out
 
 

@@ -1,4 +1,4 @@
-"""The one-launch route map + permute of small batches (at most 8192 routes, row-major token scales) against the oracle,
+"""The one-launch route map + permute of small batches (at most 16384 routes, row-major token scales) against the oracle,
 on both sides of its size limit, with masked routes and a shared expert, and with rows longer than 8192 elements."""
 import numpy as np
 import pytest
@@ -57,9 +57,9 @@ def _check_map_and_rows(p, model):
 @pytest.mark.parametrize("tma_gather", [False, True])
 @pytest.mark.parametrize("tokens", [1, 3, 37, 512, 1023, 1024, 1025])
 def test_small_batch_map_rows_and_output(tokens, tma_gather):
-    """7 routed slots + 1 shared expert = 8 routes per token: 1024 tokens are exactly 8192 routes (the last size of the
-    one-launch form), 1025 take the separate route-map and permute kernels; both must give the same tables. With the
-    permuted copy of the payload rows and without it (FC1 fetching the token rows by TMA gather)."""
+    """7 routed slots + 1 shared expert = 8 routes per token, all of these sizes in one launch (16384 routes are its last).
+    With the permuted copy of the payload rows and without it (FC1
+    fetching the token rows by TMA gather)."""
     import kernelschema_b200 as ks
     from gpu_util import run_model
     p = make_moe_case(100 + tokens, tokens, 512, 256, 24, 7, shared=1, routing="zipf", masked=tokens > 3)
@@ -101,11 +101,12 @@ def test_small_batch_rows_longer_than_8192():
 
 
 def test_repeat_calls_with_changing_batch_sizes_share_one_layer():
-    """One layer object serves a decode batch, a larger batch (separate kernels) and a decode batch again."""
+    """One layer object serves a large batch (2100 x 8 routes: separate route-map and permute kernels), decode batches (one launch)
+    and the large batch again."""
     import kernelschema_b200 as ks
     from gpu_util import run_model
     model = ks.Model()
-    for tokens in (600, 5, 600, 64):
+    for tokens in (2100, 600, 5, 2100, 64):
         p = make_moe_case(300 + tokens, tokens, 512, 256, 24, 8, routing="zipf")
         p_run = dict(p)
         got, _, model = run_model(p_run, model)
@@ -114,12 +115,13 @@ def test_repeat_calls_with_changing_batch_sizes_share_one_layer():
 
 
 @pytest.mark.parametrize("tma_gather", [False, True])
-def test_large_batch_both_payload_modes(tma_gather):
-    """6000 routes (separate route-map and permute kernels): FC1 reading the token rows by TMA gather and FC1 reading the
+@pytest.mark.parametrize("tokens", [1500, 4100])
+def test_large_batch_both_payload_modes(tokens, tma_gather):
+    """6000 routes (one launch) and 16400 (separate route-map and permute kernels): FC1 reading the token rows by TMA gather and FC1 reading the
     permuted copy give the same result; partially filled tiles (only some gather boxes issued) are the common case here."""
     import kernelschema_b200 as ks
     from gpu_util import run_model
-    p = make_moe_case(77, 1500, 1024, 512, 16, 4, routing="zipf", masked=True)
+    p = make_moe_case(77, tokens, 1024, 512, 16, 4, routing="zipf", masked=True)
     got, _, model = run_model(p, ks.Model(tma_gather=tma_gather))
     _check_map_and_rows(p, model)
     assert_layer_parity(got, o.moe_expected(p), f"tma_gather={tma_gather}")

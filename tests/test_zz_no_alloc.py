@@ -39,11 +39,13 @@ def _call_noalloc(lib, ids, w, t, k, shared, e, offset, cap, tiles):
     return out
 
 
-def test_noalloc_route_map_equals_regular_entry_point_twice():
+@pytest.mark.parametrize("t,e", [(3000, 256), (31000, 24)])
+def test_noalloc_route_map_equals_regular_entry_point_twice(t, e):
+    """27000 routes are two launches, 279000 (and 272007 in the second call) three."""
     import kernelschema_b200 as ks
     from kernelschema_b200 import _lib
     lib = _lib.load()
-    t, k, shared, e, offset = 3000, 8, 1, 256, 0
+    k, shared, offset = 8, 1, 0
     layer = ks.MoELayer(256, 256, e, k, t, num_shared_experts=shared)
     ws = layer.workspace()
     cap, tiles = ws["row_capacity"], ws["tile_capacity"]
