@@ -3,7 +3,7 @@
 // Follows, bit for bit, the reference input generator's quantize():
 //   moe/nvfp4_fused_moe/problem/input.py:53-71            (global scale 1)
 //   gemm/dense/bf16_nvfp4_gemm/problem/input.py:40-64     (global scale != 1)
-// One thread owns one 16-element block: 32 bytes loaded, one 64-bit payload store, a quarter of a scale word.
+// One thread owns one 16-element block: 32 bytes loaded, one 64-bit payload store, one scale byte.
 // HBM-bound: 2 B read + 0.5625 B written per element.
 #include <math.h>
 
@@ -20,66 +20,40 @@ DEV size_t sf_tiled_offset(int64_t row, int64_t blk, int64_t chunks_per_row) {
          (size_t)(blk & 3);
 }
 
-// A block of threads = rows_per_block rows x threads_per_row 16-element blocks (one integer division per thread); every
-// thread has the loads of kRowsInFlight rows out before it computes. It was bound by the issue rate (223 instructions per 16
-// elements at 71 % of the issue slots, 8192 x 7168 in 33 us): hence packed arithmetic, packed maxima, the table instead of a
-// reciprocal per block, corrected multiplications instead of two divisions, and one scale store per four threads.
-constexpr int kRowsInFlight = 2;
-
+// A block of threads = rows_per_block rows x threads_per_row 16-element blocks (one integer division per thread). Bound by HBM
+// and, next to it, by issue; what hides both is many warps that are each at another point, so a thread holds one block at a
+// time in at most 32 registers (64 warps per SM) and a launch is a few waves of blocks: 8192 x 7168 25.0 us with row-major scales
+// (6.0 TB/s), 26.1 tiled. One wave of 28 warps per SM with the loads of two rows each in flight and a table of reciprocals in shared
+// memory took 31.0 and 32.5, and a batch of 64 x 7168, which waits for the table, 2.5 against 2.0. Joining four scale bytes by
+// shuffles into one store costs more than the stores (27.0).
 template <bool EXACT_DIV, bool WIDE>      // WIDE: rows start on 32-byte boundaries, one 256-bit load per block
-__global__ void __launch_bounds__(256, 4) k_quantize_nvfp4(const __nv_bfloat16* __restrict__ x, int64_t rows, int blocks_per_row,
+__global__ void __launch_bounds__(256, EXACT_DIV ? 1 : 8) k_quantize_nvfp4(const __nv_bfloat16* __restrict__ x, int64_t rows, int blocks_per_row,
                                                         int64_t row_stride, float gs, uint8_t* __restrict__ payload,
                                                         uint8_t* __restrict__ scales, int sf_layout, int threads_per_row,
-                                                        int rows_per_block, int word_scales) {
-  __shared__ ScaleRow table[128];
+                                                        int rows_per_block) {
   pdl_trigger();
-  if (!EXACT_DIV) {
-    fill_scale_table(table, gs);
-    __syncthreads();
-  }
   const float rgs = __frcp_rn(gs);
-  const int r = (int)threadIdx.x / threads_per_row;
+  const int r = rows_per_block == 1 ? ((int)threadIdx.x >= threads_per_row) : (int)threadIdx.x / threads_per_row;
   const int blk0 = (int)threadIdx.x - r * threads_per_row;
-  const uint32_t quad = 0xFu << (threadIdx.x & 28);               // four neighbouring 16-element blocks of one row
   if (r >= rows_per_block) return;
-  const int64_t step = (int64_t)gridDim.x * rows_per_block;
   pdl_wait();
-  for (int64_t row0 = (int64_t)blockIdx.x * rows_per_block + r; row0 < rows; row0 += step * kRowsInFlight)
+  for (int64_t row = (int64_t)blockIdx.x * rows_per_block + r; row < rows; row += (int64_t)gridDim.x * rows_per_block)
     for (int blk = blk0; blk < blocks_per_row; blk += threads_per_row) {
-      uint32_t w[kRowsInFlight][8];
-#pragma unroll
-      for (int i = 0; i < kRowsInFlight; ++i) {
-        const int64_t row = row0 + i * step;
-        if (row >= rows) break;
-        const __nv_bfloat16* src = x + row * row_stride + blk * 16;
-        if (WIDE) {
-          asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                       : "=r"(w[i][0]), "=r"(w[i][1]), "=r"(w[i][2]), "=r"(w[i][3]), "=r"(w[i][4]), "=r"(w[i][5]), "=r"(w[i][6]),
-                         "=r"(w[i][7])
-                       : "l"(src));
-        } else {
-          const uint4 lo = __ldg(reinterpret_cast<const uint4*>(src)), hi = __ldg(reinterpret_cast<const uint4*>(src) + 1);
-          w[i][0] = lo.x; w[i][1] = lo.y; w[i][2] = lo.z; w[i][3] = lo.w;
-          w[i][4] = hi.x; w[i][5] = hi.y; w[i][6] = hi.z; w[i][7] = hi.w;
-        }
+      const __nv_bfloat16* src = x + row * row_stride + blk * 16;
+      uint32_t w[8];
+      if (WIDE) {
+        asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+                     : "l"(src));
+      } else {
+        const uint4 lo = __ldg(reinterpret_cast<const uint4*>(src)), hi = __ldg(reinterpret_cast<const uint4*>(src) + 1);
+        w[0] = lo.x; w[1] = lo.y; w[2] = lo.z; w[3] = lo.w;
+        w[4] = hi.x; w[5] = hi.y; w[6] = hi.z; w[7] = hi.w;
       }
-#pragma unroll
-      for (int i = 0; i < kRowsInFlight; ++i) {
-        const int64_t row = row0 + i * step;
-        if (row >= rows) break;
-        uint32_t packed[2];
-        const uint32_t sbyte = quantize_block<EXACT_DIV>(w[i], gs, rgs, table, packed);
-        *reinterpret_cast<uint2*>(payload + row * ((int64_t)blocks_per_row * 8) + (int64_t)blk * 8) = make_uint2(packed[0], packed[1]);
-        const size_t at = sf_layout == 0 ? (size_t)(row * blocks_per_row + blk) : sf_tiled_offset(row, blk, blocks_per_row >> 2);
-        if (word_scales) {
-          uint32_t word = sbyte << (8 * (blk & 3));
-          word |= __shfl_xor_sync(quad, word, 1);
-          word |= __shfl_xor_sync(quad, word, 2);
-          if ((blk & 3) == 0) *reinterpret_cast<uint32_t*>(scales + at) = word;
-        } else {
-          scales[at] = (uint8_t)sbyte;
-        }
-      }
+      uint32_t packed[2];
+      const uint32_t sbyte = quantize_block<EXACT_DIV>(w, gs, rgs, packed);
+      *reinterpret_cast<uint2*>(payload + row * ((int64_t)blocks_per_row * 8) + (int64_t)blk * 8) = make_uint2(packed[0], packed[1]);
+      scales[sf_layout == 0 ? (size_t)(row * blocks_per_row + blk) : sf_tiled_offset(row, blk, blocks_per_row >> 2)] = (uint8_t)sbyte;
     }
 }
 
@@ -100,20 +74,21 @@ __global__ void k_sf_to_tiles(const uint8_t* __restrict__ src, int64_t rows, int
 int launch_quantize_nvfp4(const void* x, int64_t rows, int64_t cols, int64_t row_stride, float gs, void* payload, void* scales,
                           int sf_layout, cudaStream_t st) {
   if (rows == 0) return 0;
-  const int bpr = (int)(cols >> 4);                       // a multiple of 4
-  // threads of a row: its 16-element blocks in equal passes of at most 256, a multiple of 4; short rows share a block
+  const int bpr = (int)(cols >> 4);
+  // threads of a row: its 16-element blocks in equal passes of at most 256; short rows share a block (16384 x 512: 6.0 us, 8.4 with
+  // a block per row)
   const int passes = (bpr + 255) / 256;
-  const int tpr = ((bpr + passes - 1) / passes + 3) / 4 * 4;
-  const int rpb = 256 / tpr;
+  const int tpr = (bpr + passes - 1) / passes;
+  const int64_t spread = rows / sm_count();                              // a short batch: first a block for every SM
+  const int rpb = (int)(spread < 1 ? 1 : spread < 256 / tpr ? spread : 256 / tpr);
   const int threads = (rpb * tpr + 31) / 32 * 32;
-  const int64_t resident = (int64_t)sm_count() * (1024 / threads);       // one wave at 64 registers a thread
+  const int64_t most = (int64_t)sm_count() * 32;
   const int64_t want = (rows + rpb - 1) / rpb;
-  const int64_t blocks = want < resident ? want : resident;
+  const int64_t blocks = want < most ? want : most;
   const bool wide = ((uintptr_t)x & 31) == 0 && row_stride % 16 == 0;
-  const int word_scales = ((uintptr_t)scales & 3) == 0;
   auto go = [&](auto kern) {
     return (int)launch_chain(kern, dim3((unsigned)blocks), dim3(threads), 0, st, (const __nv_bfloat16*)x, rows, bpr, row_stride, gs,
-                             (uint8_t*)payload, (uint8_t*)scales, sf_layout, tpr, rpb, word_scales);
+                             (uint8_t*)payload, (uint8_t*)scales, sf_layout, tpr, rpb);
   };
   if (!quantize_fast(gs)) return go(k_quantize_nvfp4<true, false>);
   return wide ? go(k_quantize_nvfp4<false, true>) : go(k_quantize_nvfp4<false, false>);

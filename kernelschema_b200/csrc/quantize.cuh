@@ -6,23 +6,6 @@
 
 namespace b200 {
 
-// Packed fp32 arithmetic: two IEEE operations per instruction and lane.
-DEV uint64_t pack_f32x2(uint32_t lo, uint32_t hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
-  return r;
-}
-DEV uint64_t mul_f32x2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-DEV uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-
 // RN(a / b) from r = RN(1 / b): Markstein's residual correction, twice. The first step brings the quotient within an ulp, the
 // second (whose residual is then exact in one fma) rounds it correctly.
 DEV float div_rn(float a, float b, float r) {
@@ -30,12 +13,6 @@ DEV float div_rn(float a, float b, float r) {
   q = __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
   return __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
 }
-
-// What a block of 16 divides by, for every E4M3 scale byte: d = RN(stored * gs) (the reference divides by that) and
-// -RN(1 / d). 128 entries in shared memory, filled once per thread block.
-struct ScaleRow {
-  float d, neg_r;
-};
 
 // One block of 16 bf16 values (eight words) -> its E4M3 scale byte and 16 E2M1 codes.
 //
@@ -48,7 +25,7 @@ struct ScaleRow {
 // q1 = (-rem) * (-r) + q0 round alike, and both zeros come out with the sign of x (they encode as 0 and 8).
 // EXACT_DIV selects IEEE division instead (global scales so small or large that the residual could leave the normal range).
 template <bool EXACT_DIV>
-DEV uint32_t quantize_block(const uint32_t (&w)[8], float gs, float rgs, const ScaleRow* __restrict__ table, uint32_t (&packed)[2]) {
+DEV uint32_t quantize_block(const uint32_t (&w)[8], float gs, float rgs, uint32_t (&packed)[2]) {
   __nv_bfloat162 m = __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[0]));      // the largest magnitude, exact in bf16
 #pragma unroll
   for (int i = 1; i < 8; ++i) m = __hmax2(m, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[i])));
@@ -59,54 +36,35 @@ DEV uint32_t quantize_block(const uint32_t (&w)[8], float gs, float rgs, const S
     scale = __fdiv_rn(peak, 6.0f);
     if (gs != 1.0f) scale = __fdiv_rn(scale, gs);
   } else {
-    // operands beyond 6144 * gs and 1024 * gs only ever give a scale that the clamp below turns into 448
+    // a peak beyond 6144 * gs only ever gives a scale that the clamp below turns into 448
     scale = div_rn(fminf(peak, 6144.0f * gs), 6.0f, 1.0f / 6.0f);
     scale = div_rn(scale, gs, rgs);
   }
   scale = fminf(fmaxf(scale, 0.001953125f), 448.0f);               // clamp(2^-9, 448)
   const uint32_t sbyte = cvt_e4m3(scale);
-  if (EXACT_DIV) {
-    const float d = __fmul_rn(e4m3_to_f32(sbyte), gs);
+  const float d = __fmul_rn(e4m3_to_f32(sbyte), gs);               // the reference divides by stored * gs
+  const float nr = EXACT_DIV ? 0.f : -__frcp_rn(d);
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      float q[8];
+  for (int h = 0; h < 2; ++h) {
+    float q[8];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const uint32_t u = w[4 * h + i];
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t u = w[4 * h + i];
+      if (EXACT_DIV) {
         q[2 * i] = __fdiv_rn(__uint_as_float(u << 16), d);
         q[2 * i + 1] = __fdiv_rn(__uint_as_float(u & 0xFFFF0000u), d);
+      } else {
+        const float2 nx = make_float2(__uint_as_float(u * 65536u + 0x80000000u), __uint_as_float((u & 0xFFFF0000u) ^ 0x80000000u));
+        const float2 nr2 = make_float2(nr, nr), q0 = mul2(nx, nr2), q1 = fma2(fma2(q0, make_float2(d, d), nx), nr2, q0);
+        q[2 * i] = q1.x;
+        q[2 * i + 1] = q1.y;
       }
-      packed[h] = cvt_e2m1x8(q);
     }
-  } else {
-    const ScaleRow row = table[sbyte];
-    const uint32_t nr = __float_as_uint(row.neg_r), db = __float_as_uint(row.d);
-    const uint64_t nr2 = pack_f32x2(nr, nr), d2 = pack_f32x2(db, db);
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      float q[8];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const uint32_t u = w[4 * h + i];
-        const uint64_t nx = pack_f32x2(u * 65536u + 0x80000000u, (u & 0xFFFF0000u) ^ 0x80000000u);
-        const uint64_t q0 = mul_f32x2(nx, nr2);
-        const uint64_t q1 = fma_f32x2(fma_f32x2(q0, d2, nx), nr2, q0);
-        q[2 * i] = __uint_as_float((uint32_t)q1);
-        q[2 * i + 1] = __uint_as_float((uint32_t)(q1 >> 32));
-      }
-      packed[h] = cvt_e2m1x8(q);
-    }
+    packed[h] = cvt_e2m1x8(q);
   }
   return sbyte;
 }
 
-// Fills the table with the threads of one block (a block barrier has to follow).
-DEV void fill_scale_table(ScaleRow* table, float gs) {
-  for (int i = threadIdx.x; i < 128; i += blockDim.x) {
-    const float d = __fmul_rn(e4m3_to_f32((uint32_t)i), gs);
-    table[i] = {d, -__frcp_rn(d)};
-  }
-}
 // stored * gs stays a normal number with room for the residual of a bf16 numerator inside 2^-40 .. 2^40
 inline bool quantize_fast(float gs) { return gs >= 0x1p-40f && gs <= 0x1p40f; }
 

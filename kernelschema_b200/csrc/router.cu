@@ -143,7 +143,6 @@ __global__ void __launch_bounds__(256) k_router_logits_small(const __nv_bfloat16
 __global__ void __launch_bounds__(256) k_front_small(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, int T, int H,
                                                      int E, float* __restrict__ logits, float gs, uint8_t* __restrict__ payload,
                                                      uint8_t* __restrict__ scales) {
-  __shared__ ScaleRow table[128];
   pdl_trigger();
   const int router_blocks = (E + 1) / 2;
   if ((int)blockIdx.x < router_blocks) {
@@ -151,8 +150,6 @@ __global__ void __launch_bounds__(256) k_front_small(const __nv_bfloat16* __rest
     logits_small<8>(x, w, T, H, E, logits);
     return;
   }
-  fill_scale_table(table, gs);
-  __syncthreads();
   pdl_wait();
   const int64_t row = (int)blockIdx.x - router_blocks;
   const float rgs = __frcp_rn(gs);
@@ -162,7 +159,7 @@ __global__ void __launch_bounds__(256) k_front_small(const __nv_bfloat16* __rest
     const uint4 lo = __ldg(src), hi = __ldg(src + 1);
     const uint32_t v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
     uint32_t packed[2];
-    scales[row * blocks_per_row + blk] = (uint8_t)quantize_block<false>(v, gs, rgs, table, packed);
+    scales[row * blocks_per_row + blk] = (uint8_t)quantize_block<false>(v, gs, rgs, packed);
     *reinterpret_cast<uint2*>(payload + row * (H >> 1) + (int64_t)blk * 8) = make_uint2(packed[0], packed[1]);
   }
 }

@@ -51,8 +51,8 @@ def test_quantize_matches_oracle(rows, cols, scale):
 @pytest.mark.parametrize("rows,cols,pad,offset", [(1, 64, 0, 0), (9999, 64, 0, 0), (300, 192, 8, 1), (9500, 320, 0, 0), (130, 4160, 8, 0),
                                                   (4800, 4096, 16, 3)])
 def test_quantize_short_rows_odd_strides_and_scale_alignment(rows, cols, pad, offset):
-    """Several rows per block, two rows per thread in flight, rows that start on 16- but not 32-byte boundaries, and scale
-    buffers on odd addresses, in both layouts."""
+    """One row and several rows per block, rows that start on 16- but not 32-byte boundaries, and scale buffers on odd
+    addresses, in both layouts."""
     import kernelschema_b200 as ks
     x = torch.randn(rows, cols + pad, generator=torch.Generator().manual_seed(rows)).to(torch.bfloat16)
     oq, os_ = o.quantize(x[:, :cols].float().numpy(), 16, 0.0021)
