@@ -209,10 +209,15 @@ k_gemm_w4a16(const __grid_constant__ CUtensorMap tm_a, const W4A16Params p) {
   // items: the whole tiles, then (tail tile, split) with the split fastest; tile = (mt, nt), n fastest: the CTAs of a wave share
   // A's rows and sweep the weights (L2-resident). A split covers k-groups [g0, g1).
   const int total_items = p.full_tiles + p.tail_tiles * p.splits;
-  auto item_tile = [&](int item) { return item < p.full_tiles ? item : p.full_tiles + (item - p.full_tiles) / p.splits; };
-  auto item_split = [&](int item) { return item < p.full_tiles ? -1 : (item - p.full_tiles) % p.splits; };
-  auto item_g0 = [&](int item) { return max(item_split(item), 0) * p.groups_per_split; };
-  auto item_g1 = [&](int item) { return item < p.full_tiles ? groups : min(groups, (item_split(item) + 1) * p.groups_per_split); };
+  struct Item {
+    int tile, split, g0, g1;                // split -1: the whole of K
+  };
+  auto item_at = [&](int item) -> Item {    // once per item and role: the divisions cost a few hundred cycles
+    const int t = item - p.full_tiles;
+    if (t < 0) return {item, -1, 0, groups};
+    const int q = t / p.splits, s = t - q * p.splits;
+    return {p.full_tiles + q, s, s * p.groups_per_split, min(groups, (s + 1) * p.groups_per_split)};
+  };
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer of A
@@ -220,8 +225,9 @@ k_gemm_w4a16(const __grid_constant__ CUtensorMap tm_a, const W4A16Params p) {
       uint32_t s = 0, ph = 1;
       bool ok = true;
       for (int item = blockIdx.x; ok && item < total_items; item += gridDim.x) {
-        const int mt = item_tile(item) / n_nt;
-        for (int ks = 4 * item_g0(item); ks < 4 * item_g1(item); ++ks) {
+        const Item at = item_at(item);
+        const int mt = at.tile / n_nt, ks1 = 4 * at.g1;
+        for (int ks = 4 * at.g0; ks < ks1; ++ks) {
           if (!mbar_wait(bar_empty + 8 * s, ph)) { if (p.status) atomicCAS(p.status, 0, 121); ok = false; break; }
           mbar_expect_tx(bar_full_a + 8 * s, C::kABytes);
           tma_load_2d(s_a + s * C::kABytes, &tm_a, bar_full_a + 8 * s, ks * 128, mt * 256);
@@ -237,9 +243,9 @@ k_gemm_w4a16(const __grid_constant__ CUtensorMap tm_a, const W4A16Params p) {
       uint32_t s = 0, ph = 0, it = 0;
       bool ok = true;
       for (int item = blockIdx.x; ok && item < total_items; item += gridDim.x, ++it) {
-        const int mt = item_tile(item) / n_nt;
-        const bool second = p.M - mt * 256 > 128;          // rows 128..255 of the tile hold real rows
-        const int nk = 4 * (item_g1(item) - item_g0(item));
+        const Item at = item_at(item);
+        const bool second = p.M - at.tile / n_nt * 256 > 128;          // rows 128..255 of the tile hold real rows
+        const int nk = 4 * (at.g1 - at.g0);
         const uint32_t buf = it % C::kAccBufs;
         if (!mbar_wait(bar_acc_empty + 8 * buf, ((it / C::kAccBufs) & 1) ^ 1)) { if (p.status) atomicCAS(p.status, 0, 122); break; }
         tc_fence_after();
@@ -275,8 +281,8 @@ k_gemm_w4a16(const __grid_constant__ CUtensorMap tm_a, const W4A16Params p) {
     const uint32_t patch = s_patch + (uint32_t)(warp - 2) * C::kPatchBytes;
     // one k-group of the warp's rows: through the patch lane -> row 4i + lane / 8, 16-byte piece lane % 8, else each lane its own
     // row; and the scales of the lane's own row
-    auto fetch = [&](int item, int g) {
-      const size_t row0 = (size_t)(item_tile(item) % n_nt) * BN + (r & ~31);
+    auto fetch = [&](const Item& at, int g) {
+      const size_t row0 = (size_t)(at.tile % n_nt) * BN + (r & ~31);
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int row = C::kPatch ? 4 * i + (lane >> 3) : lane, piece = C::kPatch ? lane & 7 : i;
@@ -284,10 +290,13 @@ k_gemm_w4a16(const __grid_constant__ CUtensorMap tm_a, const W4A16Params p) {
       }
       nxt_sf = __ldg(reinterpret_cast<const uint4*>(p.b_sf + (row0 + lane) * (size_t)(p.K >> 4)) + g);
     };
-    if ((int)blockIdx.x < total_items) fetch(blockIdx.x, item_g0(blockIdx.x));
+    Item at = item_at(blockIdx.x);
+    if ((int)blockIdx.x < total_items) fetch(at, at.g0);
     for (int item = blockIdx.x; ok && item < total_items; item += gridDim.x) {
-      const int g1 = item_g1(item);
-      for (int g = item_g0(item); ok && g < g1; ++g) {
+      const Item cur_item = at;
+      const int g1 = at.g1;
+      if (item + (int)gridDim.x < total_items) at = item_at(item + gridDim.x);      // the next item
+      for (int g = cur_item.g0; ok && g < g1; ++g) {
         uint32_t line[C::kPatch ? 1 : 32];
         if constexpr (!C::kPatch) {
 #pragma unroll
@@ -306,8 +315,8 @@ k_gemm_w4a16(const __grid_constant__ CUtensorMap tm_a, const W4A16Params p) {
         if (C::kPatch) __syncwarp();
         const uint32_t cur_sf[4] = {nxt_sf.x, nxt_sf.y, nxt_sf.z, nxt_sf.w};
         // next lines: the following k-group of this item, or the first of this CTA's next item
-        if (g + 1 < g1) fetch(item, g + 1);
-        else if (item + (int)gridDim.x < total_items) fetch(item + gridDim.x, item_g0(item + gridDim.x));
+        if (g + 1 < g1) fetch(cur_item, g + 1);
+        else if (item + (int)gridDim.x < total_items) fetch(at, at.g0);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {                       // the four 64-wide k-steps of the group
           uint32_t cur[8];
@@ -342,8 +351,8 @@ k_gemm_w4a16(const __grid_constant__ CUtensorMap tm_a, const W4A16Params p) {
     const float alpha = p.alpha ? *p.alpha : 1.0f;
     uint32_t it = 0;
     for (int item = blockIdx.x; item < total_items; item += gridDim.x, ++it) {
-      const int tile = item_tile(item);
-      const int mt = tile / n_nt, nt = tile % n_nt;
+      const Item at = item_at(item);
+      const int mt = at.tile / n_nt, nt = at.tile - mt * n_nt;
       const uint32_t buf = it % C::kAccBufs;
       int okw = 1;
       if (lane == 0) okw = mbar_wait(bar_acc_full + 8 * buf, (it / C::kAccBufs) & 1) ? 1 : 0;
@@ -353,9 +362,7 @@ k_gemm_w4a16(const __grid_constant__ CUtensorMap tm_a, const W4A16Params p) {
       const int row = mt * 256 + half * 128 + quad * 32 + lane;
       const bool live = row < p.M;
       const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + buf * 2 * BN + half * BN;
-      const int split = item_split(item);
-      float* partial_row = split < 0 || p.splits == 1 ? nullptr
-                                                      : p.partial + (((size_t)split * p.tail_tiles + (tile - p.full_tiles)) * p.M + row) * BN;
+      float* partial_row = at.split < 0 ? nullptr : p.partial + (((size_t)at.split * p.tail_tiles + (at.tile - p.full_tiles)) * p.M + row) * BN;
       store_cols<BN>(p, taddr, row, live, nt * BN, alpha, partial_row, [&]() {
         tc_fence_before();
         __syncwarp();
