@@ -407,8 +407,8 @@ __global__ void __launch_bounds__(256) k_w4a16_reduce(const W4A16Params p, int b
 // the SMs hold (at most eight, at least one k-group each). Behind whole waves that pays for its partial tiles and the second launch
 // only when a tile is long: from 16 k-groups on. The plan of a batch of 33 to 128 rows does not depend on its rows, so a row has
 // one value in all of them. Above, which tiles end up in the last wave depends on the batch: a split there would give a row other
-// last bits at another position, so there is none (that gives up time: 8192 x 4096 x 12288 710 us with a split, 769 without;
-// 300 x 4096 x 4096 39 and 62). `room`: the caller has a workspace for the partial tiles.
+// last bits at another position, so there is none (that gives up time: 8192 x 4096 x 12288 696 us with a split, 759 without;
+// 129 x 4096 x 4096 23 and 42, 1000 x 4096 x 4096 56 and 45). `room`: the caller has a workspace for the partial tiles.
 struct W4A16Plan {
   int bn, full_tiles, tail_tiles, splits;
 };
@@ -417,8 +417,12 @@ static W4A16Plan w4a16_plan(int64_t m, int64_t n, int64_t k, int sms, bool room)
   // Up to 128 rows half of a wide tile's accumulators idle: it pays when the tiles are long and fill the device, by their number
   // (M = 64, N = 25600, K = 8192: 120 us against 158) or by a split that there is room for (M = 64, N = 4096, K = 12288: 31 us against
   // 36; N = 2048, K = 4096: 16 against 12). A split that falls away leaves half as many CTAs as narrow tiles do (M = 64, N = 4096,
-  // K = 8192: 116 us against 81; M = 128, N = 8192, K = 12288: 179 against 120).
-  pl.bn = n % 256 == 0 && (m > 128 || (room && n >= 4096 && k >= 8192)) ? 256 : 128;
+  // K = 8192: 116 us against 81; M = 128, N = 8192, K = 12288: 179 against 120). Above 128 rows narrow tiles are the better ones while
+  // all of them run at once: half the work of a wide tile each, and no trip through the patch that a single tile per SM cannot hide
+  // (129 x 4096 x 4096 63 us wide, 42 narrow; 1000 x 4096 x 4096, the last of that width, 61 and 45; 1200 rows 63 wide). Both widths
+  // add in the same order.
+  const int64_t wide_tiles = (m + 255) / 256 * (n / 256);
+  pl.bn = n % 256 == 0 && (m > 128 ? wide_tiles * 2 > sms : room && n >= 4096 && k >= 8192) ? 256 : 128;
   const int64_t tiles = (m + 255) / 256 * (n / pl.bn), groups = k / 256, tail = tiles % sms;
   int64_t s = tail ? sms / tail : 1;
   if (s > 8) s = 8;

@@ -258,11 +258,11 @@ def test_w4a16_split_on_two_streams_and_in_a_graph():
     assert torch.equal(out, want[0])
 
 
-@pytest.mark.parametrize("n,k,sizes", [(4096, 4096, (129, 300, 1111, 2600)), (3328, 4352, (200, 3000)), (1152, 8192, (150, 1300)),
+@pytest.mark.parametrize("n,k,sizes", [(4096, 4096, (129, 300, 1024, 1025, 1280, 1281, 2600)), (3328, 4352, (200, 3000)), (1152, 8192, (150, 1300)),
                                        (4096, 8192, (33, 64, 65, 128)), (20480, 4096, (40, 128)), (4096, 12288, (1, 8, 9, 16)), (2048, 7168, (17, 24, 32))])
 def test_w4a16_a_row_has_one_value(n, k, sizes):
     """A row gives the same bits at any position and in any batch of 1..16, 17..32, 33..128 and more than 128 rows: long K, fewer
-    tiles than SMs as well as a partly filled last wave behind whole ones. With split_k=False the bits are those of more than 128
+    tiles than SMs (128-wide up to 1024 rows x 4096, 256-wide above) as well as a partly filled last wave behind whole ones. With split_k=False the bits are those of more than 128
     rows at every size."""
     import kernelschema_b200 as ks
     gen = torch.Generator(device="cuda").manual_seed(n + k)
