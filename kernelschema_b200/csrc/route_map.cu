@@ -7,7 +7,7 @@
 // inside its expert segment is its rank in ascending flat index t*K+k (the reference leaves that
 // order arbitrary), so every integer output is reproducible and can be compared bit for bit.
 // No global atomics. One launch for small builds (with the permute, where that applies), histograms + scan-and-scatter for
-// larger ones, a scan launch of its own beyond kHistMaxBlocks chunks.
+// larger ones, a scan launch of its own for many chunks or very many experts (two_launch_build).
 #include "kernels.cuh"
 #include "ptx.cuh"
 #include "topk.cuh"
@@ -293,10 +293,15 @@ __global__ void __launch_bounds__(kRouteThreads) k_route_scatter(RouteView r, co
 // and instead of exchanging histograms with the other blocks it reads ALL expert ids itself (a few tens of KB): that
 // gives it every expert's total (segment starts, tile list) and the count in the chunks before its own (its base inside
 // the segment). Up to kHistMaxBlocks chunks a first launch counts them and the blocks read the counts instead of the ids (a
-// separate one-block scan took 10 us of the three-launch build at 131 072 routes). The counts of foreign chunks are accumulated with shared-memory atomics; a count does not depend on the
-// order of the additions, so every output stays reproducible. Block 0 also writes the per-expert tables.
+// separate one-block scan took 10 us of the three-launch build at 131 072 routes). The counts of foreign chunks are accumulated
+// with shared-memory atomics; a count does not depend on the order of the additions, so every output stays reproducible. Block 0 also writes the per-expert tables.
 constexpr int kFusedMaxBlocks = 8;
-constexpr int kHistMaxBlocks = 128;              // beyond, every block reading every count costs more than the scan launch
+// Chunks up to which the blocks read the counts themselves; beyond, every block reading every count costs more than the scan
+// launch. That cost grows with the experts: with up to 640 two launches win from the first such size on (2100 x 8 routes
+// 17.3 us against 17.5, 32768 x 8 26.6 against 34.2), with up to 896 from 16 chunks on (2100 x 8 19.3 against 18.7, 4096 x 8 even,
+// 16384 x 8 23.2 against 30.9), with 1000 nowhere (2100 x 8 21.2 against 18.9, 16384 x 8 25.7 against 24.6, 32768 x 8 34.6 against 32.2).
+constexpr int kHistMaxBlocks = 128;
+static bool two_launch_build(int nblk, int etot) { return nblk <= kHistMaxBlocks && etot <= (nblk < 16 ? 640 : 896); }
 constexpr int kGatherMaxRoutes = 16384;          // the fused form that also permutes the rows
 constexpr int kGatherMaxChunk = 256;             // routes a block of it may own (8 warps); 32 where it selects the experts itself
 
@@ -598,7 +603,7 @@ int launch_route_map(const int32_t* ids, const float* scores, int64_t id_stride,
   const size_t smem = sizeof(int) * kRouteWarps * (size_t)etot;
   cudaError_t err = cudaSuccess;
   if (nblk > 0) err = launch_chain(k_route_hist, dim3(nblk), dim3(kRouteThreads), smem, st, r, etot, b.block_hist);
-  if (err == cudaSuccess && nblk > 0 && nblk <= kHistMaxBlocks)
+  if (err == cudaSuccess && nblk > 0 && two_launch_build(nblk, etot))
     return (int)launch_chain(k_route_fused, dim3(nblk), dim3(kRouteThreads), sizeof(int) * (kRouteWarps + 2) * (size_t)etot, st, r, scores,
                              etot, b, (const int32_t*)b.block_hist);
   if (err == cudaSuccess)

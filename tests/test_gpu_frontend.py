@@ -196,12 +196,13 @@ def test_router_logits(t, h, e):
 @pytest.mark.parametrize("t,k,e,shared,offset", [(1, 8, 128, 0, 0), (300, 4, 8, 0, 0), (4096, 8, 256, 1, 0),
                                                  (1000, 8, 32, 0, 64), (50, 2, 4, 2, 0), (2049, 1, 3, 0, 0), (600, 8, 512, 0, 0), (1500, 8, 128, 1, 0),
                                                  (300, 8, 1000, 1, 0), (5000, 8, 1000, 0, 0),
-                                                 (32768, 8, 128, 0, 0), (29127, 8, 8, 1, 0), (52429, 5, 40, 0, 0), (32769, 8, 1000, 0, 64),
+                                                 (32768, 8, 128, 0, 0), (4096, 8, 895, 1, 0), (4096, 8, 896, 1, 0), (3840, 8, 640, 0, 0),
+                                                 (3840, 8, 641, 0, 0), (29127, 8, 8, 1, 0), (52429, 5, 40, 0, 0), (32769, 8, 1000, 0, 64),
                                                  (60000, 8, 7, 1, 0)])
 def test_route_map_matches_oracle(t, k, e, shared, offset):
-    """One launch up to 16384 routes, histograms + scan-and-scatter up to 262144 (32768 x 8 and 29127 x 9 are the last sizes),
-    histograms, scan and scatter beyond (52429 x 5 is the first): 40 experts over 129 blocks and 8 over 264 scan with a warp per
-    expert, 1000 with a thread per expert."""
+    """One launch up to 16384 routes, histograms + scan-and-scatter up to 262144 (32768 x 8 and 29127 x 9 are the last sizes) and 896
+    experts (640 below 16 chunks of 2048 routes), histograms, scan and scatter beyond (52429 x 5 is the first): 40 experts over
+    129 blocks and 8 over 264 scan with a warp per expert, 1000 with a thread per expert."""
     import kernelschema_b200 as ks
     rng = np.random.default_rng(t * 7 + e)
     span = e * 4 if offset else e
