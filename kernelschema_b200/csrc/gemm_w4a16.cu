@@ -8,18 +8,17 @@
 // reference only by the order of the fp32 additions.
 //
 // Tile: 256 rows of A (two 128-row accumulators) x BN weight rows, K in steps of 64; one decoded weight tile feeds two
-// MMAs. The kernel is bound by shared-memory bandwidth (per k-step the tile's A and decoded B are written once and read
-// by the MMAs), so the wide form BN = 256 is taken when N allows it: 160 KB of shared-memory traffic per
-// 256 x 256 x 64 step against 112 KB per 256 x 128 x 64 step. Its two 256-column accumulators fill the 512 TMEM columns,
-// so the epilogue of a tile (a few microseconds) is not overlapped; BN = 128 (N % 256 != 0) alternates between two
-// accumulator pairs.
+// MMAs. Weight loads, decoding, operand traffic and MMAs share an SM's time and none alone is the bound (8192 x 4096 x 12288,
+// 734 us, with one part left out: no weight loads 554, no MMAs 596, no decoding 614). The wide form BN = 256 is taken where N and
+// the number of tiles allow it (w4a16_plan) because it moves less for the same work: 160 KB of shared-memory traffic per
+// 256 x 256 x 64 step against 112 KB per 256 x 128 x 64 step. Its two 256-column accumulators fill the 512 TMEM columns, so the
+// epilogue of a tile (a few microseconds) is not overlapped; BN = 128 alternates between two accumulator pairs.
 // Warp roles: 0 = TMA producer of A (bf16, 128-byte swizzle); 1 = TMEM owner + MMA issuer; then BN/32 decoder warps, one
-// thread per weight row of the tile. In the wide form a warp loads its 32 rows' lines (128 bytes = 256 weights each) one k-group ahead, four
-// rows per instruction, and turns them to a row per lane in a shared-memory patch of its own: loaded row by row, an
-// instruction touches 32 lines, and those passes through the L1 pipe compete with the operand traffic (8192 x 4096 x 12288:
-// 734 us, 554 with no weight loads at all). A thread expands its row with byte permutes and one bf16 multiply per pair, and
-// writes bf16 into shared memory
-// in the layout a 128-byte-swizzled TMA load would have produced (16-byte chunk c of row r at
+// thread per weight row of the tile. In the wide form a warp loads its 32 rows' lines (128 bytes = 256 weights each) one k-group
+// ahead, four rows per instruction, and turns them to a row per lane in a shared-memory patch of its own: loaded row by row, an
+// instruction touches 32 lines, and those passes through the L1 pipe compete with the operand traffic (8192 x 4096 x 12288
+// 796 us, 759 through the patch). A thread expands its row with byte permutes and one bf16 multiply per pair, and writes bf16 into
+// shared memory in the layout a 128-byte-swizzled TMA load would have produced (16-byte chunk c of row r at
 // r * 128 + ((c ^ (r & 7)) * 16)), then fence.proxy.async + mbarrier arrive; the last 8 warps = epilogue.
 // Every wait is bounded and reports through the status word.
 //
@@ -407,8 +406,8 @@ __global__ void __launch_bounds__(256) k_w4a16_reduce(const W4A16Params p, int b
 // the SMs hold (at most eight, at least one k-group each). Behind whole waves that pays for its partial tiles and the second launch
 // only when a tile is long: from 16 k-groups on. The plan of a batch of 33 to 128 rows does not depend on its rows, so a row has
 // one value in all of them. Above, which tiles end up in the last wave depends on the batch: a split there would give a row other
-// last bits at another position, so there is none (that gives up time: 8192 x 4096 x 12288 696 us with a split, 759 without;
-// 129 x 4096 x 4096 23 and 42, 1000 x 4096 x 4096 56 and 45). `room`: the caller has a workspace for the partial tiles.
+// last bits at another position, so there is none, which gives up time (8192 x 4096 x 12288 696 us with a split, 759 without;
+// 129 x 4096 x 4096 23 and 42). `room`: the caller has a workspace for the partial tiles.
 struct W4A16Plan {
   int bn, full_tiles, tail_tiles, splits;
 };
