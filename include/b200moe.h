@@ -152,10 +152,10 @@ int b200moe_gemm_nvfp4(const void* a_q, const void* a_sf_tiled, const void* b_q,
  * workspace (optional, 16-byte aligned device memory of at least b200moe_gemm_bf16_nvfp4_workspace_bytes(m, n, k) bytes;
  * that function returns 0 when none is useful): for M <= 128 it lets several CTAs share the reduction of an output tile of
  * the last, partly filled wave (fp32 partial sums added in a fixed order: results stay reproducible). Without it every tile
- * is reduced by one CTA, which leaves most of the device idle when there are few tiles. Up to 32 rows need none.
- * A row's result depends on the row, B, alpha and K alone among batches of 1..16, 17..32, 33..128 and more than 128 rows;
- * between these ranges the order of the additions differs. workspace_bytes < 0 asks for the same result at every M: each
- * element is one sum in ascending k (slow at small M). */
+ * is reduced by one CTA, which leaves most of the device idle when there are few tiles. Up to 16 rows need none.
+ * A row's result depends on the row, B, alpha and on whether there is a workspace, not on M, among batches of 1..16,
+ * 17..32, 33..128 and more than 128 rows; between these ranges the order of the additions differs. workspace_bytes < 0 asks
+ * for the same result at every M: each element is one sum in ascending k (slow at small M). */
 int64_t b200moe_gemm_bf16_nvfp4_workspace_bytes(int64_t m, int64_t n, int64_t k);
 int b200moe_gemm_bf16_nvfp4(const void* a, int64_t a_stride, const void* b_q, const void* b_descale, const float* alpha, void* out,
                             int64_t m, int64_t n, int64_t k, int64_t out_stride, void* workspace, int64_t workspace_bytes,

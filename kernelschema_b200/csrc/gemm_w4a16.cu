@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(256) k_w4a16_reduce(const W4A16Params p, int b
 
 // Tile width and, up to 128 rows, the split of the last wave. The tiles left over after whole waves are shared by as many CTAs as
 // the SMs hold (at most eight, at least one k-group each). Behind whole waves that pays for its partial tiles and the second launch
-// only when a tile is long: from 16 k-groups on. The plan of a batch of 33 to 128 rows does not depend on its rows, so a row has
+// only when a tile is long: from 16 k-groups on. The plan of a batch of 17 to 128 rows does not depend on its rows, so a row has
 // one value in all of them. Above, which tiles end up in the last wave depends on the batch: a split there would give a row other
 // last bits at another position, so there is none, which gives up time (8192 x 4096 x 12288 696 us with a split, 759 without;
 // 129 x 4096 x 4096 23 and 42). `room`: the caller has a workspace for the partial tiles.
@@ -426,7 +426,7 @@ static W4A16Plan w4a16_plan(int64_t m, int64_t n, int64_t k, int sms, bool room)
   int64_t s = tail ? sms / tail : 1;
   if (s > 8) s = 8;
   if (s > groups) s = groups;
-  if (s < 2 || !room || m > 128 || w4a16_decode_fits(m) || (tiles > tail && groups < 16)) s = 1;
+  if (s < 2 || !room || m > 128 || w4a16_decode_wins(m, n, k) || (tiles > tail && groups < 16)) s = 1;
   pl.splits = (int)s;
   pl.tail_tiles = s > 1 ? (int)tail : 0;
   pl.full_tiles = (int)(tiles - pl.tail_tiles);
@@ -449,11 +449,13 @@ int launch_gemm_w4a16(const void* a, int64_t a_stride, const void* b_q, const vo
                       int64_t k, void* out, int64_t out_stride, void* workspace, int64_t workspace_bytes, int32_t* status,
                       cudaStream_t st) {
   if (m == 0) return 0;
-  // workspace_bytes < 0: one sum in ascending k per element at every size, so the tile kernel, unsplit
-  if (workspace_bytes >= 0 && w4a16_decode_fits(m)) return launch_gemm_w4a16_decode(a, a_stride, b_q, b_sf, alpha, m, n, k, out, out_stride, st);
   const int sms = sm_count();
   W4A16Plan pl = w4a16_plan(m, n, k, sms, true);
-  if (pl.splits > 1 && (!workspace || workspace_bytes < w4a16_partial_bytes(pl, m))) pl = w4a16_plan(m, n, k, sms, false);
+  const bool no_room = pl.splits > 1 && (!workspace || workspace_bytes < w4a16_partial_bytes(pl, m));
+  // workspace_bytes < 0: one sum in ascending k per element at every size, so the tile kernel, unsplit
+  if (workspace_bytes >= 0 && m <= kW4A16DecodeMaxM && (no_room || w4a16_decode_wins(m, n, k)))
+    return launch_gemm_w4a16_decode(a, a_stride, b_q, b_sf, alpha, m, n, k, out, out_stride, st);
+  if (no_room) pl = w4a16_plan(m, n, k, sms, false);
   const int bn = pl.bn;
   CUtensorMap ta;
   int rc = make_operand_map(&ta, a, (uint64_t)m, (uint64_t)k * 2, 256, (uint64_t)a_stride * 2);

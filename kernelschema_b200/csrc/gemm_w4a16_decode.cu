@@ -199,15 +199,21 @@ k_gemm_w4a16_decode(const __nv_bfloat16* __restrict__ a, int64_t a_stride, const
   cluster_sync_all();                                          // nobody leaves while a peer still reads its sums
 }
 
+// Blocks per row tile: double while all are resident at once and the added blocks would have K to work on. Counting two per SM
+// for 32 tokens, of which one is resident, made two uneven waves of clusters (32 x 2048 x 7168 22.4 us against 12.4 with one). With
+// one block per SM the GPCs do not hold as many clusters of eight as there are SMs for, so those stop at half the device.
+int dec_split(int64_t n, int64_t k, int per_sm) {
+  const int64_t tiles = n / kDecRows, units = k / kDecUnit, slots = (int64_t)sm_count() * per_sm;
+  const int most = per_sm > 1 || tiles * 16 <= slots ? 8 : 4;
+  int split = 1;
+  while (split < most && tiles * split * 2 <= slots && units > (int64_t)split * kDecWarps) split *= 2;
+  return split;
+}
+
 template <int NT>
 int launch_nt(const void* a, int64_t a_stride, const void* b_q, const void* b_sf, const float* alpha, int64_t m, int64_t n, int64_t k,
               void* out, int64_t out_stride, cudaStream_t st) {
-  // Blocks per row tile: double while all are resident at once and the added blocks would have K to work on. Counting two per SM
-  // for 32 tokens, of which one is resident, made two uneven waves of clusters (32 x 2048 x 7168 22.4 us against 12.4 with one,
-  // 32 x 8192 x 12288 56.7 against 50.5; 32 x 7168 x 18432, whose 112 tiles are one short wave, 78.7 against 83.5).
-  const int64_t tiles = n / kDecRows, units = k / kDecUnit, slots = (int64_t)sm_count() * dec_blocks_per_sm<NT>();
-  int split = 1;
-  while (split < 8 && tiles * split * 2 <= slots && units > (int64_t)split * kDecWarps) split *= 2;
+  const int split = dec_split(n, k, dec_blocks_per_sm<NT>());
   static SmemOptIn opt_in;
   if (int e = opt_in.ensure(k_gemm_w4a16_decode<NT>, dec_smem_bytes<NT>())) return e;
   cudaLaunchConfig_t cfg = {};
@@ -230,7 +236,17 @@ int launch_nt(const void* a, int64_t a_stride, const void* b_q, const void* b_sf
 
 }  // namespace
 
-bool w4a16_decode_fits(int64_t m) { return m <= kW4A16DecodeMaxM; }
+// Where this kernel is the faster one: up to 16 rows always; up to 32 while a warp takes at most four units of K, in one wave of
+// blocks. Its issue time grows with the units and nothing overlaps them, the tile kernel's does not (microseconds a call among
+// others, here / tile kernel: 32 x 8192 x 4096, four units, 17.6 / 25.7; 32 x 4096 x 8192, four, 20.1 / 21.9; 32 x 4096 x 12288, six,
+// 33.5 / 31.7; 32 x 6144 x 8192, eight, 43.1 / 30.8; 32 x 8192 x 12288, twelve, 69.6 / 54.2; two waves, 32 x 16384 x 4096, 44.5 / 42.6).
+// By N and K alone within a range, so a row has one value in all batches of the range.
+bool w4a16_decode_wins(int64_t m, int64_t n, int64_t k) {
+  if (m <= 16) return true;
+  if (m > kW4A16DecodeMaxM) return false;
+  const int64_t split = dec_split(n, k, dec_blocks_per_sm<4>()), tiles = n / kDecRows, units = k / kDecUnit, sms = sm_count();
+  return tiles * split <= sms && (units + split * kDecWarps - 1) / (split * kDecWarps) <= 4;
+}
 
 int launch_gemm_w4a16_decode(const void* a, int64_t a_stride, const void* b_q, const void* b_sf, const float* alpha, int64_t m,
                              int64_t n, int64_t k, void* out, int64_t out_stride, cudaStream_t st) {

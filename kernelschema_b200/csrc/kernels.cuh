@@ -165,7 +165,7 @@ int launch_gemm_w4a16(const void* a, int64_t a_stride, const void* b_q, const vo
                       cudaStream_t st);
 // A handful of tokens (gemm_w4a16_decode.cu): no workspace, one launch.
 constexpr int kW4A16DecodeMaxM = 32;
-bool w4a16_decode_fits(int64_t m);
+bool w4a16_decode_wins(int64_t m, int64_t n, int64_t k);
 int launch_gemm_w4a16_decode(const void* a, int64_t a_stride, const void* b_q, const void* b_sf, const float* alpha, int64_t m,
                              int64_t n, int64_t k, void* out, int64_t out_stride, cudaStream_t st);
 int64_t gemm_w4a16_workspace_bytes(int64_t m, int64_t n, int64_t k);

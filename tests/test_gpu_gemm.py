@@ -154,7 +154,8 @@ def test_w4a16_matches_oracle(m, n, k, outliers):
 
 
 @pytest.mark.parametrize("m,n,k", [(1, 128, 256), (7, 384, 2304), (8, 4096, 12288), (9, 1024, 4096), (16, 8192, 512), (17, 256, 2048),
-                                   (31, 7168, 768), (32, 128, 12288)])
+                                   (31, 7168, 768), (32, 128, 12288), (17, 8192, 4096),
+                                   (32, 8192, 4352), (20, 1024, 12288), (24, 9600, 2048)])
 def test_w4a16_decode_sizes_all_codes(m, n, k):
     """A handful of tokens: every code and every scale byte (subnormal scales and the 0.5 code among them) in random places,
     a strided A, and rows beyond M left alone. Sums of K products differ from the oracle's only by the order of the fp32
@@ -259,7 +260,8 @@ def test_w4a16_split_on_two_streams_and_in_a_graph():
 
 
 @pytest.mark.parametrize("n,k,sizes", [(4096, 4096, (129, 300, 1024, 1025, 1280, 1281, 2600)), (3328, 4352, (200, 3000)), (1152, 8192, (150, 1300)),
-                                       (4096, 8192, (33, 64, 65, 128)), (20480, 4096, (40, 128)), (4096, 12288, (1, 8, 9, 16)), (2048, 7168, (17, 24, 32))])
+                                       (4096, 8192, (33, 64, 65, 128)), (20480, 4096, (40, 128)), (4096, 12288, (1, 8, 9, 16)), (2048, 7168, (17, 24, 32)),
+                                       (6144, 8192, (17, 24, 32)), (1024, 12288, (17, 32))])
 def test_w4a16_a_row_has_one_value(n, k, sizes):
     """A row gives the same bits at any position and in any batch of 1..16, 17..32, 33..128 and more than 128 rows: long K, fewer
     tiles than SMs (128-wide up to 1024 rows x 4096, 256-wide above) as well as a partly filled last wave behind whole ones. With split_k=False the bits are those of more than 128
