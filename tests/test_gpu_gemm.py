@@ -157,8 +157,9 @@ def test_w4a16_matches_oracle(m, n, k, outliers):
                                    (31, 7168, 768), (32, 128, 12288), (17, 8192, 4096),
                                    (32, 8192, 4352), (20, 1024, 12288), (24, 9600, 2048)])
 def test_w4a16_decode_sizes_all_codes(m, n, k):
-    """A handful of tokens: every code and every scale byte (subnormal scales and the 0.5 code among them) in random places,
-    a strided A, and rows beyond M left alone. Sums of K products differ from the oracle's only by the order of the fp32
+    """A handful of tokens, and from 17 rows on both sides of the rule that leaves long K (32 x 8192 x 4352) and a second wave of
+    blocks (24 x 9600 x 2048) to the tile kernel: every code and every scale byte (subnormal scales and the 0.5 code among them)
+    in random places, a strided A, and rows beyond M left alone. Sums of K products differ from the oracle's only by the order of the fp32
     additions, so a bf16 step (2^-8) of the result plus 2^-20 of the sum of magnitudes bounds every element."""
     import kernelschema_b200 as ks
     rng = np.random.default_rng(m + n + k)
