@@ -168,6 +168,11 @@ constexpr int kW4A16DecodeMaxM = 32;
 bool w4a16_decode_wins(int64_t m, int64_t n, int64_t k);
 int launch_gemm_w4a16_decode(const void* a, int64_t a_stride, const void* b_q, const void* b_sf, const float* alpha, int64_t m,
                              int64_t n, int64_t k, void* out, int64_t out_stride, cudaStream_t st);
+// Many tokens (gemm_w4a16_expand.cu): the weights expanded to bf16 once, in a scratch of n * k * 2 bytes, then a bf16 GEMM.
+constexpr int64_t kW4A16ExpandMax = 1ll << 28;
+bool w4a16_expand_wins(int64_t m, int64_t n, int64_t k);
+int launch_gemm_w4a16_expand(const void* a, int64_t a_stride, const void* b_q, const void* b_sf, const float* alpha, int64_t m,
+                             int64_t n, int64_t k, void* out, int64_t out_stride, void* scratch, int32_t* status, cudaStream_t st);
 int64_t gemm_w4a16_workspace_bytes(int64_t m, int64_t n, int64_t k);
 int make_sf_map(CUtensorMap* map, const void* base, uint64_t n_chunks);
 

@@ -164,6 +164,16 @@ def _w4a16_workspace(device: torch.device, stream: int, need: int) -> torch.Tens
     return ws
 
 
+def _w4a16_expanded(device: torch.device, need: int) -> torch.Tensor | None:
+    """Scratch for the expanded weights of one call with many rows (up to 256 MB): taken from the caching allocator and given back
+    when the call has been launched, so no buffer of that size stays with a thread or a stream. Without memory for it the call
+    runs the kernel that needs none."""
+    try:
+        return torch.empty(need, dtype=torch.uint8, device=device)
+    except torch.OutOfMemoryError:
+        return None
+
+
 def mm_bf16_nvfp4(a: torch.Tensor, b: torch.Tensor, b_descale: torch.Tensor, alpha: torch.Tensor | None = None,
                   out: torch.Tensor | None = None, status: torch.Tensor | None = None, split_k: bool = True) -> torch.Tensor:
     """out[M, N] = bf16(alpha * a @ decode(b)^T): bf16 activations [M, K] (not quantised), NVFP4 weights uint8 [N, K/2] with
@@ -188,7 +198,7 @@ def mm_bf16_nvfp4(a: torch.Tensor, b: torch.Tensor, b_descale: torch.Tensor, alp
     ws, stream = None, _stream()
     need = int(lib.b200moe_gemm_bf16_nvfp4_workspace_bytes(m, n, k)) if split_k else -1
     if need > 0:
-        ws = _w4a16_workspace(a.device, stream, need)
+        ws = _w4a16_workspace(a.device, stream, need) if m <= 128 else _w4a16_expanded(a.device, need)
     _lib.check(lib.b200moe_gemm_bf16_nvfp4(a.data_ptr(), a.stride(0), b.data_ptr(), b_descale.data_ptr(), _ptr(alpha), out.data_ptr(),
                                            m, n, k, out.stride(0), _ptr(ws), need, _ptr(status), stream),
                "b200moe_gemm_bf16_nvfp4")

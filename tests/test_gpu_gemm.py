@@ -327,3 +327,31 @@ def test_w4a16_split_k_small_m(m, n, k):
         r = compare_outputs(got, ref)
         assert r["rel_l2"] <= 1e-3 and r["max_abs"] <= 2e-2 * r["rms"], r
         assert (np.abs(got - ref) <= 0.01 + 0.05 * np.abs(ref)).all()
+
+
+@pytest.mark.parametrize("m,n,k", [(129, 128, 1280), (256, 384, 2304), (257, 1152, 4096), (300, 640, 1280), (385, 4096, 12288), (1025, 2176, 1536),
+                                   (3000, 1280, 2304)])
+def test_w4a16_expanded_weights(m, n, k):
+    """Above 128 rows the weights are expanded to bf16 first: every payload byte and every finite scale code, odd rows (a last row tile of
+    1, 44 and 129 rows), a half-empty 256-wide column tile, both tile widths, expansions of one and of several waves, ten calls in a
+    row. Same bits as the kernel that decodes tile by tile; that one and the product agree with 64-bit sums to one bf16 rounding
+    (2^-9 of the element) plus fp32 accumulation (k * 2^-24 of the sum of magnitudes at most)."""
+    import kernelschema_b200 as ks
+    from kernelschema_b200 import _lib
+    assert _lib.load().b200moe_gemm_bf16_nvfp4_workspace_bytes(m, n, k) == n * k * 2
+    gen = torch.Generator(device="cuda").manual_seed(m + n)
+    wide = torch.randn(m, k + 8, device="cuda", generator=gen).to(torch.bfloat16)
+    a = wide[:, :k]
+    bq = torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device="cuda", generator=gen)
+    sf = torch.randint(0, 127, (n, k // 16), dtype=torch.uint8, device="cuda", generator=gen)
+    sf |= torch.randint(0, 2, sf.shape, dtype=torch.uint8, device="cuda", generator=gen) << 7
+    alpha = torch.full((1,), 2.0 ** -9, device="cuda")
+    y = [ks.mm_bf16_nvfp4(a, bq, sf, alpha) for _ in range(10)]
+    want = ks.mm_bf16_nvfp4(a, bq, sf, alpha, split_k=False)
+    assert all(torch.equal(v, want) for v in y)
+    code = torch.tensor([0, 0.5, 1, 1.5, 2, 3, 4, 6, -0.0, -0.5, -1, -1.5, -2, -3, -4, -6], device="cuda", dtype=torch.float64)
+    w = code[torch.stack([bq & 15, bq >> 4], dim=-1).long()].view(n, k) * sf.view(torch.float8_e4m3fn).double().repeat_interleave(16, dim=1)
+    rows = torch.unique(torch.cat([torch.arange(min(m, 130)), torch.arange(m - 130, m)])).cuda()
+    x = a[rows].double()
+    exact, mag = (x @ w.t()) * 2.0 ** -9, (x.abs() @ w.abs().t()) * 2.0 ** -9
+    assert ((y[0][rows].double() - exact).abs() <= exact.abs() * 2.0 ** -8 + mag * (k * 2.0 ** -24)).all()
