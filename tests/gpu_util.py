@@ -18,8 +18,9 @@ def guarded_output(t, h):
     return backing, backing[64:-64].view(t, h)
 
 
-def run_model(p, model=None):
-    """Run the drop-in Model on a numpy case; returns (output fp32 numpy, backing tensor, model)."""
+def run_model(p, model=None, shift_ids=0):
+    """Run the drop-in Model on a numpy case; returns (output fp32 numpy, backing tensor, model). `shift_ids`: the expert ids start that
+    many elements behind a 256-byte boundary."""
     model = model or ks.Model()
     ids, scores = p["topk_ids"]
     t = p["hidden_states"].shape[0]
@@ -27,8 +28,11 @@ def run_model(p, model=None):
     backing, out = guarded_output(t, h)
     etot = p["gemm1_weights"].shape[0]
     shared = int(p.get("num_fused_shared_experts") or 0)
+    ids_dev = to_dev(ids.astype(np.int32))
+    if shift_ids:
+        ids_dev = torch.cat([ids_dev.new_zeros(shift_ids), ids_dev.flatten()])[shift_ids:].view(ids_dev.shape)
     kw = dict(
-        topk_ids=(to_dev(ids.astype(np.int32)), to_dev(scores.astype(np.float32))), routing_bias=None,
+        topk_ids=(ids_dev, to_dev(scores.astype(np.float32))), routing_bias=None,
         hidden_states=to_dev(p["hidden_states"]), hidden_states_scale=to_dev(p["hidden_states_scale"], torch.float8_e4m3fn),
         gemm1_weights=to_dev(p["gemm1_weights"]), gemm1_weights_scale=to_dev(p["gemm1_weights_scale"], torch.float8_e4m3fn),
         gemm1_bias=None, gemm1_alpha=to_dev(p["gemm1_alpha"]), gemm1_beta=to_dev(p["gemm1_beta"]),

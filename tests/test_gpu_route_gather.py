@@ -125,3 +125,16 @@ def test_large_batch_both_payload_modes(tokens, tma_gather):
     got, _, model = run_model(p, ks.Model(tma_gather=tma_gather))
     _check_map_and_rows(p, model)
     assert_layer_parity(got, o.moe_expected(p), f"tma_gather={tma_gather}")
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("tokens,top_k,hidden", [(1581, 3, 2048), (1583, 3, 2304), (3163, 3, 1024), (2047, 8, 2048)])
+def test_many_routes_counted_four_at_a_time(tokens, top_k, hidden, shift):
+    """Routed slots only, so the ids are counted with 128-bit loads (4743, 4749 and 9489 routes leave one or three over), and one by one
+    when they do not start at a 16-byte boundary (`shift`); rows of up to 2048 elements are copied four at a time, longer ones singly."""
+    import kernelschema_b200 as ks
+    from gpu_util import run_model
+    p = make_moe_case(500 + tokens, tokens, hidden, 256, 24, top_k, routing="zipf", masked=True)
+    got, _, model = run_model(p, ks.Model(), shift_ids=shift)
+    _check_map_and_rows(p, model)
+    assert_layer_parity(got, o.moe_expected(p), f"T={tokens} H={hidden} shift={shift}")
