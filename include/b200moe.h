@@ -121,6 +121,10 @@ const char* b200moe_last_error(void);
  * scales: layout B200MOE_SF_ROW_MAJOR or B200MOE_SF_TILED (caller sizes it for rows rounded up to 128). */
 int b200moe_quantize_nvfp4(const void* x, int64_t rows, int64_t cols, int64_t row_stride, float global_scale, void* payload,
                            void* scales, int32_t scale_layout, void* stream);
+/* The same with tiled scales whose last tile is whole: the rows that it has beyond the matrix, which the call above leaves as they are,
+ * become zero. scales 4-byte aligned. */
+int b200moe_quantize_nvfp4_tiles(const void* x, int64_t rows, int64_t cols, int64_t row_stride, float global_scale, void* payload,
+                                 void* scales, void* stream);
 
 /* Row-major scale bytes [rows, cols/16] -> 128x4 tiles (the block_scales() step of NV/problem/input.py:82-87
  * for one matrix). dst holds ceil(rows/128)*128 * cols/16 bytes; padding rows become 0. */

@@ -74,6 +74,8 @@ SIGNATURES = {
     "b200moe_last_error": (C.c_char_p, []),
     "b200moe_quantize_nvfp4": (C.c_int, [C.c_void_p, C.c_int64, C.c_int64, C.c_int64, C.c_float, C.c_void_p, C.c_void_p,
                                          C.c_int32, C.c_void_p]),
+    "b200moe_quantize_nvfp4_tiles": (C.c_int, [C.c_void_p, C.c_int64, C.c_int64, C.c_int64, C.c_float, C.c_void_p, C.c_void_p,
+                                               C.c_void_p]),
     "b200moe_scales_to_tiles": (C.c_int, [C.c_void_p, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p]),
     "b200moe_route_topk": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int64, C.c_int32, C.c_int32, C.c_void_p, C.c_void_p,
                                      C.c_void_p]),

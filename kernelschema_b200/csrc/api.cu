@@ -376,16 +376,27 @@ extern "C" {
 int b200moe_abi_version(void) { return B200MOE_ABI_VERSION; }
 const char* b200moe_last_error(void) { return g_err; }
 
-int b200moe_quantize_nvfp4(const void* x, int64_t rows, int64_t cols, int64_t row_stride, float global_scale, void* payload,
-                           void* scales, int32_t scale_layout, void* stream) {
+static int quantize_checked(const void* x, int64_t rows, int64_t cols, int64_t row_stride, float global_scale, void* payload, void* scales,
+                            int32_t scale_layout, bool clear_tile, void* stream) {
   if (rows < 0 || cols <= 0 || cols % 64) return fail(740, "quantize: cols=%lld must be a positive multiple of 64", (long long)cols);
   if (row_stride < cols || row_stride % 8) return fail(741, "quantize: row_stride must be >= cols and a multiple of 8");
   if (rows && (!x || !payload || !scales)) return fail(742, "quantize: null pointer");
   if (((uintptr_t)x & 15) || ((uintptr_t)payload & 7)) return fail(743, "quantize: x must be 16-byte and payload 8-byte aligned");
   if (!(global_scale > 0.f)) return fail(744, "quantize: global_scale must be positive");
   if (scale_layout != B200MOE_SF_ROW_MAJOR && scale_layout != B200MOE_SF_TILED) return fail(745, "quantize: unknown scale_layout");
-  return cuda_fail(launch_quantize_nvfp4(x, rows, cols, row_stride, global_scale, payload, scales, scale_layout, (cudaStream_t)stream),
+  if (clear_tile && ((uintptr_t)scales & 3)) return fail(743, "quantize: scales must be 4-byte aligned to be cleared");
+  return cuda_fail(launch_quantize_nvfp4(x, rows, cols, row_stride, global_scale, payload, scales, scale_layout, clear_tile, (cudaStream_t)stream),
                    "quantize");
+}
+
+int b200moe_quantize_nvfp4(const void* x, int64_t rows, int64_t cols, int64_t row_stride, float global_scale, void* payload,
+                           void* scales, int32_t scale_layout, void* stream) {
+  return quantize_checked(x, rows, cols, row_stride, global_scale, payload, scales, scale_layout, false, stream);
+}
+
+int b200moe_quantize_nvfp4_tiles(const void* x, int64_t rows, int64_t cols, int64_t row_stride, float global_scale, void* payload,
+                                 void* scales, void* stream) {
+  return quantize_checked(x, rows, cols, row_stride, global_scale, payload, scales, B200MOE_SF_TILED, true, stream);
 }
 
 int b200moe_scales_to_tiles(const void* src, int64_t rows, int64_t cols, void* dst, void* stream) {
@@ -897,7 +908,7 @@ static int step_impl(b200moe_layer* h, const b200moe_step_args* a, cudaStream_t 
                             h->step_hs, st);
   else
     rc = launch_quantize_nvfp4(a->x, T, c.hidden, a->x_stride, a->activation_global_scale, h->step_hq, h->step_hs,
-                               B200MOE_SF_ROW_MAJOR, qs);
+                               B200MOE_SF_ROW_MAJOR, false, qs);
   if (c.top_k > 0) {
     if (!one_front) rc_router = router_logits_any(a->x, a->gate_weight, T, c.hidden, c.num_experts, h->step_logits, st);
     if (rc_router) where = "step: router logits";

@@ -103,7 +103,7 @@ struct GemmParams {
 };
 
 int launch_quantize_nvfp4(const void* x, int64_t rows, int64_t cols, int64_t row_stride, float gs, void* payload, void* scales,
-                          int sf_layout, cudaStream_t st);
+                          int sf_layout, bool clear_tile, cudaStream_t st);   // clear_tile: a tiled image's rows beyond the matrix become 0
 int launch_sf_to_tiles(const void* src, int64_t rows, int64_t blocks_per_row, void* dst, cudaStream_t st);
 int launch_route_topk(const float* logits, const float* bias, int64_t T, int E, int K, int32_t* ids, float* weights,
                       cudaStream_t st);

@@ -69,12 +69,14 @@ def nvfp4_quantize(x: torch.Tensor, global_scale: float = 1.0, tiled_scales: boo
     else:
         payload = torch.empty((rows, cols // 2), dtype=torch.uint8, device=x.device)
         if tiled_scales:
-            # the kernel writes every row it has; only a ragged last tile holds others
-            alloc = torch.zeros if rows % 128 else torch.empty
-            scales = alloc(((rows + 127) // 128, cols // 64, 32, 16), dtype=torch.uint8, device=x.device)
+            scales = torch.empty(((rows + 127) // 128, cols // 64, 32, 16), dtype=torch.uint8, device=x.device)
         else:
             scales = torch.empty((rows, cols // 16), dtype=torch.uint8, device=x.device)
     lib = _lib.load()
+    if tiled_scales and out is None:       # a ragged last tile holds rows that the matrix does not have: they become zero
+        _lib.check(lib.b200moe_quantize_nvfp4_tiles(x.data_ptr(), rows, cols, x.stride(0), float(global_scale), payload.data_ptr(),
+                                                    scales.data_ptr(), _stream()), "b200moe_quantize_nvfp4_tiles")
+        return payload, scales
     _lib.check(lib.b200moe_quantize_nvfp4(x.data_ptr(), rows, cols, x.stride(0), float(global_scale), payload.data_ptr(),
                                           scales.data_ptr(), _lib.SF_TILED if tiled_scales else _lib.SF_ROW_MAJOR, _stream()),
                "b200moe_quantize_nvfp4")

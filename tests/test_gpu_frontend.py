@@ -67,6 +67,20 @@ def test_quantize_short_rows_odd_strides_and_scale_alignment(rows, cols, pad, of
         assert not s[:offset].any() and not s[offset + n:].any()
 
 
+@pytest.mark.parametrize("rows,cols", [(1, 64), (1, 8192), (127, 192), (129, 320), (300, 4160), (9999, 64), (257, 7168)])
+def test_quantize_clears_a_ragged_last_tile(rows, cols):
+    """Without `out` the tiled scales come from dirty memory: the rows that the last tile has beyond the matrix are zero, by threads of
+    blocks with one and several rows, fewer and more of them than there are words to clear."""
+    import kernelschema_b200 as ks
+    x = torch.randn(rows, cols, generator=torch.Generator().manual_seed(rows)).to(torch.bfloat16)
+    want = o.block_scales(o.quantize(x.float().numpy(), 16, 0.0021)[1][None])[0]
+    x = x.cuda()
+    for _ in range(3):
+        dirty = torch.full((want.size,), 255, dtype=torch.uint8, device="cuda")
+        del dirty
+        assert np.array_equal(ks.nvfp4_quantize(x, 0.0021, tiled_scales=True)[1].cpu().numpy(), want)
+
+
 def _torch_quantize_true_division(x, gs):
     """The reference quantize() (gemm/dense/bf16_nvfp4_gemm/problem/input.py:40-64) in torch ops on the device with
     tensor / tensor divisions only (IEEE round-to-nearest; tensor / python-scalar would multiply by a reciprocal)."""
