@@ -27,7 +27,8 @@ def _shim():
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current device's current stream (`torch.cuda.current_stream()` builds a Stream object: 5.4 us a call)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _need_cuda(*tensors) -> None:
