@@ -444,7 +444,11 @@ int b200moe_router_logits(const void* x, const void* w, int64_t T, int32_t H, in
 
 int b200moe_gemm_nvfp4(const void* a_q, const void* a_sf, const void* b_q, const void* b_sf, float alpha, void* out, int64_t m,
                        int64_t n, int64_t k, int64_t out_stride, int32_t tile_n, int32_t* status, void* stream) {
-  const int bn = tile_n ? tile_n : (n % 256 == 0 ? 256 : 128);
+  // While all 128-wide tiles run at once they are the faster ones: half of the work each on SMs that would idle (microseconds 256 / 128
+  // wide: 512 x 1024 x 1024 5.5 / 4.2, 512 x 2048 x 8192 16.4 / 11.7, 256 x 8192 x 8192 16.7 / 12.1). Beyond one wave the wide tile moves
+  // less for the same product (2048 x 2048 x 8192 14.4 / 20.6). Both add in the same order.
+  const int64_t wide_tiles = (m + 127) / 128 * (n / 256);
+  const int bn = tile_n ? tile_n : (n % 256 == 0 && wide_tiles * 2 > sm_count() ? 256 : 128);
   if (bn != 128 && bn != 256 && bn != 512) return fail(760, "gemm: tile_n must be 0, 128, 256 or 512");
   if (m < 0 || n <= 0 || k <= 0 || k % 256 || n % (bn == 512 ? 256 : bn))
     return fail(761, "gemm: need K %% 256 == 0 and N %% tile_n == 0 (N %% 256 == 0 for the CTA-pair tile)");

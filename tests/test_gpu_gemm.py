@@ -355,3 +355,14 @@ def test_w4a16_expanded_weights(m, n, k):
     x = a[rows].double()
     exact, mag = (x @ w.t()) * 2.0 ** -9, (x.abs() @ w.abs().t()) * 2.0 ** -9
     assert ((y[0][rows].double() - exact).abs() <= exact.abs() * 2.0 ** -8 + mag * (k * 2.0 ** -24)).all()
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 256, 512), (130, 512, 2304), (128, 18944, 512), (128, 19200, 512), (4736, 512, 768), (4737, 512, 768)])
+def test_dense_gemm_default_tile_width(m, n, k):
+    """tile_n = 0 on both sides of the line where the 128-wide tiles stop running at once (148 of them): the bits of either explicit width."""
+    import kernelschema_b200 as ks
+    gen = torch.Generator(device="cuda").manual_seed(m + n)
+    aq, asf = ks.nvfp4_quantize(torch.randn(m, k, device="cuda", generator=gen).to(torch.bfloat16), 1.0, tiled_scales=True)
+    bq, bsf = ks.nvfp4_quantize(torch.randn(n, k, device="cuda", generator=gen).to(torch.bfloat16), 1.0, tiled_scales=True)
+    y = [ks.mm_nvfp4(aq, asf, bq, bsf, alpha=0.5, tile_n=t) for t in (0, 128, 256)]
+    assert torch.equal(y[0], y[1]) and torch.equal(y[0], y[2])
