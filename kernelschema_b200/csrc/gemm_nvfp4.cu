@@ -23,12 +23,12 @@
 // tensor cycles). 8192^3, lane test -> elect.sync: CTA-pair kernel
 // 356 -> 223 us (one thread issues for two SMs), 128 x 128 tiles 279 -> 266 us, 128 x 256 tiles 231 -> 227 us.
 //
-// With a long k-loop and enough rows the stage ring is bound by its round trip (TMA latency, hand-over, MMA, commit; about
-// 1.5 us over four stages), not by issue: there the MMA thread copies a stage's scale factors itself, in order before its MMAs,
-// because copier warps between TMA and MMA cost a barrier hop per stage (8192^3 222 -> 207 us without them, 203 us with no scale
-// copies at all; DeepSeek-V3 FC1 at T = 8192 1030 -> 978 us). A batch that streams weights, or a short k-loop, drains stages that
-// are already there at the issue rate, and two copier warps beside the MMA thread are faster (Qwen3 FC1 T = 64 43.4 us against
-// 45.4, T = 16384 183 against 187; T = 1 23.4 us a step against 24.3).
+// The stage ring is bound by its round trip (TMA latency, hand-over, MMA, commit; about 1.5 us over four stages), not by issue, so the
+// MMA thread copies a stage's scale factors itself, in order before its MMAs: copier warps between TMA and MMA cost a barrier hop per
+// stage (8192^3 222 -> 207 us without them, 203 us with no scale copies at all; dense 1024 x 8192 x 4096 19.6 -> 16.7 us, 16384 x 7168 x
+// 2048 118.8 -> 116.6, 128-wide tiles 3000 x 3968 x 8192 53.8 -> 50.3; layer T = 1, Qwen3, 23.7 -> 22.7 us a step, T = 100, 256 experts
+// of 256 channels 158.1 -> 153.5). Two copier warps remain for layer launches of 256-wide tiles with a long k-loop that stream weights
+// (copier_form).
 #include "kernels.cuh"
 #include "ptx.cuh"
 
@@ -233,13 +233,11 @@ DEV void epilogue_cols(const GemmParams& p, uint32_t taddr, const EpiScale& sc, 
   }
 }
 
-// Warp roles: 0 = TMA producer, 1 = TMEM owner + issuer of the MMAs (and of the scale copies), then kGemmCopiers scale copiers,
+// Warp roles: 0 = TMA producer, 1 = TMEM owner + issuer of the MMAs (and of the scale copies), then COP (2 or 0) scale copiers,
 // then 4 * BN/EC epilogue warps; epilogue warp w owns TMEM lane quadrant w & 3 and an EC-column group.
-template <int EC>
-constexpr int kGemmCopiers = EC == 64 ? 2 : 0;
 // any four consecutive warps own the four TMEM lane quadrants (quadrant = warp & 3), so the epilogue groups may start anywhere
-template <int BN, int EC>
-constexpr int gemm_threads() { return 32 * (2 + kGemmCopiers<EC> + 4 * BN / EC); }
+template <int BN, int EC, int COP>
+constexpr int gemm_threads() { return 32 * (2 + COP + 4 * BN / EC); }
 
 // Scale-factor copy j of a stage (j < 4: A scales of k-block j; then B scales, 128-row half h, k-block q) from the
 // stage's shared-memory slots into its TMEM buffer.
@@ -275,12 +273,12 @@ DEV void copier_loop(const GemmParams& p, uint32_t tmem, uint32_t s_sfa, uint32_
   }
 }
 
-template <int MODE, int BN, int EC>
-__global__ void __launch_bounds__(gemm_threads<BN, EC>(), 1)
+template <int MODE, int BN, int EC, int COP>
+__global__ void __launch_bounds__(gemm_threads<BN, EC, COP>(), 1)
 k_gemm_nvfp4(const __grid_constant__ ActMaps am, const __grid_constant__ CUtensorMap tm_b, const GemmParams p) {
   using C = GemmCfg<BN>;
   constexpr int kEpiWarps = 4 * BN / EC;
-  constexpr int kCopiers = kGemmCopiers<EC>;
+  constexpr int kCopiers = COP;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t s_a = smem_base;
@@ -779,12 +777,12 @@ int launch_gemm_nvfp4_pair(int mode, const CUtensorMap& ta, const CUtensorMap& t
   return launch_pair<kGemmDense>(ta, tb, tsa, tsb, p, grid, st);
 }
 
-template <int MODE, int BN, int EC>
+template <int MODE, int BN, int EC, int COP>
 static int launch_one(const ActMaps& ta, const CUtensorMap& tb, const GemmParams& p, int grid, cudaStream_t st) {
-  auto kern = k_gemm_nvfp4<MODE, BN, EC>;
+  auto kern = k_gemm_nvfp4<MODE, BN, EC, COP>;
   static SmemOptIn opt_in;
   if (int e = opt_in.ensure(kern, GemmCfg<BN>::kSmemBytes)) return e;
-  return (int)launch_chain(kern, dim3(grid), dim3(gemm_threads<BN, EC>()), GemmCfg<BN>::kSmemBytes, st, ta, tb, p);
+  return (int)launch_chain(kern, dim3(grid), dim3(gemm_threads<BN, EC, COP>()), GemmCfg<BN>::kSmemBytes, st, ta, tb, p);
 }
 
 // The form for tensor-bound launches with a long k-loop: eight epilogue warps x 128 columns (hidden by the loop, less power) and
@@ -796,11 +794,18 @@ static int launch_one(const ActMaps& ta, const CUtensorMap& tb, const GemmParams
 // and 15.8.
 static bool long_loop_form(int mode, int k, int64_t rows_hint) { return k >= 4096 && rows_hint >= (mode == kGemmDense ? 2048 : 32768); }
 
+// Copier warps beside the MMA thread, for layers with a long k-loop: the stages of a weight stream arrive in bursts and are drained
+// at the issue rate (DeepSeek-V3 T = 64, K = 7168, 412 us a step with copiers, 414.5 without).
+static bool copier_form(int k) { return k >= 4096; }
+
 template <int MODE>
 static int launch_mode(int bn, const ActMaps& ta, const CUtensorMap& tb, const GemmParams& p, int grid, cudaStream_t st) {
-  if (bn == 128) return launch_one<MODE, 128, 64>(ta, tb, p, grid, st);
-  if (bn == 256) return long_loop_form(MODE, p.K, p.rows_hint) ? launch_one<MODE, 256, 128>(ta, tb, p, grid, st) : launch_one<MODE, 256, 64>(ta, tb, p, grid, st);
-  return 703;
+  if (bn == 128) return launch_one<MODE, 128, 64, 0>(ta, tb, p, grid, st);
+  if (bn != 256) return 703;
+  if (long_loop_form(MODE, p.K, p.rows_hint)) return launch_one<MODE, 256, 128, 0>(ta, tb, p, grid, st);
+  if constexpr (MODE != kGemmDense)
+    if (copier_form(p.K)) return launch_one<MODE, 256, 64, 2>(ta, tb, p, grid, st);
+  return launch_one<MODE, 256, 64, 0>(ta, tb, p, grid, st);
 }
 
 int launch_gemm_nvfp4(int mode, int bn, const ActMaps& ta, const CUtensorMap& tb, const GemmParams& p, int grid,
