@@ -22,6 +22,9 @@
 // r * 128 + ((c ^ (r & 7)) * 16)), then fence.proxy.async + mbarrier arrive; the last 8 warps = epilogue.
 // Every wait is bounded and reports through the status word.
 //
+// Above 128 rows this kernel serves calls without a workspace and the few shapes where expanding the weights first is not faster
+// (gemm_w4a16_expand.cu, the same bits).
+//
 // Up to 128 rows the tiles of a last, partly filled wave are split along K (fp32 partial tiles, added in split order by
 // k_w4a16_reduce) as long as that fills the idle SMs; a problem with fewer tiles than SMs is all tail. From 129 rows on nothing is
 // split: every element is one sum in ascending k, whatever tile and batch its row sits in.
