@@ -155,8 +155,8 @@ int b200moe_gemm_nvfp4(const void* a_q, const void* a_sf_tiled, const void* b_q,
  * the result differs from the fp32 reference only by the order of the fp32 additions.
  * workspace (optional, 16-byte aligned device memory of at least b200moe_gemm_bf16_nvfp4_workspace_bytes(m, n, k) bytes;
  * that function returns 0 when none is useful): above 128 rows it holds the weights expanded to bf16 (N * K * 2 bytes, never more
- * than 256 MB), written and read by every call, for a plain bf16 GEMM; without it the weights are decoded tile by tile, to the same
- * bits. For M <= 128 it lets several CTAs share the reduction of an output tile of
+ * than 256 MB), written and read by every call, for a plain bf16 GEMM, if it starts on a 32-byte boundary; without it, or on a 16-byte
+ * boundary only, the weights are decoded tile by tile, to the same bits. For M <= 128 it lets several CTAs share the reduction of an output tile of
  * the last, partly filled wave (fp32 partial sums added in a fixed order: results stay reproducible). Without it every tile
  * is reduced by one CTA, which leaves most of the device idle when there are few tiles. Up to 16 rows need none.
  * A row's result depends on the row, B, alpha and on whether there is a workspace, not on M, among batches of 1..16,

@@ -428,7 +428,7 @@ int launch_gemm_w4a16(const void* a, int64_t a_stride, const void* b_q, const vo
                       int64_t k, void* out, int64_t out_stride, void* workspace, int64_t workspace_bytes, int32_t* status,
                       cudaStream_t st) {
   if (m == 0) return 0;
-  if (workspace && w4a16_expand_wins(m, n, k) && workspace_bytes >= n * k * 2)
+  if (w4a16_expand_room(workspace, workspace_bytes, n, k) && w4a16_expand_wins(m, n, k))
     return launch_gemm_w4a16_expand(a, a_stride, b_q, b_sf, alpha, m, n, k, out, out_stride, workspace, status, st);
   const int sms = sm_count();
   W4A16Plan pl = w4a16_plan(m, n, k, sms, true);

@@ -171,6 +171,11 @@ int launch_gemm_w4a16_decode(const void* a, int64_t a_stride, const void* b_q, c
 // Many tokens (gemm_w4a16_expand.cu): the weights expanded to bf16 once, in a scratch of n * k * 2 bytes, then a bf16 GEMM.
 constexpr int64_t kW4A16ExpandMax = 1ll << 28;
 bool w4a16_expand_wins(int64_t m, int64_t n, int64_t k);
+// A workspace that can hold them. The expansion stores 32 bytes at a time; callers may hand in memory on a 16-byte boundary only, and
+// such a call takes the tile kernel (same bits).
+inline bool w4a16_expand_room(const void* workspace, int64_t workspace_bytes, int64_t n, int64_t k) {
+  return workspace && ((uintptr_t)workspace & 31) == 0 && workspace_bytes >= n * k * 2;
+}
 int launch_gemm_w4a16_expand(const void* a, int64_t a_stride, const void* b_q, const void* b_sf, const float* alpha, int64_t m,
                              int64_t n, int64_t k, void* out, int64_t out_stride, void* scratch, int32_t* status, cudaStream_t st);
 int64_t gemm_w4a16_workspace_bytes(int64_t m, int64_t n, int64_t k);

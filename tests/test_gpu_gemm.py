@@ -357,6 +357,33 @@ def test_w4a16_expanded_weights(m, n, k):
     assert ((y[0][rows].double() - exact).abs() <= exact.abs() * 2.0 ** -8 + mag * (k * 2.0 ** -24)).all()
 
 
+@pytest.mark.parametrize("offset", [0, 16, 32, 48])
+def test_w4a16_workspace_of_a_c_caller(offset):
+    """Above 128 rows the C entry takes a workspace on any 16-byte boundary. On a 32-byte boundary the weights are expanded into its
+    n * k * 2 bytes and nothing behind them is written; on a 16-byte boundary only it is left alone. Same bits."""
+    import kernelschema_b200 as ks
+    from kernelschema_b200 import _lib
+    m, n, k = 200, 1152, 4096
+    lib = _lib.load()
+    need = lib.b200moe_gemm_bf16_nvfp4_workspace_bytes(m, n, k)
+    assert need == n * k * 2
+    gen = torch.Generator(device="cuda").manual_seed(offset)
+    a = torch.randn(m, k, device="cuda", generator=gen).to(torch.bfloat16)
+    bq = torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device="cuda", generator=gen)
+    sf = torch.randint(0, 127, (n, k // 16), dtype=torch.uint8, device="cuda", generator=gen)
+    want = ks.mm_bf16_nvfp4(a, bq, sf, split_k=False)
+    ws = torch.full((need + 64,), 0xA5, dtype=torch.uint8, device="cuda")
+    assert ws.data_ptr() % 64 == 0
+    out = torch.empty_like(want)
+    stream = torch.cuda.current_stream().cuda_stream
+    rc = lib.b200moe_gemm_bf16_nvfp4(a.data_ptr(), k, bq.data_ptr(), sf.data_ptr(), None, out.data_ptr(), m, n, k, n,
+                                     ws.data_ptr() + offset, need, None, stream)
+    assert rc == 0 and torch.equal(out, want)
+    written = ws != 0xA5
+    assert not written[:offset].any() and not written[offset + need:].any()
+    assert written.any() == (offset % 32 == 0)
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 256, 512), (130, 512, 2304), (128, 18944, 512), (128, 19200, 512), (4736, 512, 768), (4737, 512, 768)])
 def test_dense_gemm_default_tile_width(m, n, k):
     """tile_n = 0 on both sides of the line where the 128-wide tiles stop running at once (148 of them): the bits of either explicit width."""

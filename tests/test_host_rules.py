@@ -42,6 +42,18 @@ def test_selection_inside_the_route_map_owns_at_most_one_warp_of_routes(tmp_path
     assert int(widest) == 32 and int(full) == 1
 
 
+def test_expanded_weights_need_a_workspace_on_a_32_byte_boundary(tmp_path):
+    """The entry accepts a workspace on any 16-byte boundary; the expansion stores 32 bytes at a time and takes only one on a 32-byte
+    boundary that holds all weights."""
+    assert _run(tmp_path, """
+  const int64_t n = 128, k = 1280;
+  for (uintptr_t at = 1 << 20; at < (1 << 20) + 512; at += 16)
+    for (int64_t bytes : {(int64_t)-1, (int64_t)0, n * k * 2 - 1, n * k * 2, n * k * 2 + 1})
+      if (w4a16_expand_room((const void*)at, bytes, n, k) != (at % 32 == 0 && bytes >= n * k * 2)) return 1;
+  printf("%d", (int)w4a16_expand_room(nullptr, n * k * 2, n, k));
+  return 0;""") == ["0"]
+
+
 def test_split_k_scratch_of_many_threads(monkeypatch):
     """Threads that use more streams than a thread keeps scratch for: every call gets a buffer that no other thread holds, nothing
     raises while buffers are replaced, and each thread keeps at most eight."""
