@@ -614,7 +614,6 @@ k_gemm_nvfp4_pair(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
           if (++s == C::kStages) { s = 0; ph ^= 1; }
         }
       }
-      pdl_trigger();
     }
   } else if (warp >= 2 && warp < kPairEpiWarp) {
     // ------------------------------------------------------------------ scale-factor copiers (leader; every copy acts on both CTAs)
@@ -763,7 +762,7 @@ static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
   auto kern = k_gemm_nvfp4_pair<MODE>;
   static SmemOptIn opt_in;
   if (int e = opt_in.ensure(kern, PairCfg::kSmemBytes)) return e;
-  return (int)launch_chain(kern, dim3(grid), dim3(kPairThreads), PairCfg::kSmemBytes, st, ta, tb, tsa, tsb, p);
+  return (int)launch_clusters(kern, dim3(grid), dim3(kPairThreads), dim3(2), PairCfg::kSmemBytes, st, ta, tb, tsa, tsb, p);
 }
 
 // grid = 2 CTAs per work-item stream, at most one pair per two SMs

@@ -82,7 +82,7 @@ k_gemm_w4a16_decode(const __nv_bfloat16* __restrict__ a, int64_t a_stride, const
   const int64_t row0 = (int64_t)((int)blockIdx.x / split) * kDecRows;
   const int units = K / kDecUnit;
   uint4* xs = dec_smem + warp * (NT * 8 * kDecUnit * 2 / 16);  // [NT][4 words of a lane][8 tokens x 4 lanes] 16-byte pieces
-  pdl_trigger();
+  if (split == 1) pdl_trigger();                               // never from a cluster (launch_clusters)
   pdl_wait();
 
   float acc[4][NT][4];
@@ -216,22 +216,14 @@ int launch_nt(const void* a, int64_t a_stride, const void* b_q, const void* b_sf
   const int split = dec_split(n, k, dec_blocks_per_sm<NT>());
   static SmemOptIn opt_in;
   if (int e = opt_in.ensure(k_gemm_w4a16_decode<NT>, dec_smem_bytes<NT>())) return e;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(n / kDecRows * split));
-  cfg.blockDim = dim3(32 * kDecWarps);
-  cfg.dynamicSmemBytes = dec_smem_bytes<NT>();
-  cfg.stream = st;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = (unsigned)split;
-  attr[1].val.clusterDim.y = 1;
-  attr[1].val.clusterDim.z = 1;
-  cfg.attrs = pdl_enabled() ? attr : attr + 1;
-  cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  return (int)cudaLaunchKernelEx(&cfg, k_gemm_w4a16_decode<NT>, (const __nv_bfloat16*)a, a_stride, (const uint8_t*)b_q,
-                                 (const uint8_t*)b_sf, alpha, (__nv_bfloat16*)out, out_stride, (int)m, (int)k, split);
+  const dim3 grid((unsigned)(n / kDecRows * split)), block(32 * kDecWarps);
+  const auto *x = (const __nv_bfloat16*)a;
+  const auto *q = (const uint8_t*)b_q, *sf = (const uint8_t*)b_sf;
+  auto *y = (__nv_bfloat16*)out;
+  if (split == 1)
+    return (int)launch_chain(k_gemm_w4a16_decode<NT>, grid, block, dec_smem_bytes<NT>(), st, x, a_stride, q, sf, alpha, y, out_stride, (int)m, (int)k, 1);
+  return (int)launch_clusters(k_gemm_w4a16_decode<NT>, grid, block, dim3((unsigned)split), dec_smem_bytes<NT>(), st, x, a_stride, q, sf, alpha, y,
+                              out_stride, (int)m, (int)k, split);
 }
 
 }  // namespace

@@ -9,8 +9,12 @@
 // k_gemm_bf16_pair: a cluster of two CTAs drives tcgen05.mma.cta_group::2 on 256 x 256 tiles, so each SM fetches 128 rows of A and
 // 128 of B per 64-wide k-step (32 KB for 512 tensor cycles). Seven stages; two 256-column accumulators fill TMEM, so a tile's
 // epilogue runs beside the next tile's k-loop.
-// Both launches are in plain stream order, not programmatic: overlapped, the waiting blocks of an expansion of several waves and the
-// clusters of the GEMM before it stopped one another from being scheduled.
+// Both launches are in plain stream order, not programmatic. A programmatic form of the two, ten calls of 129 x 4096 x 12288 back to back,
+// did not finish, and no bounded wait expired in it. The cause was not found. By the rule that a dependent grid starts only when every
+// block before it has triggered or ended, no block can have been kept out. If that rule failed for clusters, then only through blocks
+// of the NEXT expansion, let in by the GEMM's trigger and waiting on the SMs (several waves of them) while clusters still looked
+// for room: that GEMM has 64 blocks, so waiting clusters of its own left 84 SMs to the expansion before it.
+// Here nothing is let in early, and no cluster kernel of the library triggers (launch_clusters in kernels.cuh).
 // Additions per element run in ascending k like the tile kernel's: same bits.
 #include "kernels.cuh"
 #include "ptx.cuh"

@@ -53,6 +53,29 @@ inline cudaError_t launch_chain(void (*kern)(KArgs...), dim3 grid, dim3 block, s
   return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
+// The same for a kernel that runs as clusters of more than one block. Such a kernel never calls pdl_trigger: what follows it is released by
+// its end alone, so blocks of a next launch that wait on the SMs and clusters that still look for room cannot meet. (A cluster kernel
+// and a launch of several waves, both programmatic, once did not finish when called back to back: see gemm_w4a16_expand.cu.)
+// A trigger gave nothing: W4A16 of 16 x 4096 x 12288 17.2 us a call with it, 16.8 without; without the attribute 18.4.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_clusters(void (*kern)(KArgs...), dim3 grid, dim3 block, dim3 cluster, size_t smem, cudaStream_t st, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cluster.x;
+  attr[0].val.clusterDim.y = cluster.y;
+  attr[0].val.clusterDim.z = cluster.z;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+
 // Device buffers produced by the route-map build.
 struct RouteMapBuffers {
   int32_t* block_hist;     // [nblk, E'] scratch

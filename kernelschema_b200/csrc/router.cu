@@ -343,7 +343,7 @@ k_router_logits_ksplit(const __grid_constant__ CUtensorMap tm_x, const __grid_co
   tc_fence_after();
   uint32_t tmem;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(s_slot));
-  pdl_trigger();
+  if (k_split == 1) pdl_trigger();                // never from a cluster (launch_clusters)
   pdl_wait();
   const int steps = (H >> 6) / k_split, ks0 = (int)rank * steps;
   const uint32_t stage_bytes = kLkABytes + (uint32_t)e_slice * 128;
@@ -448,21 +448,10 @@ int launch_router_logits_ksplit(const void* x, const void* w, int64_t T, int H, 
   if (rc) return rc;
   static SmemOptIn opt_in;
   if (int e = opt_in.ensure(k_router_logits_ksplit, kLkSmem)) return e;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((T + 127) / 128), (unsigned)(e_pad / e_slice), (unsigned)k_split);
-  cfg.blockDim = dim3(192);
-  cfg.dynamicSmemBytes = kLkSmem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 1;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = (unsigned)k_split;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  return (int)cudaLaunchKernelEx(&cfg, k_router_logits_ksplit, tx, tw, (int)T, H, E, e_slice, logits, status);
+  const dim3 grid((unsigned)((T + 127) / 128), (unsigned)(e_pad / e_slice), (unsigned)k_split);
+  if (k_split == 1) return (int)launch_chain(k_router_logits_ksplit, grid, dim3(192), kLkSmem, st, tx, tw, (int)T, H, E, e_slice, logits, status);
+  return (int)launch_clusters(k_router_logits_ksplit, grid, dim3(192), dim3(1, 1, (unsigned)k_split), kLkSmem, st, tx, tw, (int)T, H, E, e_slice,
+                              logits, status);
 }
 
 int launch_route_topk(const float* logits, const float* bias, int64_t T, int E, int K, int32_t* ids, float* weights,

@@ -384,6 +384,26 @@ def test_w4a16_workspace_of_a_c_caller(offset):
     assert written.any() == (offset % 32 == 0)
 
 
+def test_cluster_kernels_between_launches_of_several_waves():
+    """Quantiser launches of several waves of blocks before and behind every kernel that runs as clusters, ten rounds without a
+    synchronize in between: the outputs of the calls one by one."""
+    import kernelschema_b200 as ks
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    x = torch.randn((8192, 4096), device="cuda", generator=gen).to(torch.bfloat16)
+    w, w_sf = ks.nvfp4_quantize(x[:4096], 1.0)
+    w_sft, w_sf = ks.scales_to_tiles(w_sf), w_sf.view(torch.uint8)
+    calls = (lambda: ks.nvfp4_quantize(x, 0.5)[0], lambda: ks.mm_bf16_nvfp4(x[:16], w, w_sf), lambda: ks.nvfp4_quantize(x, 0.25)[0],
+             lambda: ks.router_logits(x[:256], x[:128]), lambda: ks.nvfp4_quantize(x, 0.125)[0],
+             lambda: ks.mm_nvfp4(w[:512], w_sft[:4], w, w_sft, tile_n=512), lambda: ks.mm_bf16_nvfp4(x[:129], w, w_sf))
+    want = []
+    for call in calls:
+        want.append(call())
+        torch.cuda.synchronize()
+    got = [[call() for call in calls] for _ in range(10)]
+    torch.cuda.synchronize()
+    assert all(torch.equal(g, v) for row in got for g, v in zip(row, want))
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 256, 512), (130, 512, 2304), (128, 18944, 512), (128, 19200, 512), (4736, 512, 768), (4737, 512, 768)])
 def test_dense_gemm_default_tile_width(m, n, k):
     """tile_n = 0 on both sides of the line where the 128-wide tiles stop running at once (148 of them): the bits of either explicit width."""

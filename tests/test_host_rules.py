@@ -1,5 +1,6 @@
 """CPU-only checks of the host rules that size launches: a small program includes the launch header and walks every form a rule accepts."""
 import os
+import re
 import subprocess
 import sys
 import threading
@@ -40,6 +41,24 @@ def test_selection_inside_the_route_map_owns_at_most_one_warp_of_routes(tmp_path
   printf("%d %d", widest, full);
   return 0;""")
     assert int(widest) == 32 and int(full) == 1
+
+
+def test_no_cluster_kernel_lets_the_next_launch_in_early():
+    """A kernel that runs as clusters releases its dependents by its end alone: it has no pdl_trigger, or only where it runs without
+    a cluster. (Blocks of a next launch that wait on the SMs while clusters look for room are what this rules out.)"""
+    csrc, seen = os.path.join(ROOT, "kernelschema_b200", "csrc"), set()
+    for name in sorted(os.listdir(csrc)):
+        if not name.endswith(".cu"):
+            continue
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, name)).read())
+        for kernel in re.split(r"\b__global__\b", text)[1:]:
+            body = kernel[:kernel.index("\n}\n")]
+            if "cluster" not in body:
+                continue
+            seen.add(re.search(r"\b(k_\w+)\s*\(", body).group(1))
+            for line in re.findall(r"[^\n]*pdl_trigger\(\);", body):
+                assert re.match(r"\s*if \((k_)?split == 1\) pdl_trigger\(\);", line), (name, line)
+    assert seen == {"k_gemm_nvfp4_pair", "k_gemm_bf16_pair", "k_gemm_w4a16_decode", "k_router_logits_ksplit"}
 
 
 def test_expanded_weights_need_a_workspace_on_a_32_byte_boundary(tmp_path):
