@@ -344,12 +344,16 @@ DEV void gather_row(const GatherView& g, int tok, int pos, int lane) {
 }
 
 // Four rows of at most 2048 elements at a time (two vectors and one scale word a lane each), every load in flight before the first
-// store. Row i of the block's n is route lo + i; the warp takes rows i0, i0 + step, ..
-DEV void load_rows(const GatherView& g, int lo, int n, int kk, int i0, int step, int lane, uint4 (&t)[8], uint32_t (&sw)[4]) {
+// store. Row i of the block's n is route lo + i; the warp takes rows i0, i0 + step, .. A route without a position (masked, a slot without a
+// token, an expert of another rank) is neither read nor written: pos is -1, the same in the whole warp.
+DEV void load_rows(const GatherView& g, const int* s_pos, int lo, int n, int kk, int i0, int step, int lane, int (&pos)[4], uint4 (&t)[8],
+                   uint32_t (&sw)[4]) {
   const int vecs = g.a_q ? g.H >> 5 : 0, words = g.H >> 6;
 #pragma unroll
+  for (int j = 0; j < 4; ++j) pos[j] = i0 + j * step < n ? s_pos[i0 + j * step] : -1;
+#pragma unroll
   for (int j = 0; j < 4; ++j) {
-    if (i0 + j * step >= n) continue;
+    if (pos[j] < 0) continue;
     const int tok = (lo + i0 + j * step) / kk;
     const uint4* src = reinterpret_cast<const uint4*>(g.hid_q + (size_t)tok * g.q_stride) + lane;
     const uint32_t* sf_src = reinterpret_cast<const uint32_t*>(g.hid_sf + (size_t)tok * g.sf_stride) + lane;
@@ -359,15 +363,14 @@ DEV void load_rows(const GatherView& g, int lo, int n, int kk, int i0, int step,
       if (lane + 32 * i < vecs) t[2 * j + i] = __ldg(src + 32 * i);
   }
 }
-DEV void store_rows(const GatherView& g, const int* s_pos, int n, int i0, int step, int lane, const uint4 (&t)[8], const uint32_t (&sw)[4]) {
+DEV void store_rows(const GatherView& g, int lane, const int (&pos)[4], const uint4 (&t)[8], const uint32_t (&sw)[4]) {
   const int vecs = g.a_q ? g.H >> 5 : 0, words = g.H >> 6;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    const int pos = i0 + j * step < n ? s_pos[i0 + j * step] : -1;
-    if (pos < 0) continue;
-    uint4* dst = reinterpret_cast<uint4*>(g.a_q + (size_t)pos * (g.H >> 1)) + lane;
-    uint32_t* sf_dst = reinterpret_cast<uint32_t*>(g.a_sf + (size_t)(pos >> 7) * words * 512 + (size_t)(pos & 31) * 16 +
-                                                   (size_t)((pos >> 5) & 3) * 4);
+    if (pos[j] < 0) continue;
+    uint4* dst = reinterpret_cast<uint4*>(g.a_q + (size_t)pos[j] * (g.H >> 1)) + lane;
+    uint32_t* sf_dst = reinterpret_cast<uint32_t*>(g.a_sf + (size_t)(pos[j] >> 7) * words * 512 + (size_t)(pos[j] & 31) * 16 +
+                                                   (size_t)((pos[j] >> 5) & 3) * 4);
 #pragma unroll
     for (int i = 0; i < 2; ++i)
       if (lane + 32 * i < vecs) dst[32 * i] = t[2 * j + i];
@@ -585,9 +588,9 @@ __global__ void __launch_bounds__(TOPK ? kTopkGatherThreads : kRouteThreads) k_r
   const auto count = [&](int f, int e) {
     if (e >= 0 && (f < lo || f >= hi)) atomicAdd((f < lo ? before : after) + e, 1);
   };
-  // Four ids a load once a block owns more than 32 routes (from 4 737 on with 148 SMs): 14 216 routes, 1 777 tokens of H = 2048, layer call
-  // 106.6 -> 103.7 us together with the four rows at a time below. Fewer routes are counted in a round trip or two either way, and
-  // the longer code alone costs them 0.4 to 1 us.
+  // Four ids a load once a block owns more than 32 routes (from 4 737 on with 148 SMs). Layer calls with every route local, without / with
+  // them (four rows at a time below in both): 14 216 routes, H = 2048, 105.1 / 103.5 us; 8192 routes 90.7 / 89.6; 16 376 routes, H = 1024,
+  // 56.7 / 55.4. Fewer routes are counted in a round trip or two either way, and the longer code alone costs them 0.4 to 1 us.
   int scalar0 = 0;                                 // the ids from here on are counted one by one
   if (OW > 1 && flat && (reinterpret_cast<uintptr_t>(r.ids) & 15) == 0) {
     const auto local = [&](int id) { const int e = id - r.expert_offset; return e < r.E ? e : -1; };
@@ -634,12 +637,15 @@ __global__ void __launch_bounds__(TOPK ? kTopkGatherThreads : kRouteThreads) k_r
   }
   __syncthreads();
   const int n_own = hi - lo, warps = (int)(blockDim.x >> 5);
-  if (OW > 1 && gv.H <= 2048) {                    // several short rows a warp
+  // Several short rows a warp (14 216 routes, H = 2048, layer call 104.1 us one by one, 103.5 four at a time; 5600 routes 85.4 and 84.7). With
+  // an eighth of the routes local both forms take 30 us.
+  if (OW > 1 && gv.H <= 2048) {
     for (int i = warp; i < n_own; i += 4 * warps) {
+      int row_pos[4];
       uint4 row_t[8];
       uint32_t row_sw[4];
-      load_rows(gv, lo, n_own, kk, i, warps, lane, row_t, row_sw);
-      store_rows(gv, s_pos, n_own, i, warps, lane, row_t, row_sw);
+      load_rows(gv, s_pos, lo, n_own, kk, i, warps, lane, row_pos, row_t, row_sw);
+      store_rows(gv, lane, row_pos, row_t, row_sw);
     }
     return;
   }

@@ -138,3 +138,24 @@ def test_many_routes_counted_four_at_a_time(tokens, top_k, hidden, shift):
     got, _, model = run_model(p, ks.Model(), shift_ids=shift)
     _check_map_and_rows(p, model)
     assert_layer_parity(got, o.moe_expected(p), f"T={tokens} H={hidden} shift={shift}")
+
+
+@pytest.mark.parametrize("tokens,hidden,offset", [(1601, 512, 0), (1601, 512, 12), (2047, 2048, 4)])
+def test_many_routes_of_which_few_are_local(tokens, hidden, offset):
+    """A rank that owns four of sixteen experts, and masked routes: most of the routes that a block copies four at a time have no position.
+    Tokens without a local route hold a payload of the largest code and NaN scales."""
+    from gpu_util import run_model
+    full = make_moe_case(700 + offset, tokens, hidden, 256, 16, 3, routing="zipf", masked=True)
+    p = dict(full)
+    for name in ("gemm1_weights", "gemm1_weights_scale", "gemm2_weights", "gemm2_weights_scale", "gemm1_alpha", "gemm1_beta"):
+        p[name] = full[name][offset:offset + 4]
+    p["num_experts"], p["local_expert_offset"] = 4, offset
+    ids = full["topk_ids"][0]
+    foreign = ~((ids >= offset) & (ids < offset + 4)).any(axis=1)
+    assert foreign.any()
+    want = o.moe_expected(p)
+    p["hidden_states"], p["hidden_states_scale"] = full["hidden_states"].copy(), full["hidden_states_scale"].copy()
+    p["hidden_states"][foreign], p["hidden_states_scale"].view(np.uint8)[foreign] = 0x77, 0x7F
+    got, _, _ = run_model(p)
+    assert_layer_parity(got, want, f"offset {offset}")
+    assert not got[foreign].any()
