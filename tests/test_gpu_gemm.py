@@ -1,4 +1,6 @@
 """GPU parity of the tcgen05 NVFP4 GEMM (dense entry point) against the oracle's dequantise-then-matmul."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -382,6 +384,82 @@ def test_w4a16_workspace_of_a_c_caller(offset):
     written = ws != 0xA5
     assert not written[:offset].any() and not written[offset + need:].any()
     assert written.any() == (offset % 32 == 0)
+
+
+def _weights(gen, n, k):
+    import kernelschema_b200 as ks
+    q, s = ks.nvfp4_quantize((torch.randn(n, k, device="cuda", generator=gen) * k ** -0.5).to(torch.bfloat16), 1.0)
+    return q, s.view(torch.uint8)
+
+
+def test_w4a16_many_rows_on_two_streams_and_in_a_graph(monkeypatch):
+    """Above 128 rows: calls on two streams keep apart while each takes and returns its scratch; a captured call still gives its result
+    after the memory around it has been used by others; without scratch the result is the same."""
+    import kernelschema_b200 as ks
+    from kernelschema_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    m, n, k = 300, 2048, 4096
+    a = [torch.randn(m, k, device="cuda", generator=gen).to(torch.bfloat16) for _ in range(2)]
+    w = [_weights(gen, n, k) for _ in range(2)]
+    want = [ks.mm_bf16_nvfp4(a[i], *w[i], split_k=False) for i in range(2)]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    outs = [[torch.empty_like(want[0]) for _ in range(20)] for _ in range(2)]
+    torch.cuda.synchronize()
+    for r in range(20):
+        for i, st in enumerate(streams):
+            with torch.cuda.stream(st):
+                ks.mm_bf16_nvfp4(a[i], *w[i], out=outs[i][r])
+    torch.cuda.synchronize()
+    assert all(torch.equal(outs[i][r], want[i]) for i in range(2) for r in range(20))
+
+    out = [torch.empty_like(v) for v in want]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        held = ops._w4a16_expanded(a[0].device, 4096)
+        assert held is not None                     # in a graph of torch's the expanded weights have a place
+        for i in range(2):
+            ks.mm_bf16_nvfp4(a[i], *w[i], out=out[i])
+    others = [torch.full((n * k * 2,), 0x5A, dtype=torch.uint8, device="cuda") for _ in range(4)]
+    for _ in range(3):
+        out[0].zero_(), out[1].zero_()
+        ks.mm_bf16_nvfp4(torch.cat(a), *w[0])
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out[0], want[0]) and torch.equal(out[1], want[1])
+    assert all((v == 0x5A).all() for v in others)
+
+    monkeypatch.setattr(ops, "_w4a16_expanded", lambda device, need: None)
+    assert torch.equal(ks.mm_bf16_nvfp4(a[0], *w[0]), want[0])
+
+
+@pytest.mark.parametrize("m", [60, 300])
+def test_w4a16_in_a_capture_that_torch_did_not_begin(m):
+    """The allocator has no pool for such a graph, so the call must not keep scratch of the allocator's in it: what is allocated after the
+    capture stays as it is when the graph is replayed, and the outputs are those of a call without scratch."""
+    import kernelschema_b200 as ks
+    rt = C.CDLL("libcudart.so.12")                  # torch's, loaded already
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    n, k = 2048, 4096
+    a, w = torch.randn(m, k, device="cuda", generator=gen).to(torch.bfloat16), _weights(gen, n, k)
+    want = ks.mm_bf16_nvfp4(a, *w, split_k=m <= 128)
+    out, st = torch.zeros_like(want), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(st):
+        graph, exe = C.c_void_p(), C.c_void_p()
+        assert rt.cudaStreamBeginCapture(C.c_void_p(st.cuda_stream), 0) == 0
+        try:
+            ks.mm_bf16_nvfp4(a, *w, out=out)
+        finally:
+            rc = rt.cudaStreamEndCapture(C.c_void_p(st.cuda_stream), C.byref(graph))
+        assert rc == 0 and rt.cudaGraphInstantiateWithFlags(C.byref(exe), graph, C.c_ulonglong(0)) == 0
+        others = [torch.full((n * k * 2,), 0x5A, dtype=torch.uint8, device="cuda") for _ in range(4)]
+        for _ in range(3):
+            assert rt.cudaGraphLaunch(exe, C.c_void_p(st.cuda_stream)) == 0
+        st.synchronize()
+        assert all((v == 0x5A).all() for v in others)
+    scale = want.float().pow(2).mean().sqrt()       # up to 128 rows the sums run in another order without scratch
+    assert torch.equal(out, want) if m > 128 else (out.float() - want.float()).abs().max() <= scale * 2.0 ** -5
+    assert rt.cudaGraphExecDestroy(exe) == 0 and rt.cudaGraphDestroy(graph) == 0
 
 
 def test_cluster_kernels_between_launches_of_several_waves():

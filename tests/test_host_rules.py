@@ -105,3 +105,25 @@ def test_split_k_scratch_of_many_threads(monkeypatch):
         sys.setswitchinterval(interval)
     assert not errors, errors
     assert max(kept) <= 8 and len(set().union(*held)) == sum(kept)
+
+
+def test_w4a16_scratch_of_a_captured_call_lies_in_a_graph_pool(monkeypatch):
+    """On a stream that is being captured a call keeps scratch only of a graph's pool; in ordinary memory (a capture that torch did not
+    begin), under an allocator that does not tell, and where there is no memory, many rows run without."""
+    import torch
+    from kernelschema_b200 import ops
+    pool = []
+    monkeypatch.setattr(torch.cuda, "memory_snapshot", lambda: [dict(address=0, total_size=1 << 62, **p) for p in pool])
+    dev = torch.device("cpu")
+    for capturing, pool[:], kept in ((False, [], True), (True, [dict(segment_pool_id=(1, 0))], True), (True, [dict(segment_pool_id=(0, 3))], True),
+                                     (True, [dict(segment_pool_id=(0, 0))], False), (True, [dict()], False), (True, [], False)):
+        monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: capturing)
+        for ws in (ops._w4a16_expanded(dev, 4096), ops._w4a16_workspace(dev, 7, 4096)):
+            assert (ws is not None) == kept and (ws is None or ws.numel() >= 4096)
+
+    def no_memory(*args, **kwargs):
+        raise torch.OutOfMemoryError("none left")
+
+    monkeypatch.setattr(torch, "empty", no_memory)
+    for capturing in (False, True):
+        assert ops._w4a16_expanded(dev, 4096) is None
