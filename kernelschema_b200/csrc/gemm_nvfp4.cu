@@ -493,7 +493,7 @@ k_gemm_nvfp4(const __grid_constant__ ActMaps am, const __grid_constant__ CUtenso
       if (more) fetch(item + gridDim.x);
       const uint32_t buf = it % C::kAccBufs;
       int okw = 1;
-      if (lane == 0) okw = mbar_wait(bar_acc_full + 8 * buf, (it / C::kAccBufs) & 1) ? 1 : 0;
+      if (lane == 0) okw = mbar_wait(bar_acc_full + 8 * buf, (it / C::kAccBufs) & 1, nk) ? 1 : 0;
       okw = __shfl_sync(0xFFFFFFFFu, okw, 0);
       if (!okw) { if (lane == 0) report(p.status, 104); break; }
       tc_fence_after();
@@ -690,7 +690,7 @@ k_gemm_nvfp4_pair(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       const int rows = min(128, max(0, pair_rows - (int)rank * 128));
       const EpiScale sc = load_scales<MODE>(p, e);
       int okw = 1;
-      if (lane == 0) okw = mbar_wait_cluster(bar_acc_full, it & 1) ? 1 : 0;
+      if (lane == 0) okw = mbar_wait_cluster(bar_acc_full, it & 1, nk) ? 1 : 0;
       okw = __shfl_sync(0xFFFFFFFFu, okw, 0);
       if (!okw) { if (lane == 0) report(p.status, 204); break; }
       tc_fence_after();

@@ -331,7 +331,7 @@ k_gemm_w4a16(const __grid_constant__ CUtensorMap tm_a, const W4A16Params p) {
       const int mt = at.tile / n_nt, nt = at.tile - mt * n_nt;
       const uint32_t buf = it % C::kAccBufs;
       int okw = 1;
-      if (lane == 0) okw = mbar_wait(bar_acc_full + 8 * buf, (it / C::kAccBufs) & 1) ? 1 : 0;
+      if (lane == 0) okw = mbar_wait(bar_acc_full + 8 * buf, (it / C::kAccBufs) & 1, 4 * (at.g1 - at.g0)) ? 1 : 0;
       okw = __shfl_sync(0xFFFFFFFFu, okw, 0);
       if (!okw) { if (lane == 0 && p.status) atomicCAS(p.status, 0, 124); break; }
       tc_fence_after();

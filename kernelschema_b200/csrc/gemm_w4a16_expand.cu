@@ -201,7 +201,7 @@ k_gemm_bf16_pair(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       bp_tile(t, n_mt, n_nt, mt, nt);
       const uint32_t buf = it & 1;
       int okw = 1;
-      if (lane == 0) okw = mbar_wait_cluster(bar_acc_full + 8 * buf, (it >> 1) & 1) ? 1 : 0;
+      if (lane == 0) okw = mbar_wait_cluster(bar_acc_full + 8 * buf, (it >> 1) & 1, nk) ? 1 : 0;
       okw = __shfl_sync(0xFFFFFFFFu, okw, 0);
       if (!okw) { if (lane == 0 && p.status) atomicCAS(p.status, 0, 134); break; }
       tc_fence_after();

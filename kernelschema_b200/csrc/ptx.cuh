@@ -10,7 +10,9 @@
 
 namespace b200 {
 
-constexpr uint32_t kSpinLimit = 1u << 24;   // polls of try_wait before a wait is declared dead (about 4 us a poll that finds nothing: a minute)
+// Polls of try_wait before a wait is declared dead: 1.6 s (a poll that finds nothing takes 1.5 us). A wait for a whole k-loop adds four polls
+// per k-step, which takes about one microsecond; every other wait is for one step or for one tile's epilogue.
+constexpr uint32_t kSpinLimit = 1u << 20;
 
 DEV uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 // Programmatic dependent launch: `pdl_trigger` lets the next kernel of the stream start its prologue while this grid is
@@ -47,8 +49,9 @@ DEV void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 // Returns false when the phase did not complete within the poll limit.
-DEV bool mbar_wait(uint32_t bar, uint32_t parity) {
-  for (uint32_t i = 0; i < kSpinLimit; ++i) {
+DEV bool mbar_wait(uint32_t bar, uint32_t parity, int k_steps = 0) {
+  const uint32_t limit = kSpinLimit + 4u * (uint32_t)k_steps;
+  for (uint32_t i = 0; i < limit; ++i) {
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -186,8 +189,9 @@ DEV void mbar_arrive_remote(uint32_t cluster_bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
 // Wait with cluster-scope acquire (the arrivals come from the peer CTA).
-DEV bool mbar_wait_cluster(uint32_t bar, uint32_t parity) {
-  for (uint32_t i = 0; i < kSpinLimit; ++i) {
+DEV bool mbar_wait_cluster(uint32_t bar, uint32_t parity, int k_steps = 0) {
+  const uint32_t limit = kSpinLimit + 4u * (uint32_t)k_steps;
+  for (uint32_t i = 0; i < limit; ++i) {
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"

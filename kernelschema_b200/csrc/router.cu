@@ -257,7 +257,7 @@ k_router_logits_tc(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
     for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++it) {
       const uint32_t buf = it & 1;
       int okw = 1;
-      if (lane == 0) okw = mbar_wait(bar_acc_full + 8 * buf, (it >> 1) & 1) ? 1 : 0;
+      if (lane == 0) okw = mbar_wait(bar_acc_full + 8 * buf, (it >> 1) & 1, nk) ? 1 : 0;
       okw = __shfl_sync(0xFFFFFFFFu, okw, 0);
       if (!okw) { if (lane == 0 && status) atomicCAS(status, 0, 114); break; }
       tc_fence_after();
@@ -378,7 +378,7 @@ k_router_logits_ksplit(const __grid_constant__ CUtensorMap tm_x, const __grid_co
     // accumulator -> this block's partial tile in shared memory, column-major so that the 32 rows of a warp are contiguous
     const int quad = warp & 3;
     int okw = 1;
-    if (lane == 0) okw = mbar_wait(bar_acc_full, 0) ? 1 : 0;
+    if (lane == 0) okw = mbar_wait(bar_acc_full, 0, steps) ? 1 : 0;
     okw = __shfl_sync(0xFFFFFFFFu, okw, 0);
     if (!okw) {
       if (lane == 0 && status) atomicCAS(status, 0, 117);
