@@ -115,3 +115,8 @@ def test_dense_entry_refuses_bad_shapes_without_a_device(lib):
     assert lib.b200moe_gemm_bf16_nvfp4(None, 256, None, None, None, None, 8, 128, 256, 128, None, 0, None, None) == 766   # null pointers
     assert lib.b200moe_gemm_bf16_nvfp4(None, 256, None, None, None, None, 0, 128, 256, 128, None, 0, None, None) == 0     # M = 0: nothing to do
     assert lib.b200moe_gemm_bf16_nvfp4_workspace_bytes(8, 100, 256) == 0
+    # the expanded weights of more than 128 rows, up to 256 MB of them
+    assert lib.b200moe_gemm_bf16_nvfp4_workspace_bytes(129, 16384, 8192) == 1 << 28
+    assert lib.b200moe_gemm_bf16_nvfp4_workspace_bytes(129, 16384, 8448) == 0
+    assert lib.b200moe_gemm_bf16_nvfp4_workspace_bytes(4096, 16512, 8192) == 0
+    assert lib.b200moe_gemm_bf16_nvfp4_workspace_bytes(128, 16384, 8192) < 1 << 28

@@ -67,18 +67,27 @@ def test_quantize_short_rows_odd_strides_and_scale_alignment(rows, cols, pad, of
         assert not s[:offset].any() and not s[offset + n:].any()
 
 
-@pytest.mark.parametrize("rows,cols", [(1, 64), (1, 8192), (127, 192), (129, 320), (300, 4160), (9999, 64), (257, 7168)])
-def test_quantize_clears_a_ragged_last_tile(rows, cols):
-    """Without `out` the tiled scales come from dirty memory: the rows that the last tile has beyond the matrix are zero, by threads of
-    blocks with one and several rows, fewer and more of them than there are words to clear."""
+@pytest.mark.parametrize("pad", [0, 8])
+@pytest.mark.parametrize("gs", [0.0021, 1.3 * 2.0 ** -41])
+@pytest.mark.parametrize("rows,cols", [(1, 64), (1, 8192), (127, 192), (128, 192), (129, 320), (300, 4160), (9999, 64), (257, 7168)])
+def test_quantize_clears_a_ragged_last_tile(rows, cols, gs, pad):
+    """b200moe_quantize_nvfp4_tiles on scales that are all 255: the rows that the last tile has beyond the matrix are zero, by threads of
+    blocks with one and several rows, fewer and more of them than there are words to clear, with and without the corrected reciprocal
+    and the 256-bit loads (rows that start on 16- but not 32-byte boundaries), and nothing behind the last tile is written. The
+    wrapper gives the same without `out`."""
     import kernelschema_b200 as ks
-    x = torch.randn(rows, cols, generator=torch.Generator().manual_seed(rows)).to(torch.bfloat16)
-    want = o.block_scales(o.quantize(x.float().numpy(), 16, 0.0021)[1][None])[0]
-    x = x.cuda()
-    for _ in range(3):
-        dirty = torch.full((want.size,), 255, dtype=torch.uint8, device="cuda")
-        del dirty
-        assert np.array_equal(ks.nvfp4_quantize(x, 0.0021, tiled_scales=True)[1].cpu().numpy(), want)
+    from kernelschema_b200 import _lib
+    x = (torch.randn(rows, cols + pad, generator=torch.Generator().manual_seed(rows)) * (gs / 0.0021)).to(torch.bfloat16)
+    payload, scales = o.quantize(x[:, :cols].float().numpy(), 16, gs)
+    want = o.block_scales(scales[None])[0].reshape(-1)
+    x = x.cuda()[:, :cols]
+    q = torch.empty((rows, cols // 2), dtype=torch.uint8, device="cuda")
+    s = torch.full((want.size + 512,), 255, dtype=torch.uint8, device="cuda")
+    _lib.check(_lib.load().b200moe_quantize_nvfp4_tiles(x.data_ptr(), rows, cols, cols + pad, gs, q.data_ptr(), s.data_ptr(),
+                                                        torch.cuda.current_stream().cuda_stream), "b200moe_quantize_nvfp4_tiles")
+    assert np.array_equal(q.cpu().numpy(), payload)
+    assert np.array_equal(s[:want.size].cpu().numpy(), want) and (s[want.size:] == 255).all()
+    assert np.array_equal(ks.nvfp4_quantize(x, gs, tiled_scales=True)[1].cpu().numpy().reshape(-1), want)
 
 
 def _torch_quantize_true_division(x, gs):

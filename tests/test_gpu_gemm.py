@@ -336,8 +336,8 @@ def test_w4a16_split_k_small_m(m, n, k):
 def test_w4a16_expanded_weights(m, n, k):
     """Above 128 rows the weights are expanded to bf16 first: every payload byte and every finite scale code, odd rows (a last row tile of
     1, 44 and 129 rows), a half-empty 256-wide column tile, both tile widths, expansions of one and of several waves, ten calls in a
-    row. Same bits as the kernel that decodes tile by tile; that one and the product agree with 64-bit sums to one bf16 rounding
-    (2^-9 of the element) plus fp32 accumulation (k * 2^-24 of the sum of magnitudes at most)."""
+    row. Same bits as the kernel that decodes tile by tile; that one and the product agree with 64-bit sums to half a bf16 step (at most
+    2^-8 of the element, whose significand has eight bits) plus fp32 accumulation (k * 2^-24 of the sum of magnitudes at most)."""
     import kernelschema_b200 as ks
     from kernelschema_b200 import _lib
     assert _lib.load().b200moe_gemm_bf16_nvfp4_workspace_bytes(m, n, k) == n * k * 2
