@@ -56,20 +56,6 @@ struct GemmCfg {
   static constexpr int kSfCopies = 4 + 4 * (BN / 128);           // tcgen05.cp per stage
 };
 
-// Cycle accounting of the MMA thread (where it waits), compiled only into experiment builds (-DB200MOE_PROBE).
-#ifdef B200MOE_PROBE
-__device__ long long g_probe[1024 * 4];
-#define PROBE_DECL long long pr_acc = 0, pr_sf = 0, pr_c = 0; const long long pr_t0 = clock64();
-#define PROBE_T(var) const long long var = clock64();
-#define PROBE_ADD(acc, t0) acc += clock64() - (t0);
-#define PROBE_STORE if (blockIdx.x < 1024) { g_probe[blockIdx.x * 4] = clock64() - pr_t0; g_probe[blockIdx.x * 4 + 1] = pr_acc; g_probe[blockIdx.x * 4 + 2] = pr_sf; g_probe[blockIdx.x * 4 + 3] = pr_c; }
-#else
-#define PROBE_DECL
-#define PROBE_T(var)
-#define PROBE_ADD(acc, t0)
-#define PROBE_STORE
-#endif
-
 DEV void report(int32_t* status, int code) {
   if (status) atomicCAS(status, 0, code);
 }
@@ -431,15 +417,12 @@ k_gemm_nvfp4(const __grid_constant__ ActMaps am, const __grid_constant__ CUtenso
       const uint32_t sfa_lo0 = (s_sfa >> 4) & 0x3FFF, sfb_lo0 = (s_sfb >> 4) & 0x3FFF;
       uint32_t s = 0, ph = 0, it = 0;
       bool ok = true;
-      PROBE_DECL
       for (long long item = blockIdx.x; ok && item < total_items; item += gridDim.x, ++it) {
         const uint32_t buf = it % C::kAccBufs;
         const uint32_t acc = tmem + buf * BN;
         for (int ks = 0; ks < nk; ++ks) {
-          PROBE_T(pr_b)
           // the copiers waited for the stage's TMA bytes before they copied: their barrier covers the operands too
           if (!mbar_wait((kCopiers > 0 ? bar_sf : bar_full) + 8 * s, ph)) { report(p.status, 103); ok = false; break; }
-          PROBE_ADD(pr_sf, pr_b)
           tc_fence_after();
           const uint32_t sf_t = tmem + C::kSfBase + s * C::kSfCols;
           const uint32_t a_lo = a_lo0 + s * (C::kABytes >> 4), b_lo = b_lo0 + s * (C::kBBytes >> 4);
@@ -448,9 +431,7 @@ k_gemm_nvfp4(const __grid_constant__ ActMaps am, const __grid_constant__ CUtenso
             for (int j = 0; j < C::kSfCopies; ++j) sf_copy<BN>(j, sf_t, sfa_lo0 + s * (C::kSfaBytes >> 4), sfb_lo0 + s * (C::kSfbBytes >> 4));
           }
           if (ks == 0) {                               // the scale factors do not need the accumulator
-            PROBE_T(pr_a)
             if (!mbar_wait(bar_acc_empty + 8 * buf, ((it / C::kAccBufs) & 1) ^ 1)) { report(p.status, 102); ok = false; break; }
-            PROBE_ADD(pr_acc, pr_a)
             tc_fence_after();
           }
           mma_nvf4(acc, ((uint64_t)kHiOp << 32) | a_lo, ((uint64_t)kHiOp << 32) | b_lo, idesc, sf_t, sf_t + 16, ks ? 1u : 0u);
@@ -463,7 +444,6 @@ k_gemm_nvfp4(const __grid_constant__ ActMaps am, const __grid_constant__ CUtenso
         }
         if (ok) mma_commit(bar_acc_full + 8 * buf);
       }
-      PROBE_STORE
     }
   } else if (kCopiers > 0 && warp < 2 + kCopiers) {
     if (elect_one()) {
@@ -650,16 +630,11 @@ k_gemm_nvfp4_pair(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       const uint32_t a_lo0 = ((s_a >> 4) & 0x3FFF) | (1u << 16), b_lo0 = ((s_b >> 4) & 0x3FFF) | (1u << 16);
       uint32_t s = 0, ph = 0, it = 0;
       bool ok = true;
-      PROBE_DECL
       for (long long item = first; ok && item < total_items; item += stride, ++it) {
-        PROBE_T(pr_a)
         if (!mbar_wait_cluster(bar_acc_empty, (it & 1) ^ 1)) { report(p.status, 202); break; }
-        PROBE_ADD(pr_acc, pr_a)
         tc_fence_after();
         for (int ks = 0; ks < nk; ++ks) {
-          PROBE_T(pr_b)
           if (!mbar_wait(bar_sf + 8 * s, ph)) { report(p.status, 203); ok = false; break; }
-          PROBE_ADD(pr_sf, pr_b)
           tc_fence_after();
           const uint32_t sf_t = tmem + C::kSfBase + s * C::kSfCols;
           const uint32_t a_lo = a_lo0 + s * (C::kABytes >> 4), b_lo = b_lo0 + s * (C::kBBytes >> 4);
@@ -673,7 +648,6 @@ k_gemm_nvfp4_pair(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         }
         if (ok) mma_commit_pair(bar_acc_full);
       }
-      PROBE_STORE
     }
   } else {
     // ------------------------------------------------------------------ epilogue (both CTAs: own 128 rows x 256 columns)
@@ -815,11 +789,5 @@ int launch_gemm_nvfp4(int mode, int bn, const ActMaps& ta, const CUtensorMap& tb
   if (mode == kGemmFc2) return launch_mode<kGemmFc2>(bn, ta, tb, p, grid, st);
   return launch_mode<kGemmDense>(bn, ta, tb, p, grid, st);
 }
-
-#ifdef B200MOE_PROBE
-extern "C" int b200moe_probe_read(long long* host, int n) {
-  return (int)cudaMemcpyFromSymbol(host, g_probe, sizeof(long long) * n);
-}
-#endif
 
 }  // namespace b200
