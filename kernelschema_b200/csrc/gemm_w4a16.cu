@@ -397,8 +397,7 @@ static W4A16Plan w4a16_plan(int64_t m, int64_t n, int64_t k, int sms, bool room)
   // all of them run at once: half the work of a wide tile each, and no trip through the patch that a single tile per SM cannot hide
   // (129 x 4096 x 4096 63 us wide, 42 narrow; 1000 x 4096 x 4096, the last of that width, 61 and 45; 1200 rows 63 wide). Both widths
   // add in the same order.
-  const int64_t wide_tiles = (m + 255) / 256 * (n / 256);
-  pl.bn = n % 256 == 0 && (m > 128 ? wide_tiles * 2 > sms : room && n >= 4096 && k >= 8192) ? 256 : 128;
+  pl.bn = (m > 128 ? w4a16_wide_tiles(m, n, sms) : n % 256 == 0 && room && n >= 4096 && k >= 8192) ? 256 : 128;
   const int64_t tiles = (m + 255) / 256 * (n / pl.bn), groups = k / 256, tail = tiles % sms;
   int64_t s = tail ? sms / tail : 1;
   if (s > 8) s = 8;

@@ -2,9 +2,10 @@
 // contract as gemm_w4a16.cu (gemm/dense/bf16_nvfp4_gemm/problem/reference.py:10-15), in two launches.
 //
 // The tile kernel of gemm_w4a16.cu decodes a weight row again for every 256 rows of A, and its decoders share an SM's issue slots
-// and shared-memory ports with the operand traffic. From a couple of thousand rows on it is cheaper to expand the weights ONCE
-// into a bf16 scratch (k_w4a16_expand, exact: bound by its 2 written bytes a weight) and to run the product as a pure bf16
-// GEMM (k_gemm_bf16_pair, tensor-bound) that has nothing but TMA, MMAs and an overlapped epilogue in it.
+// and shared-memory ports with the operand traffic. Unless there are few rows for very many weights, or K is short, it is cheaper from 129
+// rows on (w4a16_expand_wins) to expand the weights ONCE into a bf16 scratch (k_w4a16_expand, exact: bound by its 2 written bytes a
+// weight) and to run the product as a pure bf16 GEMM (k_gemm_bf16_pair, tensor-bound) that has nothing but TMA, MMAs and an
+// overlapped epilogue in it.
 //
 // k_gemm_bf16_pair: a cluster of two CTAs drives tcgen05.mma.cta_group::2 on 256 x 256 tiles, so each SM fetches 128 rows of A and
 // 128 of B per 64-wide k-step (32 KB for 512 tensor cycles). Seven stages; two 256-column accumulators fill TMEM, so a tile's
@@ -271,17 +272,26 @@ int bp_tile_n(int64_t m, int64_t n, int pairs) {
 
 }  // namespace
 
-// Where the two launches are the faster way: nearly everywhere above 128 rows (microseconds, tile kernel / here: 256 x 4096 x 4096
-// 51 / 29, 1024 x 2048 x 8192 86 / 37, 8192 x 4096 x 12288 862 / 543). The tile kernel keeps a short K (the expansion's launch is
-// then a third of the time) while its narrow tiles run at once or there are few rows for many weights (2048 x 2048 x 1024
-// 15.1 / 16.5, 512 x 8192 x 1024 15.1 / 18.6), and up to K = 3072 few rows whose tiles fill one wave of SMs nearly whole
-// (1024 x 8192 x 1536 27.6 / 30.7, x 3072 47.7 / 49.3). Both give the same bits.
+// Where the two launches are the faster way: by the time that each way takes, in microseconds of a call among others. Both are waves of
+// tiles, a wave a few microseconds and the k-steps of 64 of one tile, a step the slower the fuller the wave; the expansion adds its
+// launches and the bytes of the weights, more for each beyond what stays in L2. Fitted to 2544 shapes (128 <= N <= 65536,
+// 256 <= K <= 28672, 129 <= M <= 8192, both ways timed): choosing by it costs 0.05 % against always taking the faster way, and where it
+// takes the expansion that is at most 9 % slower than the tile kernel. (Tile kernel / here: 256 x 4096 x 4096 43 / 25 us, 1024 x 2048 x 8192
+// 82 / 36, 8192 x 4096 x 12288 774 / 560; few rows for very many weights 129 x 16384 x 4096 44 / 62, 200 x 28672 x 2048 39 / 72; a
+// short K 2048 x 2048 x 1024 14.7 / 16.7.) With one k-group of 256 there is nothing to save. In a graph, where the two launches cost 4 us
+// less, the expansion would win from shorter loops on (2048 x 2048 x 1024 14.6 / 12.6); the rule is for separate calls. Both ways give
+// the same bits.
 bool w4a16_expand_wins(int64_t m, int64_t n, int64_t k) {
-  if (m <= 128 || n * k * 2 > kW4A16ExpandMax) return false;
-  const int64_t sms = sm_count(), narrow = (m + 255) / 256 * (n / 128);
-  const auto fills = [&](int64_t tiles) { return tiles <= sms && tiles * 10 > sms * 8; };
-  if (k <= 1024 && (narrow <= sms || n >= 8 * m)) return false;
-  return !(k <= 3072 && n >= 8 * m && (fills(narrow) || fills(narrow / 2)));
+  if (m <= 128 || k < 512 || n * k * 2 > kW4A16ExpandMax) return false;
+  const int sms = sm_count(), pairs = sms / 2;
+  const double steps = (double)(k / 64), mega = (double)(n * k) * 1e-6;
+  const bool wide = w4a16_wide_tiles(m, n, sms);
+  const int64_t tiles = (m + 255) / 256 * (n / (wide ? 256 : 128)), waves = (tiles + sms - 1) / sms;
+  const double tile_us = 2.0 + waves * (2.2 + steps * (wide ? 1.08 : 0.595 + 0.084 * tiles / (waves * sms)));
+  const int bn = bp_tile_n(m, n, pairs);
+  const int64_t pair_tiles = (m + 255) / 256 * ((n + bn - 1) / bn), pair_waves = (pair_tiles + pairs - 1) / pairs;
+  const double expand_us = 10.2 + 0.294 * mega + (mega > 20 ? 0.267 * (mega - 20) : 0);
+  return expand_us + pair_waves * (1.45 + steps * (bn == 256 ? 0.186 + 0.15 * pair_tiles / (pair_waves * pairs) : 0.141)) < tile_us;
 }
 
 int launch_gemm_w4a16_expand(const void* a, int64_t a_stride, const void* b_q, const void* b_sf, const float* alpha, int64_t m, int64_t n,

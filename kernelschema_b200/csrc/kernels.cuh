@@ -194,6 +194,8 @@ int launch_gemm_w4a16_decode(const void* a, int64_t a_stride, const void* b_q, c
 // Many tokens (gemm_w4a16_expand.cu): the weights expanded to bf16 once, in a scratch of n * k * 2 bytes, then a bf16 GEMM.
 constexpr int64_t kW4A16ExpandMax = 1ll << 28;
 bool w4a16_expand_wins(int64_t m, int64_t n, int64_t k);
+// Width of the tile kernel above 128 rows: narrow tiles while all of them run at once.
+inline bool w4a16_wide_tiles(int64_t m, int64_t n, int sms) { return n % 256 == 0 && (m + 255) / 256 * (n / 256) * 2 > sms; }
 // A workspace that can hold them. The expansion stores 32 bytes at a time; callers may hand in memory on a 16-byte boundary only, and
 // such a call takes the tile kernel (same bits).
 inline bool w4a16_expand_room(const void* workspace, int64_t workspace_bytes, int64_t n, int64_t k) {

@@ -116,7 +116,12 @@ def test_dense_entry_refuses_bad_shapes_without_a_device(lib):
     assert lib.b200moe_gemm_bf16_nvfp4(None, 256, None, None, None, None, 0, 128, 256, 128, None, 0, None, None) == 0     # M = 0: nothing to do
     assert lib.b200moe_gemm_bf16_nvfp4_workspace_bytes(8, 100, 256) == 0
     # the expanded weights of more than 128 rows, up to 256 MB of them
-    assert lib.b200moe_gemm_bf16_nvfp4_workspace_bytes(129, 16384, 8192) == 1 << 28
-    assert lib.b200moe_gemm_bf16_nvfp4_workspace_bytes(129, 16384, 8448) == 0
-    assert lib.b200moe_gemm_bf16_nvfp4_workspace_bytes(4096, 16512, 8192) == 0
-    assert lib.b200moe_gemm_bf16_nvfp4_workspace_bytes(128, 16384, 8192) < 1 << 28
+    size = lib.b200moe_gemm_bf16_nvfp4_workspace_bytes
+    assert size(2048, 16384, 8192) == 1 << 28
+    assert size(2048, 16384, 8448) == 0 and size(4096, 16512, 8192) == 0
+    assert size(128, 16384, 8192) < 1 << 28
+    # not where the tile kernel is the faster way (16 to 46 % of a call: few rows for very many weights, one k-group)
+    for m, n, k in ((129, 16384, 4096), (256, 16384, 8192), (200, 28672, 2048), (256, 65536, 2048), (4096, 4096, 256), (1400, 6144, 256)):
+        assert size(m, n, k) == 0, (m, n, k)
+    for m, n, k in ((129, 4096, 4096), (256, 4096, 4096), (1024, 2048, 8192), (8192, 4096, 12288), (8192, 1024, 3072), (768, 65536, 2048)):
+        assert size(m, n, k) == 2 * n * k, (m, n, k)
