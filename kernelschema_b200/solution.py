@@ -143,7 +143,7 @@ class DenseModel(torch.nn.Module):
     production entry ``flashinfer.mm_bf16_fp4``, problem/solution.py:11-12): same positional/keyword ``forward``; writes
     ``out`` in place and returns it. ``a`` stays bf16 (it is not quantised); ``b`` uint8 [N, K/2] with row-major E4M3
     ``b_descale`` [N, K/16]; ``alpha`` a one-element fp32 tensor or None. ``backend`` and ``enable_pdl`` are accepted and
-    ignored (there is one backend; launches always carry the programmatic-dependent-launch attribute)."""
+    ignored (there is one backend; which launches overlap by programmatic dependent launch is the library's choice)."""
 
     def forward(self, a, b, b_descale, alpha=None, *, backend=None, out_dtype=None, out=None, block_size=16, enable_pdl=True):
         from .ops import mm_bf16_nvfp4
