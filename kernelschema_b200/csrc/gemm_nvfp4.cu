@@ -27,9 +27,8 @@
 // MMA thread copies a stage's scale factors itself, in order before its MMAs: copier warps between TMA and MMA cost a barrier hop per
 // stage (8192^3 222 -> 207 us without them, 203 us with no scale copies at all; dense 1024 x 8192 x 4096 19.6 -> 16.7 us, 16384 x 7168 x
 // 2048 118.8 -> 116.6, 128-wide tiles 3000 x 3968 x 8192 53.8 -> 50.3; layer T = 1, Qwen3, 23.7 -> 22.7 us a step, T = 100, 256 experts
-// of 256 channels 158.1 -> 153.5). Layer launches of 256-wide tiles that stream weights kept two copier warps from K = 4096 on for a while;
-// over 48 layer shapes of K = 2048 to 7168, both forms timed in turn, time without / with them is 0.976 to 1.021 (K = 7168: T = 16 1.007,
-// T = 64 0.997, T = 256 0.98, T = 1024 0.99; K = 5120 and 6144 1.002 to 1.021; K = 4096 1.00 up to T = 2048, 0.976 at T = 4000).
+// of 256 channels 158.1 -> 153.5). Two copier warps remain for layer launches of 256-wide tiles with a long k-loop that stream weights
+// (copier_form).
 #include "kernels.cuh"
 #include "ptx.cuh"
 
@@ -220,11 +219,11 @@ DEV void epilogue_cols(const GemmParams& p, uint32_t taddr, const EpiScale& sc, 
   }
 }
 
-// Warp roles: 0 = TMA producer, 1 = TMEM owner + issuer of the scale copies and of the MMAs, then 4 * BN/EC epilogue warps; epilogue
-// warp w owns TMEM lane quadrant w & 3 and an EC-column group.
+// Warp roles: 0 = TMA producer, 1 = TMEM owner + issuer of the MMAs (and of the scale copies), then COP (2 or 0) scale copiers,
+// then 4 * BN/EC epilogue warps; epilogue warp w owns TMEM lane quadrant w & 3 and an EC-column group.
 // any four consecutive warps own the four TMEM lane quadrants (quadrant = warp & 3), so the epilogue groups may start anywhere
-template <int BN, int EC>
-constexpr int gemm_threads() { return 32 * (2 + 4 * BN / EC); }
+template <int BN, int EC, int COP>
+constexpr int gemm_threads() { return 32 * (2 + COP + 4 * BN / EC); }
 
 // Scale-factor copy j of a stage (j < 4: A scales of k-block j; then B scales, 128-row half h, k-block q) from the
 // stage's shared-memory slots into its TMEM buffer.
@@ -239,11 +238,33 @@ DEV void sf_copy(int j, uint32_t sf_t, uint32_t sfa_lo, uint32_t sfb_lo) {
   }
 }
 
-template <int MODE, int BN, int EC>
-__global__ void __launch_bounds__(gemm_threads<BN, EC>(), 1)
+// The scale-factor copies of copier warp C of two: every second copy of every stage.
+template <int BN, int C>
+DEV void copier_loop(const GemmParams& p, uint32_t tmem, uint32_t s_sfa, uint32_t s_sfb, uint32_t bar_full, uint32_t bar_sf,
+                     long long total_items, int nk) {
+  using Cfg = GemmCfg<BN>;
+  const uint32_t sfa_lo0 = (s_sfa >> 4) & 0x3FFF, sfb_lo0 = (s_sfb >> 4) & 0x3FFF;
+  uint32_t s = 0, ph = 0;
+  for (long long item = blockIdx.x; item < total_items; item += gridDim.x) {
+    for (int ks = 0; ks < nk; ++ks) {
+      if (!mbar_wait(bar_full + 8 * s, ph)) { report(p.status, 105); return; }
+      tc_fence_after();
+      const uint32_t sf_t = tmem + Cfg::kSfBase + s * Cfg::kSfCols;
+      const uint32_t sfa_lo = sfa_lo0 + s * (Cfg::kSfaBytes >> 4), sfb_lo = sfb_lo0 + s * (Cfg::kSfbBytes >> 4);
+#pragma unroll
+      for (int j = C; j < Cfg::kSfCopies; j += 2) sf_copy<BN>(j, sf_t, sfa_lo, sfb_lo);
+      mma_commit(bar_sf + 8 * s);                      // arrives once this thread's copies have landed
+      if (++s == Cfg::kStages) { s = 0; ph ^= 1; }
+    }
+  }
+}
+
+template <int MODE, int BN, int EC, int COP>
+__global__ void __launch_bounds__(gemm_threads<BN, EC, COP>(), 1)
 k_gemm_nvfp4(const __grid_constant__ ActMaps am, const __grid_constant__ CUtensorMap tm_b, const GemmParams p) {
   using C = GemmCfg<BN>;
   constexpr int kEpiWarps = 4 * BN / EC;
+  constexpr int kCopiers = COP;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t s_a = smem_base;
@@ -252,7 +273,8 @@ k_gemm_nvfp4(const __grid_constant__ ActMaps am, const __grid_constant__ CUtenso
   const uint32_t s_sfb = s_sfa + C::kStages * C::kSfaBytes;
   const uint32_t s_bar = s_sfb + C::kStages * C::kSfbBytes;
   const uint32_t bar_full = s_bar;                              // [kStages] TMA bytes landed
-  const uint32_t bar_empty = bar_full + 8 * C::kStages;         // [kStages] MMAs of the stage retired
+  const uint32_t bar_sf = bar_full + 8 * C::kStages;            // [kStages] the copiers' scale factors are in TMEM (kCopiers > 0)
+  const uint32_t bar_empty = bar_sf + 8 * C::kStages;           // [kStages] MMAs of the stage retired
   const uint32_t bar_acc_full = bar_empty + 8 * C::kStages;     // [kAccBufs]
   const uint32_t bar_acc_empty = bar_acc_full + 8 * C::kAccBufs;
   const uint32_t s_tmem_slot = bar_acc_empty + 8 * C::kAccBufs;
@@ -263,6 +285,7 @@ k_gemm_nvfp4(const __grid_constant__ ActMaps am, const __grid_constant__ CUtenso
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::kStages; ++s) {
       mbar_init(bar_full + 8 * s, 1);
+      if (kCopiers > 0) mbar_init(bar_sf + 8 * s, kCopiers);
       mbar_init(bar_empty + 8 * s, 1);
     }
     for (int b = 0; b < C::kAccBufs; ++b) {
@@ -398,12 +421,15 @@ k_gemm_nvfp4(const __grid_constant__ ActMaps am, const __grid_constant__ CUtenso
         const uint32_t buf = it % C::kAccBufs;
         const uint32_t acc = tmem + buf * BN;
         for (int ks = 0; ks < nk; ++ks) {
-          if (!mbar_wait(bar_full + 8 * s, ph)) { report(p.status, 103); ok = false; break; }
+          // the copiers waited for the stage's TMA bytes before they copied: their barrier covers the operands too
+          if (!mbar_wait((kCopiers > 0 ? bar_sf : bar_full) + 8 * s, ph)) { report(p.status, 103); ok = false; break; }
           tc_fence_after();
           const uint32_t sf_t = tmem + C::kSfBase + s * C::kSfCols;
           const uint32_t a_lo = a_lo0 + s * (C::kABytes >> 4), b_lo = b_lo0 + s * (C::kBBytes >> 4);
+          if constexpr (kCopiers == 0) {
 #pragma unroll
-          for (int j = 0; j < C::kSfCopies; ++j) sf_copy<BN>(j, sf_t, sfa_lo0 + s * (C::kSfaBytes >> 4), sfb_lo0 + s * (C::kSfbBytes >> 4));
+            for (int j = 0; j < C::kSfCopies; ++j) sf_copy<BN>(j, sf_t, sfa_lo0 + s * (C::kSfaBytes >> 4), sfb_lo0 + s * (C::kSfbBytes >> 4));
+          }
           if (ks == 0) {                               // the scale factors do not need the accumulator
             if (!mbar_wait(bar_acc_empty + 8 * buf, ((it / C::kAccBufs) & 1) ^ 1)) { report(p.status, 102); ok = false; break; }
             tc_fence_after();
@@ -419,10 +445,15 @@ k_gemm_nvfp4(const __grid_constant__ ActMaps am, const __grid_constant__ CUtenso
         if (ok) mma_commit(bar_acc_full + 8 * buf);
       }
     }
+  } else if (kCopiers > 0 && warp < 2 + kCopiers) {
+    if (elect_one()) {
+      if (warp == 2) copier_loop<BN, 0>(p, tmem, s_sfa, s_sfb, bar_full, bar_sf, total_items, nk);
+      else copier_loop<BN, 1>(p, tmem, s_sfa, s_sfb, bar_full, bar_sf, total_items, nk);
+    }
   } else {
     // ------------------------------------------------------------------ epilogue
     const int quad = warp & 3;
-    const int group = (warp - 2) >> 2;   // which EC accumulator columns
+    const int group = (warp - 2 - kCopiers) >> 2;   // which EC accumulator columns
     const int r_in_tile = quad * 32 + lane;
     uint32_t it = 0;
     // table entries and scales of an item are fetched while the one before it is worked on
@@ -719,12 +750,12 @@ int launch_gemm_nvfp4_pair(int mode, const CUtensorMap& ta, const CUtensorMap& t
   return launch_pair<kGemmDense>(ta, tb, tsa, tsb, p, grid, st);
 }
 
-template <int MODE, int BN, int EC>
+template <int MODE, int BN, int EC, int COP>
 static int launch_one(const ActMaps& ta, const CUtensorMap& tb, const GemmParams& p, int grid, cudaStream_t st) {
-  auto kern = k_gemm_nvfp4<MODE, BN, EC>;
+  auto kern = k_gemm_nvfp4<MODE, BN, EC, COP>;
   static SmemOptIn opt_in;
   if (int e = opt_in.ensure(kern, GemmCfg<BN>::kSmemBytes)) return e;
-  return (int)launch_chain(kern, dim3(grid), dim3(gemm_threads<BN, EC>()), GemmCfg<BN>::kSmemBytes, st, ta, tb, p);
+  return (int)launch_chain(kern, dim3(grid), dim3(gemm_threads<BN, EC, COP>()), GemmCfg<BN>::kSmemBytes, st, ta, tb, p);
 }
 
 // The form for tensor-bound launches with a long k-loop: eight epilogue warps x 128 columns (hidden by the loop, less power) and
@@ -736,11 +767,18 @@ static int launch_one(const ActMaps& ta, const CUtensorMap& tb, const GemmParams
 // and 15.8.
 static bool long_loop_form(int mode, int k, int64_t rows_hint) { return k >= 4096 && rows_hint >= (mode == kGemmDense ? 2048 : 32768); }
 
+// Copier warps beside the MMA thread, for layers with a long k-loop: the stages of a weight stream arrive in bursts and are drained
+// at the issue rate (DeepSeek-V3 T = 64, K = 7168, 412 us a step with copiers, 414.5 without).
+static bool copier_form(int k) { return k >= 4096; }
+
 template <int MODE>
 static int launch_mode(int bn, const ActMaps& ta, const CUtensorMap& tb, const GemmParams& p, int grid, cudaStream_t st) {
-  if (bn == 128) return launch_one<MODE, 128, 64>(ta, tb, p, grid, st);
+  if (bn == 128) return launch_one<MODE, 128, 64, 0>(ta, tb, p, grid, st);
   if (bn != 256) return 703;
-  return long_loop_form(MODE, p.K, p.rows_hint) ? launch_one<MODE, 256, 128>(ta, tb, p, grid, st) : launch_one<MODE, 256, 64>(ta, tb, p, grid, st);
+  if (long_loop_form(MODE, p.K, p.rows_hint)) return launch_one<MODE, 256, 128, 0>(ta, tb, p, grid, st);
+  if constexpr (MODE != kGemmDense)
+    if (copier_form(p.K)) return launch_one<MODE, 256, 64, 2>(ta, tb, p, grid, st);
+  return launch_one<MODE, 256, 64, 0>(ta, tb, p, grid, st);
 }
 
 int launch_gemm_nvfp4(int mode, int bn, const ActMaps& ta, const CUtensorMap& tb, const GemmParams& p, int grid,
