@@ -27,7 +27,7 @@
 // MMA thread copies a stage's scale factors itself, in order before its MMAs: copier warps between TMA and MMA cost a barrier hop per
 // stage (8192^3 222 -> 207 us without them, 203 us with no scale copies at all; dense 1024 x 8192 x 4096 19.6 -> 16.7 us, 16384 x 7168 x
 // 2048 118.8 -> 116.6, 128-wide tiles 3000 x 3968 x 8192 53.8 -> 50.3; layer T = 1, Qwen3, 23.7 -> 22.7 us a step, T = 100, 256 experts
-// of 256 channels 158.1 -> 153.5). Two copier warps remain for layer launches of 256-wide tiles with a long k-loop that stream weights
+// of 256 channels 158.1 -> 153.5). Two copier warps remain for layer launches of 256-wide tiles that stream weights through a long k-loop
 // (copier_form).
 #include "kernels.cuh"
 #include "ptx.cuh"
@@ -767,9 +767,11 @@ static int launch_one(const ActMaps& ta, const CUtensorMap& tb, const GemmParams
 // and 15.8.
 static bool long_loop_form(int mode, int k, int64_t rows_hint) { return k >= 4096 && rows_hint >= (mode == kGemmDense ? 2048 : 32768); }
 
-// Copier warps beside the MMA thread, for layers with a long k-loop: the stages of a weight stream arrive in bursts and are drained
-// at the issue rate (DeepSeek-V3 T = 64, K = 7168, 412 us a step with copiers, 414.5 without).
-static bool copier_form(int k) { return k >= 4096; }
+// Copier warps beside the MMA thread, for layers that stream weights through a long k-loop: their stages arrive in bursts and are drained at
+// the issue rate. DeepSeek-V3 step (FC1 K = 7168), time without / with copiers at T = 16, 32, 64, 128, 256, 512, 1024, 2048 (9 rows a
+// token): 1.004, 1.010, 1.005, 1.009, 1.005, 0.992, 0.958, 0.977. Layer calls over other K, T = 64 / 256 / 1024: 6144 1.005 / 1.003 /
+// 1.003, 5120 1.008 / 1.003 / 1.004, 4608 1.000 / 0.999 / 1.000, 4096 1.001 / 1.002 / 1.001 and 0.976 at T = 4000.
+static bool copier_form(int k, int64_t rows_hint) { return k > 4096 && rows_hint < 4096; }
 
 template <int MODE>
 static int launch_mode(int bn, const ActMaps& ta, const CUtensorMap& tb, const GemmParams& p, int grid, cudaStream_t st) {
@@ -777,7 +779,7 @@ static int launch_mode(int bn, const ActMaps& ta, const CUtensorMap& tb, const G
   if (bn != 256) return 703;
   if (long_loop_form(MODE, p.K, p.rows_hint)) return launch_one<MODE, 256, 128, 0>(ta, tb, p, grid, st);
   if constexpr (MODE != kGemmDense)
-    if (copier_form(p.K)) return launch_one<MODE, 256, 64, 2>(ta, tb, p, grid, st);
+    if (copier_form(p.K, p.rows_hint)) return launch_one<MODE, 256, 64, 2>(ta, tb, p, grid, st);
   return launch_one<MODE, 256, 64, 0>(ta, tb, p, grid, st);
 }
 

@@ -128,6 +128,28 @@ def test_tile_variants_agree():
         layer.close()
 
 
+def test_long_k_loops_on_both_sides_of_the_row_limit():
+    """K > 4096 in 256-wide tiles: the form with copier warps (511 tokens x 8 routes) and the one without (512 x 8) give a token the same
+    bits, and both those of 128-wide tiles."""
+    import kernelschema_b200 as ks
+    h, i, e, k = 4352, 256, 8, 8
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    rand = lambda lo, hi, *shape: torch.randint(lo, hi, shape, dtype=torch.uint8, device="cuda", generator=gen)
+    w1, s1, w2, s2 = rand(0, 256, e, 2 * i, h // 2), rand(40, 60, e, 2 * i, h // 16), rand(0, 256, e, h, i // 2), rand(40, 60, e, h, i // 16)
+    hq, hs = ks.nvfp4_quantize(torch.randn((513, h), device="cuda", generator=gen).to(torch.bfloat16), 1.0)
+    ids, weights = ks.route_topk(torch.randn((513, e), device="cuda", generator=gen), k)
+    outs = []
+    for tokens, tile_n in ((511, 0), (512, 0), (513, 0), (511, 128)):
+        layer = ks.MoELayer(h, i, e, k, tokens, tile_n=tile_n)
+        out = torch.empty((tokens, h), dtype=torch.bfloat16, device="cuda")
+        layer.run(ids[:tokens], weights[:tokens], hq[:tokens], hs[:tokens].view(torch.uint8), w1, s1, w2, s2, out)
+        assert layer.status() == 0
+        outs.append(out[:511].clone())
+        layer.close()
+    assert torch.isfinite(outs[0].float()).all() and outs[0].float().abs().max() > 0
+    assert all(torch.equal(outs[0], v) for v in outs[1:])
+
+
 def test_expert_offset_selects_local_experts_only():
     """local_expert_offset: only ids in [offset, offset+E) contribute (the expert-parallel building block)."""
     from gpu_util import run_model
